@@ -150,6 +150,33 @@ def test_menet_backward_matches_oracle(umi, dev):
     assert np.linalg.norm(grads - want) <= 1e-5 * np.linalg.norm(want)
 
 
+@pytest.mark.parametrize("h,w", [(16, 16), (32, 656), (560, 144), (80, 2064)])
+def test_menet_gradient_tiles(umi, dev, h, w):
+    """Forward and backward at the edges of the training kernels' tiles: fewer
+    rows than the largest dilation, a ragged last 32-column strip, several
+    walks per strip (each CTA's piece of the row order starts in the middle of
+    a dilation class), ragged 8-block and 64-block head tiles.  fp32 sums of at
+    most P = h w / 16 products each: relative error below sqrt(P) 2^-23, 1e-4
+    of the group's scale leaves room for activations whose ReLU flips."""
+    g = np.random.default_rng(h + w)
+    cur = g.integers(0, 256, (h, w), dtype=np.uint8)
+    ref = g.integers(0, 256, (h, w), dtype=np.uint8)
+    p = _params(3)
+    nblk = (h // 16) * (w // 16)
+    tgt = g.integers(-40, 40, (nblk, 2)).astype(np.int32)
+    net = umi.MeNet(h, w, device=dev, params=p)
+    net.ws.fill_(0xFF)  # NaN bytes: every value that is read was written by this pass
+    pred = net.forward(_t(cur, dev), _t(ref, dev)).cpu().numpy()
+    grads = net.backward(_t(tgt, dev)).cpu().numpy().astype(np.float64)
+    want_pred, _ = menet.forward(p, cur, ref, bf16=True)
+    want_loss, want = menet.loss_and_grad(p, cur, ref, tgt, bf16=True)
+    assert np.abs(pred - want_pred).max() <= 2e-5 * np.abs(want_pred).max() + 1e-6
+    assert abs(float(net.loss.item()) - want_loss) <= 1e-5 * abs(want_loss)
+    layers, wh, bh, _ = menet.layout()
+    for a, b in [(wo, bo) for wo, bo in layers] + [(bo, bo + menet.CH) for _, bo in layers] + [(wh, bh), (bh, bh + 2)]:
+        assert np.abs(grads[a:b] - want[a:b]).max() <= 1e-4 * (np.abs(want[a:b]).max() + 1e-12), (a, b)
+
+
 def test_menet_rejects_bad_frames(umi, dev):
     import torch
     assert umi.lib().umi_menet_workspace_bytes(100, 64) == 0
