@@ -24,8 +24,9 @@
 //    next macroblocks' windows are copied (4-byte cp.async by all threads)
 //    while the current ones are searched (full_me_pipe_kernel); the
 //    SAD-volume output keeps one CTA per group of macroblocks
-//    (full_me_kernel).  The benchmark shapes (16x16 blocks, r = 32 and 64,
-//    argmin) go to the warp-specialised kernel of full_me_ws.cu instead.
+//    (full_me_kernel).  16x16 blocks with argmin go elsewhere: ranges up to 7
+//    to the register-only kernel below, the rest to the exact elimination of
+//    full_me_elim.cu.
 #include <algorithm>
 #include <cstring>
 
@@ -35,11 +36,11 @@
 #include "tc_common.cuh"
 
 namespace umi {
-// Warp-specialised search for 16x16 blocks at r = 32, 64 (full_me_ws.cu);
-// UMI_ERR_UNSUPPORTED (nothing launched) for other shapes.
-umi_status full_me_ws(const uint8_t* cur, const uint8_t* ref, int h, int w, int b, int r, const int32_t* centers,
-                      int32_t* out, const int32_t* list, const int32_t* list_count, int max_slots, cudaStream_t st);
-}
+// Argmin search of 16x16 blocks (full_me_elim.cu): any range 1..64, any width
+// and alignment; list, list_count and centers may be null.
+umi_status full_me_elim(const uint8_t* cur, const uint8_t* ref, int h, int w, int r, const int32_t* centers,
+                        int32_t* out, const int32_t* list, const int32_t* list_count, int max_slots, cudaStream_t st);
+}  // namespace umi
 
 namespace {
 
@@ -696,13 +697,13 @@ umi_status full_me_common(const uint8_t* cur, const uint8_t* ref, int32_t h, int
 	g.win_rows = g.ng * G + b - 1;
 	g.win_need = (2 * r + b + 3) / 4 + 1;
 	g.vec_ok = umi::aligned(ref, 4) && umi::aligned(cur, 4) && (w % 4) == 0;
-	if (!volume) {  // the benchmark ranges: warp-specialised kernel (full_me_ws.cu)
-		const umi_status rc = umi::full_me_ws(cur, ref, h, w, b, r, centers, out, list, list_count, max_slots,
-		                                      umi::as_stream(stream));
-		if (rc != UMI_ERR_UNSUPPORTED) return rc == UMI_OK ? umi::ok() : rc;
-	}
 	if (!volume && !list && b == 16 && r <= 7 && g.vec_ok) {  // small windows: registers only
 		const umi_status rc = launch_small(cur, ref, centers, out, g, umi::as_stream(stream));
+		return rc == UMI_OK ? umi::ok() : rc;
+	}
+	if (!volume && b == 16) {
+		const umi_status rc = umi::full_me_elim(cur, ref, h, w, r, centers, out, list, list_count, max_slots,
+		                                        umi::as_stream(stream));
 		return rc == UMI_OK ? umi::ok() : rc;
 	}
 	g.win_words = g.win_need;
@@ -770,4 +771,12 @@ extern "C" umi_status umi_full_me_u8_list(const uint8_t* cur, const uint8_t* ref
 	if (!blocks || !n_blocks) return umi::fail(UMI_ERR_INVALID_ARG, "full_me_list: null block list");
 	if (max_blocks < 0) return umi::fail(UMI_ERR_INVALID_ARG, "full_me_list: negative capacity");
 	return full_me_common(cur, ref, h, w, b, r, centers, mv, false, stream, blocks, n_blocks, max_blocks);
+}
+
+// The searches hold no bounded waits: nothing can have given up.  Waits for
+// the stream, so that a failed launch is reported here.
+extern "C" umi_status umi_full_me_error(int32_t* bits, void* stream) {
+	UMI_TRY(umi::cuda_status(cudaStreamSynchronize(umi::as_stream(stream)), "cudaStreamSynchronize"));
+	if (bits) *bits = 0;
+	return umi::ok();
 }
