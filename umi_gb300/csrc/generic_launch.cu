@@ -24,6 +24,7 @@
 
 #include "common.h"
 #include "umi/UMI_gpu.h"
+#include "window_ops.cuh"
 
 using namespace UMI;
 
@@ -155,6 +156,14 @@ umi_status check_shape(const umi_plan& plan) {
 	return UMI_OK;
 }
 
+// The window form of a strategy (window_ops.cuh), if it has one.
+template <class Umi> struct WindowOf { using Op = void; };
+template <> struct WindowOf<NeighbourSumI32> { using Op = umi_window::NeighbourSum; };
+template <> struct WindowOf<WeightedSumI32> { using Op = umi_window::WeightedI; };
+template <> struct WindowOf<WeightedSumF32> { using Op = umi_window::WeightedF; };
+template <> struct WindowOf<CensusI32> { using Op = umi_window::Census; };
+template <bool MAX> struct WindowOf<ExtremumI32<MAX>> { using Op = umi_window::Extremum<MAX>; };
+
 template <class Umi>
 umi_status launch_as(const umi_plan& plan0, const void* const* in, const void* pad, void* const* out,
                      const void* user_const, size_t uc_bytes, cudaStream_t st) {
@@ -191,6 +200,14 @@ umi_status launch_as(const umi_plan& plan0, const void* const* in, const void* p
 	if (n_cta == 0) return umi::ok();
 	const unsigned grid = (unsigned)(n_cta < 0x7fffffff ? n_cta : 0x7fffffff);
 	const gpu_detail::LinearMaps lm = gpu_detail::linear_maps(plan);
+	using Op = typename WindowOf<Umi>::Op;
+	if constexpr (!std::is_void<Op>::value) {
+		typename Op::C wc{};
+		if (!std::is_empty<C>::value) std::memcpy(&wc, &c, sizeof(C));
+		bool done = false;
+		const umi_status s = umi_window::window_launch<Op>(plan, lm, in, pad, out[0], wc, st, &done);
+		if (s != UMI_OK || done) return s == UMI_OK ? umi::ok() : s;
+	}
 	gpu_detail::launch_generic<Umi, kOnePtr, 0x1111, E, C>(plan, c, ptrs, lm, grid, st);
 	return umi::launch_status("generic_kernel");
 }
