@@ -197,27 +197,49 @@ def launch(desc: Desc, strategy: int, ins, outs, pads=None, consts=None, stream=
     consts: the strategy's constants as a sequence of numbers (int32 or
     float32 by strategy)."""
     import numpy as np
-    import torch
     is_f = strategy in _STRATEGY_FLOAT
-    et = torch.float32 if is_f else torch.int32
-    for i, t in enumerate(list(ins) + list(outs)):
-        _need(t, et, f"memory {i}")
     plan = ctypes.c_void_p()
+    _check_memories(strategy, ins, outs)
     check(lib().umi_plan_create(ctypes.byref(desc), ctypes.byref(plan)), "umi_plan_create")
     try:
-        inp = (ctypes.c_void_p * max(1, len(ins)))(*[t.data_ptr() for t in ins])
-        outp = (ctypes.c_void_p * max(1, len(outs)))(*[t.data_ptr() for t in outs])
-        pad = None
+        pad = uc = None
         if pads is not None:
             pad = np.ascontiguousarray(pads, dtype=np.float32 if is_f else np.int32)
-        uc = None
         if consts is not None:
             uc = np.ascontiguousarray(consts, dtype=np.float32 if is_f else np.int32)
-        check(lib().umi_launch(plan, strategy, inp, pad.ctypes.data_as(ctypes.c_void_p) if pad is not None else None,
-                               outp, uc.ctypes.data_as(ctypes.c_void_p) if uc is not None else None,
-                               uc.nbytes if uc is not None else 0, _stream_ptr(stream)), "umi_launch")
+        _launch(plan, strategy, ins, outs, pad.ctypes.data_as(ctypes.c_void_p) if pad is not None else None,
+                uc.ctypes.data_as(ctypes.c_void_p) if uc is not None else None, uc.nbytes if uc is not None else 0, stream)
     finally:
         lib().umi_plan_destroy(plan)
+
+
+def _check_memories(strategy, ins, outs):
+    import torch
+    et = torch.float32 if strategy in _STRATEGY_FLOAT else torch.int32
+    for i, t in enumerate((*ins, *outs)):
+        _need(t, et, f"memory {i}")
+
+
+def _launch(plan, strategy, ins, outs, pad, consts, const_bytes, stream):
+    inp = (ctypes.c_void_p * max(1, len(ins)))(*[t.data_ptr() for t in ins])
+    outp = (ctypes.c_void_p * max(1, len(outs)))(*[t.data_ptr() for t in outs])
+    check(lib().umi_launch(plan, strategy, inp, pad, outp, consts, const_bytes, _stream_ptr(stream)), "umi_launch")
+
+
+class PlannedLaunch:
+    """launch() with its descriptor, strategy and constants laid out once, for
+    programs that call it again on other buffers (no padding values)."""
+
+    def __init__(self, desc: Desc, strategy: int, consts=()):
+        ct = ctypes.c_float if strategy in _STRATEGY_FLOAT else ctypes.c_int32
+        self.strategy, self.plan = strategy, plan_build(desc)
+        self._ref = ctypes.byref(self.plan)
+        self._consts = (ct * len(consts))(*consts) if consts else None
+        self._bytes = ctypes.sizeof(self._consts) if consts else 0
+
+    def __call__(self, ins, outs, stream=None) -> None:
+        _check_memories(self.strategy, ins, outs)
+        _launch(self._ref, self.strategy, ins, outs, None, self._consts, self._bytes, stream)
 
 
 class BatchGraph:
@@ -285,10 +307,19 @@ def check(status: int, fn: str) -> None:
         raise UmiError(status, fn, detail)
 
 
+_RAW_STREAM = None  # device index -> cudaStream_t of the calling thread's current stream
+
+
 def _stream_ptr(stream=None):
+    global _RAW_STREAM
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    if _RAW_STREAM is None:
+        # the handle without a Stream object around it: 3 us of a small call's 10
+        _RAW_STREAM = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda device: torch.cuda.current_stream(device).cuda_stream)
+    return ctypes.c_void_p(_RAW_STREAM(torch.cuda.current_device()))
 
 
 def _ptr(t):
