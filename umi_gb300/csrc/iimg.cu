@@ -268,58 +268,137 @@ size_t ws_bytes(int h, int w) {
 //   ii[y][x] = sum_{x'<=x} V[b][x'] + sum_{band rows y'<=y} sum_{x'<=x} in[y'][x'],
 //   V[b][x]  = sum_{groups g' above the group of b} S[g'][x] + W[b][x],
 // where S[g][x] is the column sum of group g and W[b][x] the column sum of the
-// bands of its group above b.  Kernel 1 (one CTA per group and 128 columns)
-// reads every group once and writes W and S (uint16: at most 128 * 255).
-// Kernel 2 (one CTA per band) loads its band's pixels, waits for kernel 1
-// (programmatic dependent launch: its launch and pixel loads overlap kernel
-// 1), forms V from at most ceil(h / 128) independent loads per column, scans
-// its RB rows and its V row along x with one block-wide scan of RB + 1
-// values per thread, and writes the band.  Two launches, both parallel over
-// the whole frame; no grid-wide wait.
+// bands of its group above b.  Kernel 1 (one CTA per group and chunk of 128
+// columns) reads every group once and writes W and S (uint16: at most 128 *
+// 255), the row sums of its chunk and the totals of W and S over it.  Kernel 2
+// (one CTA per band and segment of 1024 columns) loads its pixels, waits for
+// kernel 1 (programmatic dependent launch: its launch and pixel loads overlap
+// kernel 1), takes what lies left of its segment from the chunks' row sums and
+// totals (a few values per thread), forms V from at most ceil(h / 128)
+// independent loads per column, scans its RB rows and its V row along x with
+// one block-wide scan of RB + 1 values per thread, and writes its rows with
+// 32-byte stores.  Two launches, both parallel over the whole frame; no
+// grid-wide wait.  Before, one CTA walked a whole band: 270
+// CTAs with two dependent steps each at 4K.  Measured (graph replay, us,
+// before -> now): 2160 x 3840 22.5 -> 17.2, 1440 x 2560 16.1 -> 9.7, 1081 x
+// 1923 (no aligned row) 16.5 -> 9.0, 1080 x 1920 6.9 -> 6.6.  32-byte stores
+// give 1 us of that at 4K (16-byte ones touch every sector twice).  Frames of
+// at most 2048 columns are one segment of 256 threads: two of 128 cost more
+// in the sums to the left than they gain (1080p 7.3).
 constexpr int RB = 8;          // rows per band
 constexpr int GB = 16;         // bands per group
 constexpr int GCT = 16;        // kernel-1 threads across the columns of a group (x CPL = 128 columns)
-constexpr int SEG = NT * CPL;  // columns per kernel-2 pass (2048)
+constexpr int CHUNK = GCT * CPL;   // columns of a kernel-1 CTA
 static_assert(GB * GCT == NT, "kernel 1: one thread per band and 8 columns");
 
 struct BandGeom {
-	int h, w, nb, ng, wpad, nseg;
+	int h, w, nb, ng, wpad, nch;
 	int vec_in, vec_out;
+	int vec_out8;    // rows of out are 32-byte aligned
+	int left;        // several segments per band: kernel 1 writes the last three arrays
 	uint16_t* wsum;  // [ng * GB][wpad]  W
 	uint16_t* gsum;  // [ng][wpad]       S
+	uint16_t* rsum;  // [nch][ng * GB * RB]  row sums per chunk
+	uint32_t* wtot;  // [nch][ng * GB]   W summed over the chunk
+	uint32_t* gtot;  // [nch][ng]        S summed over the chunk
 };
 
-size_t band_ws_bytes(int h, int w) {
-	const size_t nb = umi::ceil_div(h, RB), ng = umi::ceil_div(nb, (size_t)GB), wpad = (size_t)umi::ceil_div(w, CPL) * CPL;
-	auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-	return al(ng * GB * wpad * 2) + al(ng * wpad * 2);
+// Workspace layout (offsets of the arrays above, total in bytes[5]).
+struct BandWork {
+	size_t off[5], bytes;
+	BandWork(int h, int w) {
+		const size_t nb = umi::ceil_div(h, RB), ng = umi::ceil_div(nb, (size_t)GB);
+		const size_t wpad = (size_t)umi::ceil_div(w, CPL) * CPL, nch = umi::ceil_div(w, CHUNK);
+		const size_t n[5] = {ng * GB * wpad * 2, ng * wpad * 2, nch * ng * GB * RB * 2, nch * ng * GB * 4, nch * ng * 4};
+		bytes = 0;
+		for (int i = 0; i < 5; ++i) {
+			off[i] = bytes;
+			bytes += (n[i] + 255) & ~size_t(255);
+		}
+	}
+};
+
+size_t band_ws_bytes(int h, int w) { return BandWork(h, w).bytes; }
+
+// Rows y0 .. y0 + RB - 1 of a thread's 8 columns.  Rows of any alignment are
+// read as three aligned words each, decided once for all of them (a decision
+// per row keeps the loads from being issued together), where every word lies
+// in the frame.
+__device__ __forceinline__ void load_rows(const uint8_t* __restrict__ in, const IimgGeom& g, int y0, int x,
+                                          uint2 (&raw)[RB]) {
+	const size_t o = (size_t)y0 * g.w + x;
+	if (!g.vec_in && x + 7 < g.w && y0 + RB <= g.h && o >= 3 && o + (size_t)(RB - 1) * g.w + 12 <= (size_t)g.h * g.w) {
+		uint32_t w[RB][3];
+#pragma unroll
+		for (int r = 0; r < RB; ++r) {
+			const uint32_t* s = reinterpret_cast<const uint32_t*>((reinterpret_cast<uintptr_t>(in) + o + (size_t)r * g.w) &
+			                                                      ~(uintptr_t)3);
+#pragma unroll
+			for (int k = 0; k < 3; ++k) w[r][k] = __ldg(s + k);
+		}
+#pragma unroll
+		for (int r = 0; r < RB; ++r) {
+			const int sh = 8 * (int)((reinterpret_cast<uintptr_t>(in) + o + (size_t)r * g.w) & 3);
+			raw[r] = make_uint2(__funnelshift_r(w[r][0], w[r][1], sh), __funnelshift_r(w[r][1], w[r][2], sh));
+		}
+	} else {
+#pragma unroll
+		for (int r = 0; r < RB; ++r) raw[r] = load8(in, g, y0 + r, x);
+	}
 }
 
 __global__ void __launch_bounds__(NT) iimg_group_sums(const uint8_t* __restrict__ in, const BandGeom g) {
-	__shared__ __align__(16) uint32_t cs[GB][GCT * CPL];
+	__shared__ __align__(16) uint32_t cs[GB][CHUNK];
+	__shared__ uint32_t btot[GB];  // total of each band
 	pdl_trigger();
 	const int gi = blockIdx.y, j = threadIdx.x / GCT, c = threadIdx.x % GCT;
-	const int xs = blockIdx.x * GCT * CPL, x0 = xs + c * CPL;
+	const int xs = blockIdx.x * CHUNK, x0 = xs + c * CPL;
 	IimgGeom ig{};
 	ig.h = g.h; ig.w = g.w; ig.vec_in = g.vec_in;
 	uint32_t s[CPL] = {};
+	uint32_t rows[RB / 2] = {};  // row sums of these 8 columns, two rows per word (at most 128 * 255 per chunk)
 	if (x0 < g.w) {
 		const int y0 = (gi * GB + j) * RB;
 		uint2 raw[RB];
-#pragma unroll
-		for (int r = 0; r < RB; ++r) raw[r] = load8(in, ig, y0 + r, x0);
+		load_rows(in, ig, y0, x0, raw);
 #pragma unroll
 		for (int r = 0; r < RB; ++r) {
 			uint32_t v[CPL];
 			unpack8(raw[r], v);
+			uint32_t t = 0;
 #pragma unroll
-			for (int k = 0; k < CPL; ++k) s[k] += v[k];
+			for (int k = 0; k < CPL; ++k) {
+				s[k] += v[k];
+				t += v[k];
+			}
+			rows[r >> 1] += t << (16 * (r & 1));
 		}
+	}
+	if (g.left) {
+#pragma unroll
+		for (int i = 0; i < RB / 2; ++i)
+#pragma unroll
+			for (int o = 1; o < GCT; o <<= 1) rows[i] += __shfl_xor_sync(0xffffffffu, rows[i], o);
+	}
+	if (g.left && c == 0) {
+		static_assert(RB == 8, "one 16-byte store per band");
+		*reinterpret_cast<uint4*>(g.rsum + ((size_t)blockIdx.x * g.ng * GB + gi * GB + j) * RB) =
+			make_uint4(rows[0], rows[1], rows[2], rows[3]);
+		uint32_t t = 0;
+#pragma unroll
+		for (int i = 0; i < RB / 2; ++i) t += (rows[i] & 0xffffu) + (rows[i] >> 16);
+		btot[j] = t;
 	}
 	*reinterpret_cast<uint4*>(&cs[j][c * CPL]) = make_uint4(s[0], s[1], s[2], s[3]);
 	*reinterpret_cast<uint4*>(&cs[j][c * CPL + 4]) = make_uint4(s[4], s[5], s[6], s[7]);
 	__syncthreads();
-	if (threadIdx.x < GCT * CPL) {  // one column per thread: exclusive prefix over the group's bands
+	if (g.left && threadIdx.x < GB) {
+		uint32_t run = 0;
+		for (int k = 0; k < (int)threadIdx.x; ++k) run += btot[k];
+		g.wtot[(size_t)blockIdx.x * g.ng * GB + gi * GB + threadIdx.x] = run;
+		if (threadIdx.x == GB - 1) g.gtot[(size_t)blockIdx.x * g.ng + gi] = run + btot[GB - 1];
+	}
+	if (threadIdx.x < CHUNK) {  // one column per thread: exclusive prefix over the group's bands
 		const int x = xs + threadIdx.x;
 		if (x < g.w) {
 			uint32_t run = 0;
@@ -340,109 +419,125 @@ __device__ __forceinline__ void add_u16x8(uint32_t (&v)[CPL], uint4 p) {
 	v[6] += p.w & 0xffffu; v[7] += p.w >> 16;
 }
 
-__global__ void __launch_bounds__(NT) iimg_band_out(const uint8_t* __restrict__ in, int32_t* __restrict__ out,
-                                                     const BandGeom g) {
-	__shared__ uint32_t wtot[NW][RB + 1];
+// NT2: threads, 8 columns each.
+template <int NT2>
+__global__ void __launch_bounds__(NT2, NT2 == 128 ? 6 : 2) iimg_band_out(const uint8_t* __restrict__ in, int32_t* __restrict__ out,
+                                                      const BandGeom g) {
+	constexpr int NW2 = NT2 / 32, SEG = NT2 * CPL;
+	static_assert(SEG % CHUNK == 0, "segments start on chunks");
+	__shared__ uint32_t wtot[NW2][RB + 1];
+	__shared__ uint32_t left[NW2][RB + 1];  // per warp: sums over the chunks left of the segment (rows, then the V row)
+	__shared__ __align__(16) uint32_t rowbuf[NW2][4][32 * CPL];
 	const int b = blockIdx.x, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-	const int y0 = b * RB;
+	const int y0 = b * RB, x0 = blockIdx.y * SEG + threadIdx.x * CPL;
+	const bool live = x0 < g.w;
 	IimgGeom ig{};
 	ig.h = g.h; ig.w = g.w; ig.vec_in = g.vec_in;
-	uint32_t carry[RB + 1] = {};  // totals of the segments to the left (rows, then the V row)
-	uint2 raw[RB];
-	{
-		const int x0 = threadIdx.x * CPL;
-#pragma unroll
-		for (int r = 0; r < RB; ++r) raw[r] = x0 < g.w ? load8(in, ig, y0 + r, x0) : make_uint2(0, 0);
-	}
+	uint2 raw[RB] = {};
+	if (live) load_rows(in, ig, y0, x0, raw);
 	pdl_wait();
-	for (int seg = 0; seg < g.nseg; ++seg) {
-		const int x0 = seg * SEG + threadIdx.x * CPL;
-		const bool live = x0 < g.w;
-		if (seg > 0) {
-#pragma unroll
-			for (int r = 0; r < RB; ++r) raw[r] = live ? load8(in, ig, y0 + r, x0) : make_uint2(0, 0);
-		}
-		uint32_t vv[CPL] = {};
-		if (live) {  // V = W of this band + S of every group above
-			add_u16x8(vv, __ldcg(reinterpret_cast<const uint4*>(g.wsum + (size_t)b * g.wpad + x0)));
-			const int gb = b / GB;
+	const int gb = b / GB, nleft = blockIdx.y * (SEG / CHUNK);  // groups above, chunks to the left
+	uint32_t vv[CPL] = {};
+	if (live) {  // V = W of this band + S of every group above
+		add_u16x8(vv, __ldcg(reinterpret_cast<const uint4*>(g.wsum + (size_t)b * g.wpad + x0)));
 #pragma unroll 8
-			for (int q = 0; q < gb; ++q) add_u16x8(vv, __ldcg(reinterpret_cast<const uint4*>(g.gsum + (size_t)q * g.wpad + x0)));
+		for (int q = 0; q < gb; ++q) add_u16x8(vv, __ldcg(reinterpret_cast<const uint4*>(g.gsum + (size_t)q * g.wpad + x0)));
+	}
+	if (nleft) {
+		uint32_t rl[CPL] = {}, vl = 0;
+		for (int c = threadIdx.x; c < nleft; c += NT2) {
+			add_u16x8(rl, __ldcg(reinterpret_cast<const uint4*>(g.rsum + ((size_t)c * g.ng * GB + b) * RB)));
+			vl += __ldcg(g.wtot + (size_t)c * g.ng * GB + b);
 		}
-		// thread totals of each row and of the V row, scanned over the block
-		uint32_t tsum[RB + 1];
+		for (int c = wp; c < nleft; c += NW2)
+			for (int q = lane; q < gb; q += 32) vl += __ldcg(g.gtot + (size_t)c * g.ng + q);
 #pragma unroll
-		for (int r = 0; r < RB; ++r) {
-			uint32_t v[CPL];
-			unpack8(raw[r], v);
-			uint32_t t = 0;
+		for (int r = 0; r < RB; ++r) rl[r] = __reduce_add_sync(0xffffffffu, rl[r]);
+		vl = __reduce_add_sync(0xffffffffu, vl);
+		if (lane == 0) {
 #pragma unroll
-			for (int k = 0; k < CPL; ++k) t += v[k];
-			tsum[r] = t;
+			for (int r = 0; r < RB; ++r) left[wp][r] = rl[r];
+			left[wp][RB] = vl;
 		}
-		{
-			uint32_t t = 0;
+	}
+	// thread totals of each row and of the V row, scanned over the block
+	uint32_t tsum[RB + 1];
 #pragma unroll
-			for (int k = 0; k < CPL; ++k) t += vv[k];
-			tsum[RB] = t;
+	for (int r = 0; r < RB; ++r) {
+		uint32_t v[CPL];
+		unpack8(raw[r], v);
+		uint32_t t = 0;
+#pragma unroll
+		for (int k = 0; k < CPL; ++k) t += v[k];
+		tsum[r] = t;
+	}
+	{
+		uint32_t t = 0;
+#pragma unroll
+		for (int k = 0; k < CPL; ++k) t += vv[k];
+		tsum[RB] = t;
+	}
+	uint32_t ex[RB + 1];
+#pragma unroll
+	for (int r = 0; r <= RB; ++r) {
+		const uint32_t inc = warp_incl_scan(tsum[r], lane);
+		ex[r] = inc - tsum[r];
+		if (lane == 31) wtot[wp][r] = inc;
+	}
+	__syncthreads();
+#pragma unroll
+	for (int r = 0; r <= RB; ++r) {
+#pragma unroll
+		for (int k = 0; k < NW2 - 1; ++k) ex[r] += k < wp ? wtot[k][r] : 0u;
+		if (nleft)
+#pragma unroll
+			for (int k = 0; k < NW2; ++k) ex[r] += left[k][r];
+	}
+	// outputs: T(x) = V-row prefix, plus the running column sum of the row prefixes
+	uint32_t T[CPL];
+	{
+		uint32_t tp = ex[RB];
+#pragma unroll
+		for (int k = 0; k < CPL; ++k) {
+			tp += vv[k];
+			T[k] = tp;
 		}
-		uint32_t ex[RB + 1];
+	}
 #pragma unroll
-		for (int r = 0; r <= RB; ++r) {
-			const uint32_t inc = warp_incl_scan(tsum[r], lane);
-			ex[r] = inc - tsum[r];
-			if (lane == 31) wtot[wp][r] = inc;
+	for (int r = 0; r < RB; ++r) {
+		uint32_t rp = ex[r];
+#pragma unroll
+		for (int k = 0; k < CPL; ++k) {
+			rp += (k < 4 ? (raw[r].x >> (8 * k)) : (raw[r].y >> (8 * (k - 4)))) & 0xffu;
+			T[k] += rp;
 		}
-		__syncthreads();
-		uint32_t segtot[RB + 1];
+		const int y = y0 + r;
+		if (y >= g.h) break;
+		int32_t* op = out + (size_t)y * g.w + x0;
+		if (g.vec_out8) {  // w % 8 == 0: every live thread has 8 columns
+			if (live)
+				asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(op), "r"(T[0]), "r"(T[1]),
+				             "r"(T[2]), "r"(T[3]), "r"(T[4]), "r"(T[5]), "r"(T[6]), "r"(T[7])
+				             : "memory");
+		} else if (g.vec_out) {  // w % 4 == 0
+			if (live) reinterpret_cast<int4*>(op)[0] = make_int4(T[0], T[1], T[2], T[3]);
+			if (x0 + 7 < g.w) reinterpret_cast<int4*>(op)[1] = make_int4(T[4], T[5], T[6], T[7]);
+		} else {  // any alignment: the warp's 256 columns through shared memory, four rows at a time
+			uint32_t* row = rowbuf[wp][r & 3];
+			*reinterpret_cast<uint4*>(row + CPL * lane) = make_uint4(T[0], T[1], T[2], T[3]);
+			*reinterpret_cast<uint4*>(row + CPL * lane + 4) = make_uint4(T[4], T[5], T[6], T[7]);
+			if ((r & 3) == 3 || y == g.h - 1) {
+				__syncwarp();
+				const int xw = x0 - CPL * lane + lane;
+				for (int i = 0; i <= (r & 3); ++i) {
+					int32_t* o = out + (size_t)(y - (r & 3) + i) * g.w + xw;
 #pragma unroll
-		for (int r = 0; r <= RB; ++r) {
-			uint32_t before = 0, all = 0;
-#pragma unroll
-			for (int k = 0; k < NW; ++k) {
-				const uint32_t t = wtot[k][r];
-				before += k < wp ? t : 0u;
-				all += t;
-			}
-			ex[r] += before + carry[r];
-			segtot[r] = all;
-		}
-		__syncthreads();  // wtot is rewritten by the next segment
-		// outputs: T(x) = V-row prefix, plus the running column sum of the row prefixes
-		uint32_t T[CPL], colacc[CPL];
-		{
-			uint32_t tp = ex[RB];
-#pragma unroll
-			for (int k = 0; k < CPL; ++k) {
-				tp += vv[k];
-				T[k] = tp;
-				colacc[k] = 0;
-			}
-		}
-#pragma unroll
-		for (int r = 0; r < RB; ++r) {
-			uint32_t rp = ex[r], o[CPL];
-#pragma unroll
-			for (int k = 0; k < CPL; ++k) {
-				rp += (k < 4 ? (raw[r].x >> (8 * k)) : (raw[r].y >> (8 * (k - 4)))) & 0xffu;
-				colacc[k] += rp;
-				o[k] = T[k] + colacc[k];
-			}
-			const int y = y0 + r;
-			if (live && y < g.h) {
-				int32_t* op = out + (size_t)y * g.w + x0;
-				if (g.vec_out && x0 + 7 < g.w) {
-					reinterpret_cast<int4*>(op)[0] = make_int4(o[0], o[1], o[2], o[3]);
-					reinterpret_cast<int4*>(op)[1] = make_int4(o[4], o[5], o[6], o[7]);
-				} else {
-#pragma unroll
-					for (int k = 0; k < CPL; ++k)
-						if (x0 + k < g.w) op[k] = (int32_t)o[k];
+					for (int k = 0; k < CPL; ++k)  // 128 contiguous bytes per store
+						if (xw + 32 * k < g.w) o[32 * k] = (int32_t)rowbuf[wp][i][32 * k + lane];
 				}
+				__syncwarp();
 			}
 		}
-#pragma unroll
-		for (int r = 0; r <= RB; ++r) carry[r] += segtot[r];
 	}
 }
 
@@ -476,25 +571,33 @@ extern "C" umi_status umi_iimg_u8_i32(const uint8_t* in, int32_t* out, int32_t h
 	g.nb = umi::ceil_div(h, RB);
 	g.ng = umi::ceil_div(g.nb, GB);
 	g.wpad = umi::ceil_div(w, CPL) * CPL;
-	g.nseg = umi::ceil_div(w, SEG);
+	g.nch = umi::ceil_div(w, CHUNK);
 	g.vec_in = umi::aligned(in, 8) && (w % 8) == 0;
 	g.vec_out = umi::aligned(out, 16) && (w % 4) == 0;
-	auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+	g.vec_out8 = umi::aligned(out, 32) && (w % 8) == 0;
+	// a frame of at most 2048 columns is one segment (nothing lies left of it)
+	const int nt2 = w <= 256 * CPL ? 256 : 128;
+	g.left = w > nt2 * CPL;
+	const BandWork work(h, w);
 	char* ws = static_cast<char*>(workspace);
-	g.wsum = reinterpret_cast<uint16_t*>(ws);
-	g.gsum = reinterpret_cast<uint16_t*>(ws + al((size_t)g.ng * GB * g.wpad * 2));
+	g.wsum = reinterpret_cast<uint16_t*>(ws + work.off[0]);
+	g.gsum = reinterpret_cast<uint16_t*>(ws + work.off[1]);
+	g.rsum = reinterpret_cast<uint16_t*>(ws + work.off[2]);
+	g.wtot = reinterpret_cast<uint32_t*>(ws + work.off[3]);
+	g.gtot = reinterpret_cast<uint32_t*>(ws + work.off[4]);
 	const cudaStream_t st = umi::as_stream(stream);
 	// kernel 1 follows whatever the stream ran before: plain launch
-	iimg_group_sums<<<dim3(umi::ceil_div(w, GCT * CPL), g.ng), NT, 0, st>>>(in, g);
+	iimg_group_sums<<<dim3(g.nch, g.ng), NT, 0, st>>>(in, g);
 	UMI_TRY(umi::launch_status("iimg_group_sums"));
 	cudaLaunchAttribute attr[1] = {pdl_attr()};
 	cudaLaunchConfig_t cfg{};
-	cfg.gridDim = dim3(g.nb);
-	cfg.blockDim = dim3(NT);
+	cfg.gridDim = dim3(g.nb, umi::ceil_div(w, nt2 * CPL));
+	cfg.blockDim = dim3(nt2);
 	cfg.stream = st;
 	cfg.attrs = attr;
 	cfg.numAttrs = 1;
-	UMI_TRY(umi::cuda_status(cudaLaunchKernelEx(&cfg, iimg_band_out, in, out, g), "iimg_band_out"));
+	UMI_TRY(umi::cuda_status(cudaLaunchKernelEx(&cfg, nt2 == 256 ? iimg_band_out<256> : iimg_band_out<128>, in, out, g),
+	                         "iimg_band_out"));
 	return umi::ok();
 }
 
