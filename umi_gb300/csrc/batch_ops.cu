@@ -366,7 +366,9 @@ struct CostVolume {
 // Roles (480 threads): warps 0-4 and 5-9 are two producer groups taking
 // alternate tiles, each filling its own operand stage (plain loads of two
 // operand rows per thread, split, swizzled 16-byte stores, then a proxy fence
-// and an mbarrier arrive), so two tiles' loads are in flight per SM; warp 10
+// and an mbarrier arrive); a thread loads its next tile's rows as soon as this
+// tile's registers are stored, so a group never waits for memory with nothing
+// in flight; warp 10
 // allocates TMEM (two accumulators of 192 columns) and one lane issues the
 // MMAs; warps 11-14 drain an accumulator while the next tile computes: lane p
 // of a warp holds TMEM row p (one pixel), loads the 96 columns its warp's band
@@ -374,6 +376,16 @@ struct CostVolume {
 // stores (word 63 p + j) into one of two staging buffers, and the warp writes
 // its 32 pixels x 64 disparities (8 KB, contiguous in cv) with one bulk copy.
 // Every wait is bounded (tc_common.cuh).
+//
+// What bounds it: the producers.  Reading and writing HBM takes about 2600 SM
+// cycles per tile and SM at the measured copy rate; the split and its swizzled
+// stores take 2900 without the loads, and the loads share the load/store pipe
+// with the stores: 4490 cycles per tile in all (5200 before a tile's loads were
+// issued under the previous tile's stores).  Six uneven images of 256 to 2048
+// pixels a side with 32 channels, all three operators: 1117 -> 1024 us.  Raw rows copied to
+// shared memory first (16-byte cp.async, or bulk copies, which issue one lane
+// at a time at about 60 clocks each) and all ten warps on one tile were no
+// faster: 5400, 5400 and 4541.
 namespace cvtc {
 constexpr int BM = 128, ND = 64, BNN = BM + ND, KC = 32;
 constexpr uint32_t A_BYTES = BM * 128, B_BYTES = BNN * 128;
@@ -482,26 +494,50 @@ __device__ __forceinline__ void cv_tc_phase(const Table& t, const cvtc::Params& 
 		// ---- producers: group G takes tiles G, G + 2, ... of this CTA into stage G
 		const int G = warp / 5, tg = threadIdx.x - G * PG;
 		uint8_t* st_base = base + G * STAGE_BYTES;
-		int u = 0;
-		for (int tile = blockIdx.x + G * gridDim.x; tile < total && !*abort_flag; tile += 2 * gridDim.x, ++u) {
-			const int i = find_image(t, tile);
-			const Img& im = t.img[i];
-			const int lt = tile - t.start[i], y = lt / im.tiles_x, x0 = (lt - y * im.tiles_x) * BM;
-			const size_t plane = (size_t)im.h * im.w, row0 = (size_t)y * im.w;
-			// operand rows r = tg and tg + 160 of 320: r < 128 is pixel r of A (L), else column r - 128 of B (R)
-			float va[KC], vb[KC];
-			const int r0 = tg, r1 = tg + PG;  // r1 >= 160: always a B row
-			const int xa = r0 < BM ? r0 : r0 - BM, xb = r1 - BM;
-			load_row((r0 < BM ? im.in : im.aux) + row0 + x0 + xa, plane, prm.channels, x0 + xa < im.w, va);
-			load_row(im.aux + row0 + x0 + xb, plane, prm.channels, x0 + xb < im.w, vb);
-			// the loads are in flight while the stage's previous MMAs finish
+		// operand rows r = tg and tg + 160 of 320: r < 128 is pixel r of A (L), else column r - 128 of B (R)
+		const int r0 = tg, r1 = tg + PG;  // r1 >= 160: always a B row
+		const int xa = r0 < BM ? r0 : r0 - BM, xb = r1 - BM;
+		uint8_t* bhi = st_base + 2 * A_BYTES;
+		uint8_t* dst = r0 < BM ? st_base : bhi;
+		const uint32_t lo = r0 < BM ? A_BYTES : B_BYTES;
+		// the tile whose rows are being loaded: its image, image row and first column
+		int img = 0, y = 0, x0 = 0;
+		auto place = [&](int tile) {
+			while (t.start[img + 1] <= tile) ++img;
+			const int lt = tile - t.start[img];
+			y = lt / t.img[img].tiles_x;
+			x0 = (lt - y * t.img[img].tiles_x) * BM;
+		};
+		auto load_a = [&](float (&v)[KC]) {
+			const Img& im = t.img[img];
+			load_row((r0 < BM ? im.in : im.aux) + (size_t)y * im.w + x0 + xa, (size_t)im.h * im.w, prm.channels,
+			         x0 + xa < im.w, v);
+		};
+		auto load_b = [&](float (&v)[KC]) {
+			const Img& im = t.img[img];
+			load_row(im.aux + (size_t)y * im.w + x0 + xb, (size_t)im.h * im.w, prm.channels, x0 + xb < im.w, v);
+		};
+		// The next tile's loads are issued as soon as this tile's registers are
+		// stored, one operand row after the other: a thread always has at least 32
+		// loads in flight while it converts and stores.
+		float va[KC], vb[KC];
+		int tile = blockIdx.x + G * gridDim.x;
+		if (tile < total) {
+			place(tile);
+			load_a(va);
+			load_b(vb);
+		}
+		for (int u = 0; tile < total && !*abort_flag; ++u) {
+			const int next = tile + 2 * gridDim.x;
 			if (!mbar_wait(&empty[G], (uint32_t)(u & 1) ^ 1u, abort_flag, err, kErrTimeoutEmpty)) break;
-			uint8_t* bhi = st_base + 2 * A_BYTES;
-			if (r0 < BM) store_row(st_base, st_base + A_BYTES, r0, va);
-			else store_row(bhi, bhi + B_BYTES, xa, va);
+			if (next < total) place(next);
+			store_row(dst, dst + lo, xa, va);
+			if (next < total) load_a(va);
 			store_row(bhi, bhi + B_BYTES, xb, vb);
 			fence_proxy_async_smem();  // generic-proxy stores visible to the MMA
 			mbar_arrive(&full[G]);
+			if (next < total) load_b(vb);
+			tile = next;
 		}
 	} else if (warp == 10) {
 		if (lane == 0) {
