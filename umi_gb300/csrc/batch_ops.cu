@@ -407,12 +407,14 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 	asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
 	return r;
 }
-__device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool acc) {
+__device__ __forceinline__ void mma_tf32(uint32_t one, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         bool acc) {
 	asm volatile(
-		"{\n\t.reg .pred p;\n\t"
+		"{\n\t.reg .pred p, q;\n\t"
 		"setp.ne.b32 p, %4, 0;\n\t"
-		"tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-		"l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)acc)
+		"setp.ne.b32 q, %5, 0;\n\t"
+		"@q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+		"l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)acc), "r"(one)
 		: "memory");
 }
 // shared -> global bulk copy (16-byte aligned addresses, size a multiple of 16)
@@ -468,7 +470,7 @@ __device__ __forceinline__ void cv_tc_phase(const Table& t, const cvtc::Params& 
 	uint64_t* drain = accempty + 2;
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
 	volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 	const int total = t.start[t.n];
 	if (threadIdx.x == 0) {
 		for (int s = 0; s < 2; ++s) {
@@ -540,32 +542,31 @@ __device__ __forceinline__ void cv_tc_phase(const Table& t, const cvtc::Params& 
 			tile = next;
 		}
 	} else if (warp == 10) {
-		if (lane == 0) {
-			// ---- MMA issuer
-			int i = 0;
-			for (int tile = blockIdx.x; tile < total && !*abort_flag; tile += gridDim.x, ++i) {
-				const int s = i & 1;
-				const uint32_t use = (uint32_t)(i >> 1);
-				if (!mbar_wait(&accempty[s], (use & 1) ^ 1u, abort_flag, err, kErrTimeoutAccEmpty)) break;
-				if (!mbar_wait(&full[s], use & 1, abort_flag, err, kErrTimeoutFull)) break;
-				tc_fence_after();
-				const uint32_t acc = tmem + (uint32_t)(s * BNN);
-				const uint32_t sb = smem_u32(base + s * STAGE_BYTES);
-				const uint64_t ahi = desc_kmajor_sw128(sb), alo = desc_kmajor_sw128(sb + A_BYTES);
-				const uint64_t bhi = desc_kmajor_sw128(sb + 2 * A_BYTES), blo = desc_kmajor_sw128(sb + 2 * A_BYTES + B_BYTES);
+		// ---- MMA issuer: all lanes wait, one issues
+		const uint32_t one = elect_one();
+		int i = 0;
+		for (int tile = blockIdx.x; tile < total && !*abort_flag; tile += gridDim.x, ++i) {
+			const int s = i & 1;
+			const uint32_t use = (uint32_t)(i >> 1);
+			if (!mbar_wait(&accempty[s], (use & 1) ^ 1u, abort_flag, err, kErrTimeoutAccEmpty)) break;
+			if (!mbar_wait(&full[s], use & 1, abort_flag, err, kErrTimeoutFull)) break;
+			tc_fence_after();
+			const uint32_t acc = tmem + (uint32_t)(s * BNN);
+			const uint32_t sb = smem_u32(base + s * STAGE_BYTES);
+			const uint64_t ahi = desc_kmajor_sw128(sb), alo = desc_kmajor_sw128(sb + A_BYTES);
+			const uint64_t bhi = desc_kmajor_sw128(sb + 2 * A_BYTES), blo = desc_kmajor_sw128(sb + 2 * A_BYTES + B_BYTES);
 #pragma unroll
-				for (int kk = 0; kk < KC / 8; ++kk) {  // 8 tf32 = 32 bytes per K step
-					mma_tf32(acc, ahi + 2 * kk, bhi + 2 * kk, IDESC, kk > 0);
-					mma_tf32(acc, ahi + 2 * kk, blo + 2 * kk, IDESC, true);
-					mma_tf32(acc, alo + 2 * kk, bhi + 2 * kk, IDESC, true);
-				}
-				mma_commit(&empty[s]);
-				mma_commit(&accfull[s]);
+			for (int kk = 0; kk < KC / 8; ++kk) {  // 8 tf32 = 32 bytes per K step
+				mma_tf32(one, acc, ahi + 2 * kk, bhi + 2 * kk, IDESC, kk > 0);
+				mma_tf32(one, acc, ahi + 2 * kk, blo + 2 * kk, IDESC, true);
+				mma_tf32(one, acc, alo + 2 * kk, bhi + 2 * kk, IDESC, true);
 			}
-			mma_commit(drain);  // every MMA issued above finishes before TMEM is freed
-			volatile int own = 0;
-			mbar_wait(drain, 0, &own, err, kErrTimeoutAccum);
+			mma_commit(one, &empty[s]);
+			mma_commit(one, &accfull[s]);
 		}
+		mma_commit(one, drain);  // every MMA issued above finishes before TMEM is freed
+		volatile int own = 0;
+		mbar_wait(drain, 0, &own, err, kErrTimeoutAccum);
 		__syncwarp();
 	} else {
 		// ---- epilogue: warp w drains TMEM lanes 32 (w % 4) .. + 31 (pixels of the tile)

@@ -106,7 +106,6 @@ struct ConvArgs {
 	float* out;
 	int n, c, h, w, k, r;
 	int xtiles, ktiles;
-	int vec4;  // out 16-byte aligned and w % 4 == 0: float4 stores along x
 	int* err;
 };
 struct ConvPolicy {
@@ -146,55 +145,23 @@ struct ConvPolicy {
 		tma_load_2d(b, tb, bar, tap * g.c + c0, 0);
 	}
 	// This thread holds pixel x0 + rl of the tile for output channels
-	// [k0+c, +32).  Groups of 4 channels are transposed across the 4 lanes of
-	// each quad (two butterfly shuffle stages), after which lane 4j+m holds
-	// channel 4*grp+m of pixels 4j..4j+3: one 16-byte store per lane and
-	// group instead of four 4-byte stores.  Every lane takes part in the
-	// shuffles; bounds are checked at the stores.
+	// [k0+c, +32): a warp's store of one channel is 32 consecutive pixels, one
+	// 128-byte line where the row starts on one.  Transposing 4 x 4 blocks
+	// across lanes for 16-byte stores (32 shuffles per thread and 32 channels)
+	// took 1900 clocks a pass against 800 to 1000 for these, as the shuffles
+	// share the shared-memory pipe with the MMAs' operand reads.
 	__device__ static void store(const Args& g, const Tile& t, int rl, int c, const float (&v)[32]) {
-		const int lane = rl & 31, m = lane & 3;
-		const bool b1 = (m >> 1) & 1, b0 = m & 1;
-		const int xq = t.x0 + (rl - m);  // first pixel of this lane's quad
+		const int x = t.x0 + rl, left = g.k - t.k0 - c;
+		if (x >= g.w) return;
 		const size_t plane = (size_t)g.h * g.w;
-		float* base = g.out + ((size_t)t.n * g.k) * plane + (size_t)t.y * g.w + xq;
-		const bool vec = g.vec4 && xq + 3 < g.w;
+		float* dst = g.out + ((size_t)t.n * g.k + t.k0 + c) * plane + (size_t)t.y * g.w + x;
+		if (left >= 32) {
 #pragma unroll
-		for (int grp = 0; grp < 8; ++grp) {
-			// r[k] = channel 4grp+k of this lane's pixel
-			float r0 = v[4 * grp], r1 = v[4 * grp + 1], r2 = v[4 * grp + 2], r3 = v[4 * grp + 3];
-			// stage 1 (lanes m, m^2): keep the channel pair whose high bit is b1, swap the other
-			{
-				const float s0 = b1 ? r0 : r2, s1 = b1 ? r1 : r3;
-				const float y0 = __shfl_xor_sync(0xffffffffu, s0, 2), y1 = __shfl_xor_sync(0xffffffffu, s1, 2);
-				// now (row p1, col c0): own row for p1 == b1, partner's row otherwise; channels (b1, c0)
-				const float k0 = b1 ? r2 : r0, k1 = b1 ? r3 : r1;  // own values of channels (b1, 0), (b1, 1)
-				r0 = b1 ? y0 : k0;  // pixel (0, b0), channel (b1, 0)
-				r1 = b1 ? y1 : k1;  // pixel (0, b0), channel (b1, 1)
-				r2 = b1 ? k0 : y0;  // pixel (1, b0), channel (b1, 0)
-				r3 = b1 ? k1 : y1;  // pixel (1, b0), channel (b1, 1)
-			}
-			// stage 2 (lanes m, m^1): keep channel low bit b0, swap the other
-			{
-				const float s0 = b0 ? r0 : r1, s1 = b0 ? r2 : r3;
-				const float y0 = __shfl_xor_sync(0xffffffffu, s0, 1), y1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-				const float k0 = b0 ? r1 : r0, k1 = b0 ? r3 : r2;  // own: pixels (0, b0), (1, b0), channel (b1, b0)
-				// pixel (p1, p0) of channel (b1, b0): own when p0 == b0
-				const float q00 = b0 ? y0 : k0, q01 = b0 ? k0 : y0;  // p1 = 0: p0 = 0, 1
-				const float q10 = b0 ? y1 : k1, q11 = b0 ? k1 : y1;  // p1 = 1: p0 = 0, 1
-				r0 = q00; r1 = q01; r2 = q10; r3 = q11;             // pixels 0, 1, 2, 3 of the quad
-			}
-			const int kk = t.k0 + c + 4 * grp + m;
-			if (kk < g.k) {
-				float* dst = base + (size_t)kk * plane;
-				if (vec) {
-					*reinterpret_cast<float4*>(dst) = make_float4(r0, r1, r2, r3);
-				} else {
-					if (xq < g.w) dst[0] = r0;
-					if (xq + 1 < g.w) dst[1] = r1;
-					if (xq + 2 < g.w) dst[2] = r2;
-					if (xq + 3 < g.w) dst[3] = r3;
-				}
-			}
+			for (int j = 0; j < 32; ++j, dst += plane) *dst = v[j];
+		} else {
+#pragma unroll
+			for (int j = 0; j < 32; ++j, dst += plane)
+				if (j < left) *dst = v[j];
 		}
 	}
 };
@@ -264,7 +231,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 	uint64_t* bready = drain + 1;        // resident B loaded (RES only)
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bready + 1);
 	volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 	const int ntiles = P::ntiles(g);
 	const int nk = P::nk(g);  // K-slices of A and B: ring loads per tile
 
@@ -323,8 +290,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 				if (armed[s] >= 0) mbar_wait(&full[s], (uint32_t)armed[s] & 1, &own, g.err, kErrTimeoutFull);
 			if constexpr (RES) mbar_wait(bready, 0, &own, g.err, kErrTimeoutFull);
 		}
-	} else if (warp == 1 && lane == 0) {
-		// ---- MMA issuer
+	} else if (warp == 1) {
+		// ---- MMA issuer: all lanes wait, one issues
+		const uint32_t one = elect_one();
 		bool ready = true;
 		if constexpr (RES) ready = mbar_wait(bready, 0, abort_flag, g.err, kErrTimeoutFull);
 		uint32_t q = 0;
@@ -345,14 +313,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 				const uint64_t bd =
 					desc_kmajor_sw128(smem_u32(RES ? bres + ks * B_TILE : base + s * STAGE_BYTES + A_TILE));
 #pragma unroll
-				for (int kk = 0; kk < BK / 16; ++kk) mma_f16(acc, ad + 2 * kk, bd + 2 * kk, idesc, ks > 0 || kk > 0);
-				mma_commit(&empty[s]);
+				for (int kk = 0; kk < BK / 16; ++kk) mma_f16(one, acc, ad + 2 * kk, bd + 2 * kk, idesc, ks > 0 || kk > 0);
+				mma_commit(one, &empty[s]);
 			}
 			if (!ok) break;
-			mma_commit(&accfull[a]);
+			mma_commit(one, &accfull[a]);
 		}
 		// every MMA issued above finishes before TMEM is freed
-		mma_commit(drain);
+		mma_commit(one, drain);
 		volatile int own = 0;
 		mbar_wait(drain, 0, &own, g.err, kErrTimeoutAccum);
 	} else if (warp >= 2) {
@@ -567,7 +535,7 @@ __global__ void __launch_bounds__(run_threads<T>(), 1)
 	uint64_t* bready = drain + 1;
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bready + 1);
 	volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 	const int H = T::rows(g), ntiles = T::blocks(g) * H, d = T::dil(g);
 	const int t0 = blockIdx.x * per, t1 = min(ntiles, t0 + per);
 	// the segment of the run starting at tile s0: block, first output row, end
@@ -631,8 +599,9 @@ __global__ void __launch_bounds__(run_threads<T>(), 1)
 				if (armed[s] >= 0) mbar_wait(&full[s], (uint32_t)armed[s] & 1, &own, g.err, kErrTimeoutFull);
 			mbar_wait(bready, 0, &own, g.err, kErrTimeoutFull);
 		}
-	} else if (warp == 1 && lane == 0) {
-		// ---- MMA issuer
+	} else if (warp == 1) {
+		// ---- MMA issuer: all lanes wait, one issues
+		const uint32_t one = elect_one();
 		bool ok = mbar_wait(bready, 0, abort_flag, g.err, kErrTimeoutFull);
 		// Descriptors of strip slot 0, row 0 and of weight slice 0; every
 		// operand below is one of them plus a byte offset / 16 in the start
@@ -669,21 +638,21 @@ __global__ void __launch_bounds__(run_threads<T>(), 1)
 						const uint64_t ad = as + (uint32_t)dx * a_row, bd = bs + (uint32_t)dx * (B_TILE >> 4);
 #pragma unroll
 						for (int kk = 0; kk < T::KT / 16; ++kk)
-							mma_f16(acc, ad + 2 * kk, bd + 2 * kk, idesc, dy > 0 || dx > 0 || kk > 0);
+							mma_f16(one, acc, ad + 2 * kk, bd + 2 * kk, idesc, dy > 0 || dx > 0 || kk > 0);
 					}
 				}
 				if (!ok) break;
-				mma_commit(&empty[(q0 + (uint32_t)k) % STAGES]);  // the strip of row y0 + (k - 1) d: last read here
+				mma_commit(one, &empty[(q0 + (uint32_t)k) % STAGES]);  // the strip of row y0 + (k - 1) d: last read here
 				if (k == rows - 1) {
-					mma_commit(&empty[(q0 + (uint32_t)k + 1) % STAGES]);
-					mma_commit(&empty[(q0 + (uint32_t)k + 2) % STAGES]);
+					mma_commit(one, &empty[(q0 + (uint32_t)k + 1) % STAGES]);
+					mma_commit(one, &empty[(q0 + (uint32_t)k + 2) % STAGES]);
 				}
-				mma_commit(&accfull[a]);
+				mma_commit(one, &accfull[a]);
 			}
 			q0 += (uint32_t)(rows + 2);
 			s0 = s1;
 		}
-		mma_commit(drain);
+		mma_commit(one, drain);
 		volatile int own = 0;
 		mbar_wait(drain, 0, &own, g.err, kErrTimeoutAccum);
 	} else if (warp >= 2) {
@@ -867,7 +836,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 	uint64_t* drain = accempty + 2;
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
 	volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 	const int ntiles = P::ntiles(g);
 	const int nk = P::nk(g);
 	const int nchunk = (nk + kc - 1) / kc;
@@ -921,8 +890,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 			for (int s = 0; s < SPLIT_STAGES; ++s)
 				if (armed[s] >= 0) mbar_wait(&full[s], (uint32_t)armed[s] & 1, &own, g.err, kErrTimeoutFull);
 		}
-	} else if (warp == 1 && lane == 0) {
-		// ---- MMA issuer
+	} else if (warp == 1) {
+		// ---- MMA issuer: all lanes wait, one issues
+		const uint32_t one = elect_one();
 		uint32_t q = 0, cq = 0;
 		int i = 0;
 		bool ok = true;
@@ -954,20 +924,20 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 				const uint64_t dbh = desc_kmajor_sw128(sa + 2 * SPLIT_TILE), dbl = desc_kmajor_sw128(sa + 3 * SPLIT_TILE);
 #pragma unroll
 				for (int kk = 0; kk < BK / 16; ++kk) {
-					mma_f16(hacc, dah + 2 * kk, dbh + 2 * kk, idesc, !first || kk > 0);
-					mma_f16(cacc, dah + 2 * kk, dbl + 2 * kk, idesc, ks > 0 || kk > 0);
-					mma_f16(cacc, dal + 2 * kk, dbh + 2 * kk, idesc, true);
+					mma_f16(one, hacc, dah + 2 * kk, dbh + 2 * kk, idesc, !first || kk > 0);
+					mma_f16(one, cacc, dah + 2 * kk, dbl + 2 * kk, idesc, ks > 0 || kk > 0);
+					mma_f16(one, cacc, dal + 2 * kk, dbh + 2 * kk, idesc, true);
 				}
-				mma_commit(&empty[s]);
+				mma_commit(one, &empty[s]);
 				if (ks % kc == kc - 1 || ks == nk - 1) {
-					mma_commit(&hifull[cq & 1]);
+					mma_commit(one, &hifull[cq & 1]);
 					++cq;
 				}
 			}
 			if (!ok) break;
-			mma_commit(&accfull[a]);
+			mma_commit(one, &accfull[a]);
 		}
-		mma_commit(drain);
+		mma_commit(one, drain);
 		volatile int own = 0;
 		mbar_wait(drain, 0, &own, g.err, kErrTimeoutAccum);
 	} else if (warp >= 2) {
@@ -1369,8 +1339,7 @@ extern "C" umi_status umi_conv2d_fprop_f32_f16x3(const float* x_nhwc, const floa
 	}
 	UMI_TRY(map_kmajor(&maps.bh, wh, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, k, r * r * c, SPLIT_BN));
 	UMI_TRY(map_kmajor(&maps.bl, wl, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, k, r * r * c, SPLIT_BN));
-	ConvArgs g{out_nchw, n, c, h, w, k, r, umi::ceil_div(w, BM), umi::ceil_div(k, SPLIT_BN),
-	           umi::aligned(out_nchw, 16) && w % 4 == 0, err};
+	ConvArgs g{out_nchw, n, c, h, w, k, r, umi::ceil_div(w, BM), umi::ceil_div(k, SPLIT_BN), err};
 	if ((int64_t)n * h * g.xtiles * g.ktiles > INT32_MAX) return umi::fail(UMI_ERR_UNSUPPORTED, "conv_f16x3: too many tiles");
 	CUtensorMap unused;
 	std::memset(&unused, 0, sizeof(unused));
@@ -1403,8 +1372,7 @@ umi_status conv_launch(const void* x, const void* wt, float* out, int n, int c, 
 		if (rr != CUDA_SUCCESS) return umi::fail(UMI_ERR_CUDA, "conv: input tensor map (%d)", (int)rr);
 	}
 	UMI_TRY(map_kmajor(&tb, wt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, k, r * r * c, ConvPolicy::BN));
-	ConvArgs g{out, n, c, h, w, k, r, umi::ceil_div(w, BM), umi::ceil_div(k, ConvPolicy::BN),
-	           umi::aligned(out, 16) && w % 4 == 0, err};
+	ConvArgs g{out, n, c, h, w, k, r, umi::ceil_div(w, BM), umi::ceil_div(k, ConvPolicy::BN), err};
 	const int64_t tiles = (int64_t)n * h * g.xtiles * g.ktiles;
 	if (tiles > INT32_MAX) return umi::fail(UMI_ERR_UNSUPPORTED, "conv: too many tiles");
 	int grid = 0;
@@ -1481,7 +1449,7 @@ __global__ void __launch_bounds__(roll_threads(), 1)
 	uint64_t* bready = drain + 1;
 	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bready + 1);
 	volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 	const int H = g.h, ntiles = g.xtiles * H, d = g.dil;
 	const int t0 = blockIdx.x * per, t1 = min(ntiles, t0 + per);
 	auto segment = [&](int s0, int& blk, int& y0, int& s1) {
@@ -1552,9 +1520,10 @@ __global__ void __launch_bounds__(roll_threads(), 1)
 				if (armed[s] >= 0) mbar_wait(&full[s], (uint32_t)armed[s] & 1, &own, g.err, kErrTimeoutFull);
 			mbar_wait(bready, 0, &own, g.err, kErrTimeoutFull);
 		}
-	} else if (warp == 1 && lane == 0) {
-		// ---- MMA issuer: strip m of a run of `rows` output rows feeds rows
+	} else if (warp == 1) {
+		// ---- MMA issuer: all lanes wait, one issues; strip m of a run of `rows` output rows feeds rows
 		// m - dy for dy in [lo, hi] = [max(0, m - rows + 1), min(2, m)]
+		const uint32_t one = elect_one();
 		bool ok = mbar_wait(bready, 0, abort_flag, g.err, kErrTimeoutFull);
 		const uint64_t a_base = T::desc_a(smem_u32(base), 0), b_base = T::desc_b(smem_u32(bres));
 		const uint32_t a_row = (uint32_t)(d * T::ROW_BYTES) >> 4;
@@ -1591,17 +1560,17 @@ __global__ void __launch_bounds__(roll_threads(), 1)
 					const uint64_t bd = b_base + (uint32_t)(3 * dx + lo) * (B_TILE >> 4);
 #pragma unroll
 					for (int kk = 0; kk < T::KT / 16; ++kk) {
-						mma_f16(tmem + 32u * (uint32_t)first, ad + 2 * kk, bd + 2 * kk, id1, true);
-						if (c1 < cnt) mma_f16(tmem, ad + 2 * kk, bd + (uint32_t)c1 * (B_TILE >> 4) + 2 * kk, id2, true);
+						mma_f16(one, tmem + 32u * (uint32_t)first, ad + 2 * kk, bd + 2 * kk, id1, true);
+						if (c1 < cnt) mma_f16(one, tmem, ad + 2 * kk, bd + (uint32_t)c1 * (B_TILE >> 4) + 2 * kk, id2, true);
 					}
 				}
-				mma_commit(&empty[s]);                                      // the strip's only reader
-				if (m >= 2) mma_commit(&accfull[roll_slot(r0 + m - 2)]);  // row m - 2 has all nine taps
+				mma_commit(one, &empty[s]);                                      // the strip's only reader
+				if (m >= 2) mma_commit(one, &accfull[roll_slot(r0 + m - 2)]);  // row m - 2 has all nine taps
 			}
 			r0 += rows;
 			s0 = s1;
 		}
-		mma_commit(drain);
+		mma_commit(one, drain);
 		volatile int own = 0;
 		mbar_wait(drain, 0, &own, g.err, kErrTimeoutAccum);
 	} else if (warp >= 2) {

@@ -146,19 +146,38 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// One lane of a converged warp: 1 in the elected lane, 0 in the others.
+__device__ __forceinline__ uint32_t elect_one() {
+	uint32_t one;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(one));
+	return one;
+}
+
+// An MMA warp runs its loop with all lanes and the elected one issues
+// (`one`, as a predicate of the instruction).  Descriptors and loop state are
+// then warp-uniform to the compiler; under `if (lane == 0)` each MMA took
+// about 67 clocks to issue, more than a 128 x 128 x 16 MMA takes to run
+// (a 3x3 convolution's MMAs with its stores left out: 60 -> 45 us).
+
 // D[tmem] (+)= A[smem] * B[smem]^T, kind::f16 (bf16 or f16 inputs, fp32 accumulate).
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, bool accumulate) {
+__device__ __forceinline__ void mma_f16(uint32_t one, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                        bool accumulate) {
 	asm volatile(
-		"{\n\t.reg .pred p;\n\t"
+		"{\n\t.reg .pred p, q;\n\t"
 		"setp.ne.b32 p, %4, 0;\n\t"
-		"tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-		"l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate)
+		"setp.ne.b32 q, %5, 0;\n\t"
+		"@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+		"l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate), "r"(one)
 		: "memory");
 }
-// Arrive on `bar` once every tcgen05 operation issued so far by this thread has completed.
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-	asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-	             : "memory");
+// Arrive on `bar` once every tcgen05 operation issued so far by the elected lane has completed.
+__device__ __forceinline__ void mma_commit(uint32_t one, uint64_t* bar) {
+	asm volatile(
+		"{\n\t.reg .pred q;\n\t"
+		"setp.ne.b32 q, %1, 0;\n\t"
+		"@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
+		"r"(one)
+		: "memory");
 }
 
 // Zero into 32 consecutive columns of the warp's 32 TMEM lanes, and the wait
