@@ -174,3 +174,29 @@ def test_gemm_epilogue_wait_times_out_and_context_stays_usable(umi, orc, dev):
     a, b = A[rows].float().cpu().numpy(), B.float().cpu().numpy()
     _check(C[rows].cpu().numpy(), orc.gemm_f64(a, b, b_is_nk=True), orc.gemm_f64(np.abs(a), np.abs(b), b_is_nk=True),
            1e-5)
+
+
+@pytest.mark.parametrize("n,c,h,w,k,r", [(2, 64, 3, 64, 128, 3), (2, 64, 3, 65, 128, 3), (1, 64, 5, 63, 40, 3),
+                                         (2, 128, 10, 43, 130, 5), (3, 64, 7, 7, 64, 1), (1, 64, 130, 1, 16, 3),
+                                         (1, 128, 64, 2, 128, 7), (2, 64, 4, 32, 129, 3),
+                                         (4, 64, 40, 42, 128, 3), (40, 64, 4, 5, 96, 3)])
+def test_conv2d_fprop_packed_rows(umi, orc, dev, n, c, h, w, k, r):
+    """Widths up to 64 pack whole image rows into a tile; the last tile of an
+    image is partly empty, rows straddle the filter's padding on both sides."""
+    import torch
+    x, wt = _conv_case(n, c, h, w, k, r, n * 1000 + h * 10 + k + w)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    xd, wd = x.permute(0, 2, 3, 1).contiguous().to(dev), wt.permute(0, 2, 3, 1).contiguous().to(dev)
+    out = torch.full((n * k * h * w + 9,), -7.0, device=dev)
+    # an output that starts one word past a 16-byte boundary, and nothing written around it
+    o = out[5:5 + n * k * h * w].view(n, k, h, w)
+    got = umi.conv2d_fprop_bf16(xd, wd, out=o, err=err).cpu().numpy()
+    assert int(err.item()) == 0
+    assert (out[:5] == -7.0).all() and (out[5 + n * k * h * w:] == -7.0).all()
+    xf, wf = x.float().numpy(), wt.float().numpy()
+    want = orc.conv2d_f64(xf, wf, 1, r // 2)
+    scale = orc.conv2d_f64(np.abs(xf), np.abs(wf), 1, r // 2)
+    _check(got, want, scale, 1e-5)
+    split = umi.conv2d_fprop_f32_f16x3(xd.float(), wd.float(), err=err).cpu().numpy()
+    assert int(err.item()) == 0
+    _check(split, want, scale, 2e-6)  # the bound of the split product's own tests

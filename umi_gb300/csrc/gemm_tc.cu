@@ -64,6 +64,7 @@ struct GemmPolicyT {
 		return {(id / nt) * BM, (id % nt) * BN};
 	}
 	__device__ static int nk(const Args& g) { return (g.K + BK - 1) / BK; }
+	__device__ static uint32_t a_bytes(const Args&) { return BM * BK * 2; }
 	__device__ static void load(const CUtensorMap* ta, const CUtensorMap* tb, const Args&, const Tile& t, int ks,
 	                            void* a, void* b, uint64_t* bar) {
 		tma_load_2d(a, ta, bar, ks * BK, t.m0);
@@ -97,15 +98,21 @@ __host__ __device__ constexpr uint32_t tmem_cols_for(int bn) {
 }
 
 // 2-D convolution, stride 1, zero padding r/2, as an implicit GEMM:
-// rows = 128 output pixels of one image row (n, y, x0..x0+127), columns =
-// output channels, K = (tap, input-channel slice of 64).  A slice is one TMA
-// box of the NHWC input at (c0, x0+dx-pad, y+dy-pad, n): the box's
-// out-of-bounds zero fill is the padding.  B slices come from the KRSC
-// weights viewed as (k, r*r*c).  Output NCHW fp32.
+// rows = bw x bh output pixels of one image, columns = output channels, K =
+// (tap, input-channel slice of 64).  A slice is one TMA box of the NHWC input
+// at (c0, x0+dx-pad, y0+dy-pad, n): the box's out-of-bounds zero fill is the
+// padding.  B slices come from the KRSC weights viewed as (k, r*r*c).  Output
+// NCHW fp32: a tile's pixels are one contiguous piece of each output plane.
+//
+// The box is 128 pixels of one row, or, where at least two rows of the image
+// fit (w <= 64), bw = w and bh = 128 / w whole rows: one row a tile would
+// multiply 128 - w rows of padding.
+// Measured, here and with one row a tile: 16 images of 14 x 14, 128 to 256
+// channels, 3x3 9.9 against 22.0 us; 8 of 64 x 64, 128 to 128 17.1 against 28.1.
 struct ConvArgs {
 	float* out;
 	int n, c, h, w, k, r;
-	int xtiles, ktiles;
+	int bw, bh, xtiles, ytiles, ktiles;
 	int* err;
 };
 struct ConvPolicy {
@@ -115,14 +122,19 @@ struct ConvPolicy {
 	static constexpr bool EPI_TMA = false;
 	template <class A> __device__ static unsigned long long acc_wait_ns(const A&) { return kWaitNs; }
 	using Args = ConvArgs;
-	struct Tile { int n, y, x0, k0; };
-	// tile id = ((n*h + y)*xtiles + xt)*ktiles + kt
-	__host__ __device__ static int ntiles(const Args& g) { return g.n * g.h * g.xtiles * g.ktiles; }
+	struct Tile {
+		int n, y, x0, k0;
+		int npix;  // pixels of the box inside the image: contiguous from (y, x0)
+	};
+	// tile id = ((n*ytiles + yt)*xtiles + xt)*ktiles + kt
+	__host__ __device__ static int ntiles(const Args& g) { return g.n * g.ytiles * g.xtiles * g.ktiles; }
 	__device__ static Tile tile(const Args& g, int id) {
 		const int kt = id % g.ktiles, b = id / g.ktiles;
 		const int xt = b % g.xtiles, rest = b / g.xtiles;
-		return {rest / g.h, rest % g.h, xt * BM, kt * BN};
+		const int n = rest / g.ytiles, y = (rest - n * g.ytiles) * g.bh, x0 = xt * g.bw;
+		return {n, y, x0, kt * BN, min(g.bh, g.h - y) * min(g.bw, g.w - x0)};
 	}
+	__device__ static uint32_t a_bytes(const Args& g) { return (uint32_t)(g.bw * g.bh) * BK * 2; }
 	__device__ static int nk(const Args& g) { return g.r * g.r * (g.c / BK); }
 	__device__ static void load(const CUtensorMap* ta, const CUtensorMap* tb, const Args& g, const Tile& t, int ks,
 	                            void* a, void* b, uint64_t* bar) {
@@ -144,17 +156,17 @@ struct ConvPolicy {
 		const int tap = ks / cs, c0 = (ks - tap * cs) * BK;
 		tma_load_2d(b, tb, bar, tap * g.c + c0, 0);
 	}
-	// This thread holds pixel x0 + rl of the tile for output channels
+	// This thread holds pixel rl of the tile for output channels
 	// [k0+c, +32): a warp's store of one channel is 32 consecutive pixels, one
 	// 128-byte line where the row starts on one.  Transposing 4 x 4 blocks
 	// across lanes for 16-byte stores (32 shuffles per thread and 32 channels)
 	// took 1900 clocks a pass against 800 to 1000 for these, as the shuffles
 	// share the shared-memory pipe with the MMAs' operand reads.
 	__device__ static void store(const Args& g, const Tile& t, int rl, int c, const float (&v)[32]) {
-		const int x = t.x0 + rl, left = g.k - t.k0 - c;
-		if (x >= g.w) return;
+		const int left = g.k - t.k0 - c;
+		if (rl >= t.npix) return;
 		const size_t plane = (size_t)g.h * g.w;
-		float* dst = g.out + ((size_t)t.n * g.k + t.k0 + c) * plane + (size_t)t.y * g.w + x;
+		float* dst = g.out + ((size_t)t.n * g.k + t.k0 + c) * plane + (size_t)t.y * g.w + t.x0 + rl;
 		if (left >= 32) {
 #pragma unroll
 			for (int j = 0; j < 32; ++j, dst += plane) *dst = v[j];
@@ -216,7 +228,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 	constexpr int BN = P::BN, STAGES = P::STAGES;
 	constexpr bool RES = P::RESIDENT_B;
 	constexpr uint32_t A_TILE = BM * BK * 2, B_TILE = BN * BK * 2;
-	constexpr uint32_t STAGE_BYTES = RES ? A_TILE : A_TILE + B_TILE;  // bytes one ring load brings
+	constexpr uint32_t STAGE_BYTES = RES ? A_TILE : A_TILE + B_TILE;
 	extern __shared__ uint8_t smem_raw[];
 	// 1024-byte aligned start (128-byte swizzled TMA tiles), formed by indexing
 	// the shared array so that the compiler keeps shared-memory accesses
@@ -269,13 +281,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 			for (int ks = 0; ks < nk; ++ks) P::load_b(&tb, g, ks, bres + ks * B_TILE, bready);
 		}
 		uint32_t q = 0;  // slices issued by this CTA
+		const uint32_t load_bytes = RES ? P::a_bytes(g) : P::a_bytes(g) + B_TILE;  // what one ring load brings
 		for (int id = blockIdx.x; id < ntiles && !*abort_flag; id += gridDim.x) {
 			const typename P::Tile t = P::tile(g, id);
 			for (int ks = 0; ks < nk; ++ks, ++q) {
 				const int s = (int)(q % STAGES);
 				const uint32_t round = q / STAGES;
 				if (!mbar_wait(&empty[s], (round & 1) ^ 1, abort_flag, g.err, kErrTimeoutEmpty)) break;
-				mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
+				mbar_arrive_expect_tx(&full[s], load_bytes);
 				armed[s] = (int)round;
 				if constexpr (RES)
 					P::load_a(&ta, g, t, ks, base + s * STAGE_BYTES, &full[s]);
@@ -439,6 +452,7 @@ struct ConvRun {
 		t.y = y;
 		t.x0 = (blk - t.n * g.xtiles) * BM;
 		t.k0 = 0;
+		t.npix = min(BM, g.w - t.x0);
 		ConvPolicy::store(g, t, rl, c, v);
 	}
 	struct Epi {
@@ -785,6 +799,7 @@ struct GemmSplitPolicy {
 		return {(first_m + r % gsz) * BM, (r / gsz) * SPLIT_BN};
 	}
 	__device__ static int nk(const Args& g) { return (g.K + BK - 1) / BK; }
+	__device__ static uint32_t a_bytes(const Args&) { return SPLIT_TILE; }
 	__device__ static void load4(const SplitMaps& m, const Args&, const Tile& t, int ks, uint8_t* dst, uint64_t* bar) {
 		tma_load_2d(dst, &m.ah, bar, ks * BK, t.m0);
 		tma_load_2d(dst + SPLIT_TILE, &m.al, bar, ks * BK, t.m0);
@@ -796,7 +811,7 @@ struct GemmSplitPolicy {
 	}
 };
 
-// The convolution (ConvPolicy's tiles: 128 pixels of a row x 128 output
+// The convolution (ConvPolicy's tiles: up to 128 pixels x 128 output
 // channels, K-slices (tap, 64 input channels)) with split operands.
 struct ConvSplitPolicy {
 	static constexpr bool EPI_TMA = false;
@@ -806,6 +821,7 @@ struct ConvSplitPolicy {
 	__host__ __device__ static int ntiles(const Args& g) { return ConvPolicy::ntiles(g); }
 	__device__ static Tile tile(const Args& g, int id) { return ConvPolicy::tile(g, id); }
 	__device__ static int nk(const Args& g) { return ConvPolicy::nk(g); }
+	__device__ static uint32_t a_bytes(const Args& g) { return ConvPolicy::a_bytes(g); }
 	__device__ static void load4(const SplitMaps& m, const Args& g, const Tile& t, int ks, uint8_t* dst, uint64_t* bar) {
 		const int cs = g.c / BK;
 		const int tap = ks / cs, c0 = (ks - tap * cs) * BK;
@@ -874,13 +890,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 		int armed[SPLIT_STAGES];
 		for (int s = 0; s < SPLIT_STAGES; ++s) armed[s] = -1;
 		uint32_t q = 0;
+		const uint32_t load_bytes = 2 * (P::a_bytes(g) + SPLIT_TILE);
 		for (int id = blockIdx.x; id < ntiles && !*abort_flag; id += gridDim.x) {
 			const typename P::Tile t = P::tile(g, id);
 			for (int ks = 0; ks < nk; ++ks, ++q) {
 				const int s = (int)(q % SPLIT_STAGES);
 				const uint32_t round = q / SPLIT_STAGES;
 				if (!mbar_wait(&empty[s], (round & 1) ^ 1, abort_flag, g.err, kErrTimeoutEmpty)) break;
-				mbar_arrive_expect_tx(&full[s], SPLIT_STAGE);
+				mbar_arrive_expect_tx(&full[s], load_bytes);
 				armed[s] = (int)round;
 				P::load4(maps, g, t, ks, base + s * SPLIT_STAGE, &full[s]);
 			}
@@ -1233,6 +1250,15 @@ umi_status check_chunk(int32_t chunk, int* kc) {
 	return UMI_OK;
 }
 
+ConvArgs conv_args(float* out, int n, int c, int h, int w, int k, int r, int* err, bool pack = true) {
+	int bw = BM, bh = 1;
+	if (pack && 2 * w <= BM) {
+		bw = w;
+		bh = std::min(h, BM / w);
+	}
+	return {out, n, c, h, w, k, r, bw, bh, umi::ceil_div(w, bw), umi::ceil_div(h, bh), umi::ceil_div(k, ConvPolicy::BN), err};
+}
+
 }  // namespace
 
 extern "C" size_t umi_gemm_f32_f16x3_workspace_bytes(int32_t M, int32_t N, int32_t K) {
@@ -1326,11 +1352,12 @@ extern "C" umi_status umi_conv2d_fprop_f32_f16x3(const float* x_nhwc, const floa
 	__half* wl = reinterpret_cast<__half*>(ws + 2 * al256(nx * 2) + al256(nw * 2));
 	UMI_TRY(split_operand(x_nhwc, nx, xh, xl, st));
 	UMI_TRY(split_operand(w_krsc, nw, wh, wl, st));
+	const ConvArgs g = conv_args(out_nchw, n, c, h, w, k, r, err);
 	SplitMaps maps;
 	for (int part = 0; part < 2; ++part) {
 		const cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
 		const cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
-		const cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)BM, 1, 1};
+		const cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)g.bw, (cuuint32_t)g.bh, 1};
 		const cuuint32_t es[4] = {1, 1, 1, 1};
 		const CUresult rr = enc(part ? &maps.al : &maps.ah, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, part ? xl : xh, dims,
 		                        strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1339,7 +1366,6 @@ extern "C" umi_status umi_conv2d_fprop_f32_f16x3(const float* x_nhwc, const floa
 	}
 	UMI_TRY(map_kmajor(&maps.bh, wh, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, k, r * r * c, SPLIT_BN));
 	UMI_TRY(map_kmajor(&maps.bl, wl, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, k, r * r * c, SPLIT_BN));
-	ConvArgs g{out_nchw, n, c, h, w, k, r, umi::ceil_div(w, BM), umi::ceil_div(k, SPLIT_BN), err};
 	if ((int64_t)n * h * g.xtiles * g.ktiles > INT32_MAX) return umi::fail(UMI_ERR_UNSUPPORTED, "conv_f16x3: too many tiles");
 	CUtensorMap unused;
 	std::memset(&unused, 0, sizeof(unused));
@@ -1360,11 +1386,20 @@ umi_status conv_launch(const void* x, const void* wt, float* out, int n, int c, 
 	auto enc = encode_fn();
 	if (!enc) return umi::fail(UMI_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
 	CUtensorMap ta, tb;
-	const bool strip = r == 3 && c == BK && k <= ConvStripPolicy::BN;
+	// The strip form loads a third of the operand bytes and starts sooner; packed
+	// rows cut the MMAs.  Two rows a tile do not pay for the strips' saving (57 x
+	// 57, 8 images: 8.8 us in strips, 10.7 packed; 32 images of 64 x 64: 25.8 and
+	// 25.5), three or more do once there are more rows than SMs (28 x 28: 32
+	// images 13.0 and 10.3, 128 images 37.4 and 21.6; one image 5.6 and 7.2).
+	int dev = 0, sms = 0;
+	UMI_TRY(umi::cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
+	UMI_TRY(umi::cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"));
+	const bool strip = r == 3 && c == BK && k <= ConvStripPolicy::BN && (3 * w > BM || (int64_t)n * h <= sms);
+	const ConvArgs g = conv_args(out, n, c, h, w, k, r, err, !strip);
 	{
 		const cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
 		const cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
-		const cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)(strip ? ConvStripPolicy::STRIP_ROWS : BM), 1, 1};
+		const cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)(strip ? ConvStripPolicy::STRIP_ROWS : g.bw), (cuuint32_t)g.bh, 1};
 		const cuuint32_t es[4] = {1, 1, 1, 1};
 		const CUresult rr = enc(&ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), dims, strides, box, es,
 		                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1372,9 +1407,8 @@ umi_status conv_launch(const void* x, const void* wt, float* out, int n, int c, 
 		if (rr != CUDA_SUCCESS) return umi::fail(UMI_ERR_CUDA, "conv: input tensor map (%d)", (int)rr);
 	}
 	UMI_TRY(map_kmajor(&tb, wt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, k, r * r * c, ConvPolicy::BN));
-	ConvArgs g{out, n, c, h, w, k, r, umi::ceil_div(w, BM), umi::ceil_div(k, ConvPolicy::BN), err};
-	const int64_t tiles = (int64_t)n * h * g.xtiles * g.ktiles;
-	if (tiles > INT32_MAX) return umi::fail(UMI_ERR_UNSUPPORTED, "conv: too many tiles");
+	if ((int64_t)n * h * g.xtiles * g.ktiles > INT32_MAX) return umi::fail(UMI_ERR_UNSUPPORTED, "conv: too many tiles");
+	const int64_t tiles = ConvPolicy::ntiles(g);
 	int grid = 0;
 	if (strip)  // k <= BN: one output-channel block; runs of output rows, each input row's strip loaded once per run
 		return launch_strip_run<ConvRun>(ta, tb, g, tiles, st, "strip_run_kernel<conv>");
