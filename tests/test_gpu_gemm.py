@@ -200,3 +200,25 @@ def test_conv2d_fprop_packed_rows(umi, orc, dev, n, c, h, w, k, r):
     split = umi.conv2d_fprop_f32_f16x3(xd.float(), wd.float(), err=err).cpu().numpy()
     assert int(err.item()) == 0
     _check(split, want, scale, 2e-6)  # the bound of the split product's own tests
+
+
+# One size for each tile the launcher chooses (one-CTA tiles of 64 to 256
+# columns, pairs of CTAs of 128 to 256), with ragged last tiles in M and N, an
+# odd N (no TMA stores) and a K that is not a multiple of the 64-wide slice.
+@pytest.mark.parametrize("M,N,K", [(65, 63, 8), (1100, 1025, 136), (2300, 1025, 520), (2040, 2047, 1024),
+                                   (2048, 1025, 1032), (1001, 1540, 2056), (1500, 2500, 520), (2049, 2051, 520),
+                                   (2305, 2049, 1032)])
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+def test_gemm_tile_choices(umi, orc, dev, M, N, K, dt):
+    import torch
+    g = torch.Generator(device="cpu").manual_seed(M + 3 * N + K)
+    tdt = torch.bfloat16 if dt == "bf16" else torch.float16
+    A = torch.randn(M, K, generator=g).to(tdt)
+    B = torch.randn(N, K, generator=g).to(tdt)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    flat = torch.full((M * N + 64,), -7.0, device=dev)
+    C = umi.gemm(A.to(dev), B.to(dev), out=flat[:M * N].view(M, N), err=err).cpu().numpy()
+    assert int(err.item()) == 0
+    assert (flat[M * N:] == -7.0).all()
+    assert np.isfinite(C).all()
+    _sampled_rows_cols(orc, A.float().numpy(), B.float().numpy(), C, 1e-5, nsample=min(32, M, N))

@@ -5,12 +5,13 @@
 // main/gemm.cu:8-15: accum += A * B through shared memory, scalar) for the
 // half-precision operand types, plus a split-precision FP32 emulation.
 //
-// Persistent CTAs compute 128 x 256 tiles of C:
-//   warp 0, one lane  : TMA producer, K-slices of 64 into a 4-stage ring
-//                       (A 16 KB + B 32 KB per stage, 128-byte swizzle);
-//   warp 1            : allocates 512 TMEM columns (two accumulators); one
-//                       lane issues the tcgen05.mma (M=128, N=256, K=16, 4 per
-//                       slice) and commits each slice back to the producer;
+// Persistent CTAs, or pairs of CTAs (tc_pair_kernel), compute tiles of C up to
+// 128 (256) rows by 256 columns:
+//   warp 0, one lane  : TMA producer, K-slices of 64 into a ring (128-byte
+//                       swizzle);
+//   warp 1            : allocates TMEM (two accumulators); one lane issues the
+//                       tcgen05.mma (K=16, 4 per slice) and commits each slice
+//                       back to the producer;
 //   warps 2..5        : epilogue, tcgen05.ld of their 32 TMEM lanes (rows),
 //                       fp32 stores, overlapping the next tile's MMAs.
 // All mbarrier waits are bounded (tc_common.cuh); on timeout the kernel
@@ -45,11 +46,11 @@ struct GemmArgs {
 	unsigned long long acc_wait_ns;  // limit of the epilogue's wait for a finished accumulator (kWaitNs)
 };
 
-// C[M,N] = A[M,K] B[N,K]^T: grid (N/BN, M/BM).  BN = 256, or 224 where it
-// fills the last round of persistent tiles better (gemm_launch chooses).
+// C[M,N] = A[M,K] B[N,K]^T in tiles of 128 x BN, BN = 256, 224, 128 or 64
+// (gemm_launch chooses).
 template <int BN_>
 struct GemmPolicyT {
-	static constexpr int BN = BN_, STAGES = 4;
+	static constexpr int BN = BN_, STAGES = BN_ > 128 ? 4 : 6;
 	static constexpr bool RESIDENT_B = false;
 	static constexpr int NK_RES = 0;
 	static constexpr bool EPI_TMA = true;  // epilogue through shared memory + TMA tile stores
@@ -70,24 +71,42 @@ struct GemmPolicyT {
 		tma_load_2d(a, ta, bar, ks * BK, t.m0);
 		tma_load_2d(b, tb, bar, ks * BK, t.n0);
 	}
-	// this thread's row of the tile, columns [c, c+32)
-	__device__ static void store(const Args& g, const Tile& t, int rl, int c, const float (&v)[32]) {
-		const int row = t.m0 + rl;
-		if (row >= g.M) return;
-		float* dst = g.C + (size_t)row * g.ldc + t.n0 + c;
-		if (g.vec && t.n0 + c + 31 < g.N) {
+};
+using GemmPolicy = GemmPolicyT<128>;
+
+// A warp's 32 x 32 block of C at (row0, col0), lane l holding row l: through
+// the 4 KB buffer sb in the 128-byte swizzle of the C tensor map (chunk j of
+// row r at j ^ (r & 7): conflict-free both ways).  Where C takes TMA stores
+// (g.vec) one store writes the block, clipped at the edges; otherwise the warp
+// writes one row after the other, 32 consecutive words each (a lane storing its
+// own row word by word touched 32 lines with every store: 1234 x 3001, K = 800
+// took 27.8 us, now 11.5).
+__device__ __forceinline__ void store_block(const GemmArgs& g, const CUtensorMap* tcm, uint8_t* sb, int row0, int col0,
+                                            const float (&v)[32], int lane) {
+	if (g.vec && lane == 0) bulk_wait_read_1();  // the store that last used sb (two blocks ago) has read it
+	__syncwarp();
 #pragma unroll
-			for (int i = 0; i < 32; i += 4)
-				*reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-		} else {
-#pragma unroll
-			for (int i = 0; i < 32; ++i)
-				if (t.n0 + c + i < g.N) dst[i] = v[i];
+	for (int j = 0; j < 8; ++j)
+		*reinterpret_cast<float4*>(sb + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+			make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+	if (g.vec) {
+		fence_proxy_async_smem();
+		__syncwarp();
+		if (lane == 0) {
+			tma_store_2d(tcm, sb, col0, row0);
+			bulk_commit();
+		}
+	} else {
+		__syncwarp();
+		const int rows = min(32, g.M - row0);
+		if (col0 + lane < g.N) {
+			float* dst = g.C + (size_t)row0 * g.ldc + col0 + lane;
+#pragma unroll 8
+			for (int r = 0; r < rows; ++r, dst += g.ldc)
+				*dst = *reinterpret_cast<const float*>(sb + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
 		}
 	}
-};
-using GemmPolicy = GemmPolicyT<256>;
-using GemmPolicy224 = GemmPolicyT<224>;
+}
 
 // TMEM columns of two accumulators of BN columns: the allocation unit is a
 // power of two of at least 32 columns.
@@ -340,7 +359,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 		// ---- epilogue: warp w reads TMEM lanes 32*(w%4) .. +31 (rows of the tile)
 		const int qd = warp & 3;
 		int i = 0;
-		uint32_t nst = 0;  // TMA stores issued by this warp
+		uint32_t nst = 0;  // blocks stored by this warp
 		for (int id = blockIdx.x; id < ntiles; id += gridDim.x, ++i) {
 			const int a = i & 1;
 			const uint32_t use = (uint32_t)(i >> 1);
@@ -352,39 +371,19 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 				float v[32];
 				tmem_ld32(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(a * BN + c), v);
 				if constexpr (P::EPI_TMA) {
-					if (g.vec) {
-						// 32 rows x 32 columns through a 4 KB buffer with the 128-byte
-						// swizzle of the C tensor map (chunk j of row r at j ^ (r & 7):
-						// conflict-free), then one TMA store; out-of-range rows and
-						// columns are clipped by the TMA.
-						const int row0 = t.m0 + 32 * qd, col0 = t.n0 + c;
-						if (row0 < g.M && col0 < g.N) {
-							uint8_t* sb = ebuf + (qd * 2 + (nst & 1)) * 4096;
-							if (lane == 0) bulk_wait_read_1();  // the store that last used sb has read it
-							__syncwarp();
-#pragma unroll
-							for (int j = 0; j < 8; ++j)
-								*reinterpret_cast<float4*>(sb + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-									make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-							fence_proxy_async_smem();
-							__syncwarp();
-							if (lane == 0) {
-								tma_store_2d(&tcm, sb, col0, row0);
-								bulk_commit();
-							}
-							++nst;
-						}
-						continue;
-					}
+					const int row0 = t.m0 + 32 * qd, col0 = t.n0 + c;
+					if (row0 < g.M && col0 < g.N)
+						store_block(g, &tcm, ebuf + (qd * 2 + (nst++ & 1)) * 4096, row0, col0, v, lane);
+				} else {
+					P::store(g, t, 32 * qd + lane, c, v);
 				}
-				P::store(g, t, 32 * qd + lane, c, v);
 			}
 			tc_fence_before();
 			__syncwarp();
 			if (lane == 0) mbar_arrive(&accempty[a]);
 		}
 		if constexpr (P::EPI_TMA) {
-			if (lane == 0) bulk_wait_all();  // stores done before the CTA exits
+			if (lane == 0) bulk_wait_read_all();  // the staging buffers are read before the CTA exits
 			__syncwarp();
 		}
 	}
@@ -394,6 +393,184 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 		tc_fence_after();
 		tmem_dealloc(tmem, tmem_cols_for(BN));
 	}
+}
+
+// C[M,N] = A[M,K] B[N,K]^T by pairs of CTAs (clusters of two, cta_group::2):
+// 256 x BN tiles, CTA r of the pair holding rows 128 r .. + 127 of the A slice
+// and of the accumulator and BN / 2 rows of the B slice.  Roles, ring,
+// accumulators and epilogue are tc_kernel's, with these differences:
+//   both producers load into their own CTA and complete on the even CTA's
+//   `full` barrier, which expects the bytes of both; the even CTA's MMA warp
+//   issues for the pair and its commits arrive in both CTAs; the epilogue
+//   warps of both release an accumulator on the even CTA's `accempty`.
+// A role that gives up raises both CTAs' abort flags.  The producers then load
+// whatever slices the other one has already begun, so that every `full` phase
+// completes and the even CTA can wait for all copies in flight.
+//
+// What bounds the one-CTA form at 4096^3 is the operands' way from L2: a K
+// step of 16 brings 11 KB (128 x 224) and takes 55 ns where one tile runs alone
+// but 86 on all SMs.  In a pair each CTA holds half of B, 7.5 KB: 74 ns on all
+// SMs, 4096^3 in 80 us against 87.5 (graph replays; 101 -> 92 from the host).
+// From there on the GPU's power limit binds: 8192 x 8192 x 4096 runs at 1660
+// TFLOP/s (369.8 -> 331.4 us) where long cuBLAS runs settle at 1702.
+template <int BN_>
+struct GemmPairT {
+	static constexpr int BN = BN_;
+	static constexpr uint32_t A_TILE = BM * BK * 2, B_TILE = (BN / 2) * BK * 2;
+	static constexpr uint32_t STAGE = A_TILE + B_TILE;
+	static constexpr int STAGES = 6;
+	static constexpr size_t SMEM = (size_t)STAGES * STAGE + 8 * 4096 + 1024 + 256;
+	static_assert(SMEM <= 227 * 1024 && B_TILE % 1024 == 0 && BN % 32 == 0, "fits; whole swizzle atoms and 32-column loads");
+};
+
+template <int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
+	tc_pair_kernel(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb,
+	               const __grid_constant__ CUtensorMap tcm, const GemmArgs g, const uint32_t idesc) {
+	using P = GemmPairT<BN>;
+	constexpr int STAGES = P::STAGES;
+	extern __shared__ uint8_t smem_raw[];
+	uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+	uint8_t* ebuf = base + STAGES * P::STAGE;  // epilogue staging, 2 x 4 KB per epilogue warp
+	uint64_t* full = reinterpret_cast<uint64_t*>(ebuf + 8 * 4096);  // the even CTA's are used
+	uint64_t* empty = full + STAGES;
+	uint64_t* accfull = empty + STAGES;  // [2]
+	uint64_t* accempty = accfull + 2;    // [2], the even CTA's are used
+	uint64_t* drain = accempty + 2;
+	uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+	volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+	uint32_t* issued = tmem_slot + 2;  // [2]: slices issued by CTA 0, 1 (both CTAs hold both)
+	const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+	const uint32_t rank = cluster_rank();
+	const int nt = (g.N + BN - 1) / BN, ntiles = ((g.M + 2 * BM - 1) / (2 * BM)) * nt;
+	const int nk = (g.K + BK - 1) / BK;
+	const int pair0 = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+
+	if (threadIdx.x == 0) {
+		for (int s = 0; s < STAGES; ++s) {
+			mbar_init(&full[s], 1);
+			mbar_init(&empty[s], 1);
+		}
+		for (int a = 0; a < 2; ++a) {
+			mbar_init(&accfull[a], 1);
+			mbar_init(&accempty[a], 8);  // one arrive per epilogue warp of the pair
+		}
+		mbar_init(drain, 1);
+		*abort_flag = 0;
+		fence_mbar_init();
+		tma_prefetch(&ta);
+		tma_prefetch(&tb);
+	}
+	if (warp == 1) tmem_alloc_pair(tmem_slot, tmem_cols_for(BN));
+	__syncwarp();
+	tc_fence_before();
+	cluster_sync();  // both CTAs' barriers are initialised
+	tc_fence_after();
+	const uint32_t tmem = *tmem_slot;
+
+	auto load = [&](uint32_t n, int m0, int n0, int ks) {  // slice n of this CTA's halves
+		const int s = (int)(n % STAGES);
+		if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * P::STAGE);
+		const uint32_t bar = cluster_addr(&full[s], 0);
+		tma_load_2d_pair(base + s * P::STAGE, &ta, bar, ks * BK, m0);
+		tma_load_2d_pair(base + s * P::STAGE + P::A_TILE, &tb, bar, ks * BK, n0);
+	};
+	if (warp == 0 && lane == 0) {
+		// ---- producer
+		uint32_t q = 0;  // slices issued by this CTA
+		for (int id = pair0; id < ntiles && !*abort_flag; id += npairs) {
+			const int m0 = (id / nt) * 2 * BM + (int)rank * BM, n0 = (id % nt) * BN + (int)rank * (BN / 2);
+			for (int ks = 0; ks < nk; ++ks, ++q) {
+				const int s = (int)(q % STAGES);
+				if (!mbar_wait(&empty[s], ((q / STAGES) & 1) ^ 1, abort_flag, g.err, kErrTimeoutEmpty)) break;
+				load(q, m0, n0, ks);
+			}
+		}
+		issued[rank] = q;
+		st_cluster_u32(cluster_addr(&issued[rank], rank ^ 1u), q);
+		// every commit that arrives in this CTA has arrived before it exits
+		for (uint32_t n = q > STAGES ? q - STAGES : 0; n < q; ++n)
+			if (!mbar_wait(&empty[n % STAGES], (n / STAGES) & 1, abort_flag, g.err, kErrTimeoutEmpty)) break;
+	} else if (warp == 1 && rank == 0) {
+		// ---- MMA issuer of the pair: all lanes wait, one issues
+		const uint32_t one = elect_one();
+		uint32_t q = 0;
+		int i = 0;  // local tile count
+		for (int id = pair0; id < ntiles && !*abort_flag; id += npairs, ++i) {
+			const int a = i & 1;
+			if (!mbar_wait(&accempty[a], ((uint32_t)(i >> 1) & 1) ^ 1, abort_flag, g.err, kErrTimeoutAccEmpty)) break;
+			tc_fence_after();
+			const uint32_t acc = tmem + (uint32_t)(a * BN);
+			bool ok = true;
+			for (int ks = 0; ks < nk; ++ks, ++q) {
+				const int s = (int)(q % STAGES);
+				if (!mbar_wait(&full[s], (q / STAGES) & 1, abort_flag, g.err, kErrTimeoutFull)) { ok = false; break; }
+				tc_fence_after();
+				const uint64_t ad = desc_kmajor_sw128(smem_u32(base + s * P::STAGE));
+				const uint64_t bd = desc_kmajor_sw128(smem_u32(base + s * P::STAGE + P::A_TILE));
+#pragma unroll
+				for (int kk = 0; kk < BK / 16; ++kk)
+					mma_f16_pair(one, acc, ad + 2 * kk, bd + 2 * kk, idesc, ks > 0 || kk > 0);
+				mma_commit_pair(one, &empty[s]);
+			}
+			if (!ok) break;
+			mma_commit_pair(one, &accfull[a]);
+		}
+		// every MMA issued above finishes before TMEM is freed
+		mma_commit_pair(one, drain);
+		volatile int own = 0;
+		mbar_wait(drain, 0, &own, g.err, kErrTimeoutAccum);
+	} else if (warp >= 2) {
+		// ---- epilogue: warp w reads TMEM lanes 32*(w%4) .. +31 (rows of this CTA's half)
+		const int qd = warp & 3;
+		int i = 0;
+		uint32_t nst = 0;  // blocks stored by this warp
+		for (int id = pair0; id < ntiles; id += npairs, ++i) {
+			const int a = i & 1;
+			if (!mbar_wait(&accfull[a], (uint32_t)(i >> 1) & 1, abort_flag, g.err, kErrTimeoutAccum, g.acc_wait_ns)) break;
+			tc_fence_after();
+			const int row0 = (id / nt) * 2 * BM + (int)rank * BM + 32 * qd, n0 = (id % nt) * BN;
+#pragma unroll 1
+			for (int c = 0; c < BN; c += 32) {
+				const int col0 = n0 + c;
+				if (row0 >= g.M || col0 >= g.N) break;
+				float v[32];
+				tmem_ld32(tmem + ((uint32_t)(32 * qd) << 16) + (uint32_t)(a * BN + c), v);
+				store_block(g, &tcm, ebuf + (qd * 2 + (nst++ & 1)) * 4096, row0, col0, v, lane);
+			}
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0) mbar_arrive_cluster(cluster_addr(&accempty[a], 0));
+		}
+		if (lane == 0) bulk_wait_read_all();  // the staging buffers are read before the CTA exits
+		__syncwarp();
+	}
+	if (*abort_flag) st_cluster_u32(cluster_addr(const_cast<int*>(abort_flag), rank ^ 1u), 1u);
+	tc_fence_before();
+	__syncthreads();
+	cluster_sync();  // both CTAs hold the same abort flag from here on
+	if (*abort_flag) {
+		if (threadIdx.x == 0) {
+			volatile int own = 0;
+			const uint32_t end = max(issued[0], issued[1]);
+			for (uint32_t n = issued[rank]; n < end; ++n) {
+				const int id = pair0 + (int)(n / (uint32_t)nk) * npairs;
+				load(n, (id / nt) * 2 * BM + (int)rank * BM, (id % nt) * BN + (int)rank * (BN / 2), (int)(n % (uint32_t)nk));
+			}
+			if (rank == 0)
+				for (uint32_t n = end > STAGES ? end - STAGES : 0; n < end; ++n)
+					mbar_wait(&full[n % STAGES], (n / STAGES) & 1, &own, g.err, kErrTimeoutFull);
+		}
+		__syncthreads();
+		cluster_sync();
+	}
+	if (threadIdx.x == 0) {  // the last commit has arrived here: nothing of the other CTA's is under way
+		volatile int own = 0;
+		mbar_wait(drain, 0, &own, g.err, kErrTimeoutAccum);
+	}
+	__syncthreads();
+	tc_fence_after();
+	if (warp == 1) tmem_dealloc_pair(tmem, tmem_cols_for(BN));
 }
 
 template <class P>
@@ -806,9 +983,6 @@ struct GemmSplitPolicy {
 		tma_load_2d(dst + 2 * SPLIT_TILE, &m.bh, bar, ks * BK, t.n0);
 		tma_load_2d(dst + 3 * SPLIT_TILE, &m.bl, bar, ks * BK, t.n0);
 	}
-	__device__ static void store(const Args& g, const Tile& t, int rl, int c, const float (&v)[32]) {
-		GemmPolicy::store(g, t, rl, c, v);
-	}
 };
 
 // The convolution (ConvPolicy's tiles: up to 128 pixels x 128 output
@@ -998,35 +1172,19 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
 				for (int j = 0; j < 32; ++j) v[j] = fmaf(v[j], kSplitLoScale, run[c + j]);  // exact scaling, one rounding
 				if constexpr (P::EPI_TMA) {
-					if (g.vec) {
-						const int row0 = t.m0 + 32 * qd, col0 = t.n0 + c;
-						if (row0 < g.M && col0 < g.N) {
-							uint8_t* sb = ebuf + (qd * 2 + (nst & 1)) * 4096;
-							if (lane == 0) bulk_wait_read_1();
-							__syncwarp();
-#pragma unroll
-							for (int j = 0; j < 8; ++j)
-								*reinterpret_cast<float4*>(sb + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-									make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-							fence_proxy_async_smem();
-							__syncwarp();
-							if (lane == 0) {
-								tma_store_2d(&tcm, sb, col0, row0);
-								bulk_commit();
-							}
-							++nst;
-						}
-						continue;
-					}
+					const int row0 = t.m0 + 32 * qd, col0 = t.n0 + c;
+					if (row0 < g.M && col0 < g.N)
+						store_block(g, &tcm, ebuf + (qd * 2 + (nst++ & 1)) * 4096, row0, col0, v, lane);
+				} else {
+					P::store(g, t, 32 * qd + lane, c, v);
 				}
-				P::store(g, t, 32 * qd + lane, c, v);
 			}
 			tc_fence_before();
 			__syncwarp();
 			if (lane == 0) mbar_arrive(&accempty[a]);
 		}
 		if constexpr (P::EPI_TMA) {
-			if (lane == 0) bulk_wait_all();
+			if (lane == 0) bulk_wait_read_all();
 			__syncwarp();
 		}
 	}
@@ -1108,6 +1266,34 @@ umi_status map_kmajor(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, i
 	return UMI_OK;
 }
 
+template <int BN>
+umi_status launch_pair(const void* B, const CUtensorMap& ta, const CUtensorMap& tc, CUtensorMapDataType dt,
+                       const GemmArgs& g, int ab_type, int pairs, cudaStream_t st) {
+	CUtensorMap tb;
+	UMI_TRY(map_kmajor(&tb, B, dt, g.N, g.K, BN / 2));
+	constexpr size_t SMEM = GemmPairT<BN>::SMEM;
+	auto kern = tc_pair_kernel<BN>;
+	UMI_TRY(umi::cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM),
+	                         "cudaFuncSetAttribute"));
+	const int tiles = umi::ceil_div(g.M, 2 * BM) * umi::ceil_div(g.N, BN);
+	kern<<<2 * std::min(tiles, pairs), NTHREADS, SMEM, st>>>(ta, tb, tc, g, idesc_f16((uint32_t)ab_type, 2 * BM, BN));
+	return umi::launch_status("tc_pair_kernel");
+}
+
+template <int BN>
+umi_status launch_single(const void* B, const CUtensorMap& ta, const CUtensorMap& tc, CUtensorMapDataType dt,
+                         const GemmArgs& g, int ab_type, cudaStream_t st) {
+	using P = GemmPolicyT<BN>;
+	CUtensorMap tb;
+	UMI_TRY(map_kmajor(&tb, B, dt, g.N, g.K, BN));
+	constexpr size_t SMEM = smem_bytes<P>();
+	auto kern = tc_kernel<P>;
+	int grid = 0;
+	UMI_TRY(persistent_grid(kern, SMEM, P::ntiles(g), tmem_cols_for(BN), &grid));
+	kern<<<grid, NTHREADS, SMEM, st>>>(ta, tb, tc, g, idesc_f16((uint32_t)ab_type, BM, BN));
+	return umi::launch_status("tc_kernel<gemm>");
+}
+
 umi_status gemm_launch(const void* A, const void* B, float* C, int M, int N, int K, int ab_type, int* err,
                        cudaStream_t st, unsigned long long acc_wait_ns = kWaitNs) {
 	if (M < 0 || N < 0 || K < 0) return umi::fail(UMI_ERR_INVALID_ARG, "gemm: negative size");
@@ -1118,7 +1304,7 @@ umi_status gemm_launch(const void* A, const void* B, float* C, int M, int N, int
 	if (!umi::aligned(A, 16) || !umi::aligned(B, 16))
 		return umi::fail(UMI_ERR_INVALID_ARG, "gemm: A and B must be 16-byte aligned");
 	const CUtensorMapDataType dt = ab_type ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-	CUtensorMap ta, tb;
+	CUtensorMap ta;
 	UMI_TRY(map_kmajor(&ta, A, dt, M, K, BM));
 	GemmArgs g{C, M, N, K, N, umi::aligned(C, 16) && N % 4 == 0, err, acc_wait_ns};
 	CUtensorMap tc;
@@ -1134,35 +1320,50 @@ umi_status gemm_launch(const void* A, const void* B, float* C, int M, int N, int
 		                       CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 		if (r != CUDA_SUCCESS) return umi::fail(UMI_ERR_CUDA, "gemm: C tensor map (%d)", (int)r);
 	}
-	if ((int64_t)umi::ceil_div(M, BM) * umi::ceil_div(N, GemmPolicy224::BN) > INT32_MAX)
+	if ((int64_t)umi::ceil_div(M, BM) * umi::ceil_div(N, 224) > INT32_MAX)
 		return umi::fail(UMI_ERR_UNSUPPORTED, "gemm: too many tiles");
-	// One CTA per SM works through the tiles in rounds; a round costs about the
-	// same for every tile (the MMAs run the full width), so pick the width
-	// whose rounds x width is smaller: 4096^3 is 512 tiles of 256 (3.4 rounds
-	// on 152 SMs, 4 x 256 column-units) or 608 of 224 (exactly 4 rounds,
-	// 4 x 224).
+	// Tiles are worked through in rounds of one per SM (pair of SMs).  The
+	// cheapest tile is taken by a model in nanoseconds fitted to measurements:
+	// a K step of 16 of one tile takes 39, 42, 55, 62 at widths 64, 128, 224, 256
+	// (below 128 the width no longer matters); rows of A and B that do not start
+	// on 128-byte lines halve what TMA brings, then its bytes (4 KB of A, 32 of
+	// each column of B, half of that in a pair) at 90 a nanosecond bound the
+	// step.  One-CTA tiles on nearly every SM take an eighth longer (their
+	// operands' traffic); a pair costs 1.1 us once and more in its epilogue,
+	// which hides behind the next round's MMAs.
+	// Measured, pair and one-CTA tiles at their best widths: 4096^3 81.1 and 89.7
+	// us, 3000 x 2500 x 4096 39.6 and 43.4, 1000 x 1540 x 2056 14.6 and 16.3, but
+	// 2048^3 15.7 and 14.3, 512^3 7.9 and 4.9 (6.9 with tiles of 256).
 	int dev = 0, sms = 0;
 	UMI_TRY(umi::cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
 	UMI_TRY(umi::cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"));
-	const int64_t mt = umi::ceil_div(M, BM);
-	const int64_t r256 = umi::ceil_div(mt * umi::ceil_div(N, 256), (int64_t)sms);
-	const int64_t r224 = umi::ceil_div(mt * umi::ceil_div(N, 224), (int64_t)sms);
-	if (r224 * 224 < r256 * 256) {
-		UMI_TRY(map_kmajor(&tb, B, dt, N, K, GemmPolicy224::BN));
-		constexpr size_t SMEM = smem_bytes<GemmPolicy224>();
-		auto kern = tc_kernel<GemmPolicy224>;
-		int grid = 0;
-		UMI_TRY(persistent_grid(kern, SMEM, GemmPolicy224::ntiles(g), tmem_cols_for(GemmPolicy224::BN), &grid));
-		kern<<<grid, NTHREADS, SMEM, st>>>(ta, tb, tc, g, idesc_f16((uint32_t)ab_type, BM, GemmPolicy224::BN));
-		return umi::launch_status("tc_kernel<gemm 224>");
+	const int64_t mt = umi::ceil_div(M, BM), mp = umi::ceil_div(M, 2 * BM), pairs = std::max(1, sms / 2);
+	int bn = 0, best_pair = 0;
+	int64_t best = INT64_MAX;
+	auto consider = [&](int width, int step, int pair) {
+		const int64_t tiles = (pair ? mp : mt) * umi::ceil_div(N, width), slots = pair ? pairs : sms;
+		if (K % 64 != 0) step = std::max(step, (4096 + width * (pair ? 16 : 32)) / 90);
+		int64_t round = umi::ceil_div((int64_t)K, (int64_t)16) * step, epi = pair ? 600 + 5 * width : 6 * width;
+		if (!pair && tiles * 10 > slots * 9) round += round / 8;
+		const int64_t cost = umi::ceil_div(tiles, slots) * std::max(round, epi) + epi + (pair ? 1100 : 0);
+		if (cost < best) {
+			best = cost;
+			bn = width;
+			best_pair = pair;
+		}
+	};
+	const int widths[4] = {256, 224, 128, 64}, steps[4] = {62, 55, 42, 39};
+	for (int i = 0; i < 4; ++i) consider(widths[i], steps[i], 0);
+	for (int i = 0; i < 3; ++i) consider(widths[i], steps[i], 1);
+	if (best_pair) {
+		if (bn == 256) return launch_pair<256>(B, ta, tc, dt, g, ab_type, (int)pairs, st);
+		if (bn == 224) return launch_pair<224>(B, ta, tc, dt, g, ab_type, (int)pairs, st);
+		return launch_pair<128>(B, ta, tc, dt, g, ab_type, (int)pairs, st);
 	}
-	UMI_TRY(map_kmajor(&tb, B, dt, N, K, GemmPolicy::BN));
-	constexpr size_t SMEM = smem_bytes<GemmPolicy>();
-	auto kern = tc_kernel<GemmPolicy>;
-	int grid = 0;
-	UMI_TRY(persistent_grid(kern, SMEM, GemmPolicy::ntiles(g), tmem_cols_for(GemmPolicy::BN), &grid));
-	kern<<<grid, NTHREADS, SMEM, st>>>(ta, tb, tc, g, idesc_f16((uint32_t)ab_type, BM, GemmPolicy::BN));
-	return umi::launch_status("tc_kernel<gemm>");
+	if (bn == 256) return launch_single<256>(B, ta, tc, dt, g, ab_type, st);
+	if (bn == 224) return launch_single<224>(B, ta, tc, dt, g, ab_type, st);
+	if (bn == 128) return launch_single<128>(B, ta, tc, dt, g, ab_type, st);
+	return launch_single<64>(B, ta, tc, dt, g, ab_type, st);
 }
 
 }  // namespace

@@ -127,6 +127,8 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* s
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // at most one bulk group of this thread still reading its shared-memory source
 __device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+// every bulk group of this thread has read its shared-memory source
+__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 // every bulk group of this thread complete
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // generic-proxy shared-memory writes visible to the async proxy (TMA)
@@ -177,6 +179,65 @@ __device__ __forceinline__ void mma_commit(uint32_t one, uint64_t* bar) {
 		"setp.ne.b32 q, %1, 0;\n\t"
 		"@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)),
 		"r"(one)
+		: "memory");
+}
+
+// ---- CTA pairs (clusters of two): one MMA over both CTAs' shared memory and TMEM
+__device__ __forceinline__ uint32_t cluster_rank() {
+	uint32_t r;
+	asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+	return r;
+}
+__device__ __forceinline__ void cluster_sync() {  // every thread of both CTAs
+	asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// the address, in the cluster's shared window, of CTA `rank`'s copy of p
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+	uint32_t a;
+	asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+	return a;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+	asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
+	asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+// a TMA load into this CTA that completes on an mbarrier of either CTA of the pair
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m, uint32_t bar, int x, int y) {
+	asm volatile(
+		"cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+			smem_u32(dst)),
+		"l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(x), "r"(y)
+		: "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* slot, uint32_t ncols) {  // one whole warp of each CTA
+	asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(ncols)
+	             : "memory");
+	asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {  // one whole warp of each CTA
+	asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// M = 256: each CTA holds 128 rows of A and of D and half the rows of B; issued by the even CTA
+__device__ __forceinline__ void mma_f16_pair(uint32_t one, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             bool accumulate) {
+	asm volatile(
+		"{\n\t.reg .pred p, q;\n\t"
+		"setp.ne.b32 p, %4, 0;\n\t"
+		"setp.ne.b32 q, %5, 0;\n\t"
+		"@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+		"l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate), "r"(one)
+		: "memory");
+}
+// arrives on the barrier at bar's offset in both CTAs
+__device__ __forceinline__ void mma_commit_pair(uint32_t one, uint64_t* bar) {
+	asm volatile(
+		"{\n\t.reg .pred q;\n\t"
+		"setp.ne.b32 q, %1, 0;\n\t"
+		"@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t}" ::"r"(
+			smem_u32(bar)),
+		"r"(one), "h"((uint16_t)3)
 		: "memory");
 }
 
