@@ -130,3 +130,26 @@ def test_gemm_f32_generic_plain_path(umi, orc, dev, M, N, K):
     C = umi.gemm_f32_generic(torch.from_numpy(a).to(dev), torch.from_numpy(b).to(dev)).cpu().numpy()
     want = orc.gemm_f64(a, b, b_is_nk=True)
     assert _scaled_err(C, want, orc.gemm_f64(np.abs(a), np.abs(b), b_is_nk=True)) <= TOL
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (129, 131, 72), (200, 260, 200)])
+def test_gemm_f32_f16x3_workspace_sizes(umi, orc, dev, M, N, K):
+    """The workspace the size function names (rows padded to 128-byte lines)
+    and one for rows without padding give the same bits; less is refused."""
+    import torch
+    g = np.random.default_rng(M + N + K)
+    a, b = g.standard_normal((M, K)).astype(np.float32), g.standard_normal((N, K)).astype(np.float32)
+    A, B = torch.from_numpy(a).to(dev), torch.from_numpy(b).to(dev)
+    al = lambda x: (x + 255) // 256 * 256
+    full = int(umi.lib().umi_gemm_f32_f16x3_workspace_bytes(M, N, K))
+    plain = 2 * al(M * K * 2) + 2 * al(N * K * 2)
+    assert plain <= full
+    got = []
+    for nb in (full, plain):
+        ws = torch.full((nb + 256,), 0x5A, dtype=torch.uint8, device=dev)
+        got.append(umi.gemm_f32_f16x3(A, B, workspace=ws[:nb]).cpu().numpy())
+        assert (ws[nb:] == 0x5A).all()
+    assert np.array_equal(got[0], got[1])
+    assert _scaled_err(got[0], orc.gemm_f64(a, b, b_is_nk=True), orc.gemm_f64(np.abs(a), np.abs(b), b_is_nk=True)) <= TOL
+    with pytest.raises(umi.UmiError):
+        umi.gemm_f32_f16x3(A, B, workspace=torch.empty(plain - 256, dtype=torch.uint8, device=dev))
