@@ -24,9 +24,10 @@
 //    next macroblocks' windows are copied (4-byte cp.async by all threads)
 //    while the current ones are searched (full_me_pipe_kernel); the
 //    SAD-volume output keeps one CTA per group of macroblocks
-//    (full_me_kernel).  16x16 blocks with argmin go elsewhere: ranges up to 7
-//    to the register-only kernel below, the rest to the exact elimination of
-//    full_me_elim.cu.
+//    (full_me_kernel).  It serves 8x8 blocks with centres or lists, or few of
+//    them; other 8x8 blocks go to the strips of full_me_8.cu, 16x16 blocks with
+//    ranges up to 7 to the register-only kernel below, the rest to the exact
+//    elimination of full_me_elim.cu.
 #include <algorithm>
 #include <cstring>
 
@@ -40,6 +41,8 @@ namespace umi {
 // and alignment; list, list_count and centers may be null.
 umi_status full_me_elim(const uint8_t* cur, const uint8_t* ref, int h, int w, int r, const int32_t* centers,
                         int32_t* out, const int32_t* list, const int32_t* list_count, int max_slots, cudaStream_t st);
+// Argmin search of every 8x8 block at its own place (full_me_8.cu).
+umi_status full_me_8(const uint8_t* cur, const uint8_t* ref, int h, int w, int r, int32_t* out, cudaStream_t st);
 }  // namespace umi
 
 namespace {
@@ -86,13 +89,11 @@ __device__ __forceinline__ int slot_block(const MeGeom& g, int slot) {
 template <int B, int G> struct MeRegs { static constexpr int value = B == 16 ? (5 * G + 31) / 8 * 8 + 8 : 64; };
 template <> struct MeRegs<16, 13> { static constexpr int value = 80; };
 
-template <int B, int G, bool VOLUME>
+template <int B, int G>
 __global__ void __launch_bounds__(512) __maxnreg__((MeRegs<B, G>::value))
-full_me_kernel(const uint8_t* __restrict__ cur, const uint8_t* __restrict__ ref, const int32_t* __restrict__ centers,
-               int32_t* __restrict__ out, const MeGeom g) {
+full_me_kernel(const uint8_t* __restrict__ cur, const uint8_t* __restrict__ ref, int32_t* __restrict__ out, const MeGeom g) {
 	extern __shared__ __align__(128) uint32_t smem[];
 	constexpr int BW = B / 4;  // words per block row
-	__shared__ uint32_t best[64];
 	const int tid = threadIdx.x;
 	const int mb0 = blockIdx.x * g.m;
 
@@ -107,8 +108,7 @@ full_me_kernel(const uint8_t* __restrict__ cur, const uint8_t* __restrict__ ref,
 		const int blk = slot_block(g, mb0 + m);
 		if (blk < 0) break;
 		const int by = blk / g.nbx, bx = blk - by * g.nbx;
-		const int cy = centers ? centers[2 * blk] : 0, cx = centers ? centers[2 * blk + 1] : 0;
-		const int gy0 = by * B + cy - g.r, gx0 = bx * B + cx - g.r;
+		const int gy0 = by * B - g.r, gx0 = bx * B - g.r;
 		uint32_t* win = smem + m * g.mb_stride;
 		const int gx = gx0 + 4 * wd0;
 		const bool vec = g.vec_ok && gx >= 0 && gx + 3 < g.w && (gx & 3) == 0;
@@ -139,7 +139,6 @@ full_me_kernel(const uint8_t* __restrict__ cur, const uint8_t* __restrict__ ref,
 			for (int k = 0; k < 4; ++k) v |= (uint32_t)__ldg(src + k) << (8 * k);
 			cb[tid] = v;
 		}
-		if (tid == 0) best[m] = 0xffffffffu;
 	}
 	__syncthreads();
 	// 2. Shifted copies s = 1..3: word k holds bytes [4k+s, 4k+s+4) of the row.
@@ -212,31 +211,10 @@ full_me_kernel(const uint8_t* __restrict__ cur, const uint8_t* __restrict__ ref,
 				for (int q = 0; q < G; ++q) acc[q] = sad4_acc(cv[k], ring[(py + q) % G][k], acc[q]);
 		}
 		const int iy0 = grp * G;
-		if (VOLUME) {
-			int32_t* o = out + (size_t)blk * g.ndx * g.ndx;
+		int32_t* o = out + (size_t)blk * g.ndx * g.ndx;
 #pragma unroll
-			for (int q = 0; q < G; ++q)
-				if (iy0 + q < g.ndx) o[(iy0 + q) * g.ndx + ix] = (int32_t)acc[q];
-		} else {
-			uint32_t key = 0xffffffffu;
-#pragma unroll
-			for (int q = 0; q < G; ++q)
-				if (iy0 + q < g.ndx) key = min(key, (acc[q] << 15) | (uint32_t)((iy0 + q) * g.ndx + ix));
-			atomicMin(&best[m], key);
-		}
-	}
-	if (VOLUME) return;
-	__syncthreads();
-	for (int m = tid; m < g.m; m += blockDim.x) {
-		const int blk = slot_block(g, mb0 + m);
-		if (blk < 0) break;
-		const uint32_t key = best[m];
-		const int idx = (int)(key & 0x7fffu);
-		const int iy = idx / g.ndx, ix = idx - iy * g.ndx;
-		const int cy = centers ? centers[2 * blk] : 0, cx = centers ? centers[2 * blk + 1] : 0;
-		out[3 * blk + 0] = cy + iy - g.r;
-		out[3 * blk + 1] = cx + ix - g.r;
-		out[3 * blk + 2] = (int32_t)(key >> 15);
+		for (int q = 0; q < G; ++q)
+			if (iy0 + q < g.ndx) o[(iy0 + q) * g.ndx + ix] = (int32_t)acc[q];
 	}
 }
 
@@ -618,10 +596,10 @@ int pick_g(int ndx) {
 	return best;
 }
 
-template <int B, int G, bool V>
-umi_status launch_g(const uint8_t* cur, const uint8_t* ref, const int32_t* centers, int32_t* out, const MeGeom& g,
-                    int threads, size_t smem, cudaStream_t st) {
-	auto kern = full_me_kernel<B, G, V>;
+template <int B, int G>
+umi_status launch_g(const uint8_t* cur, const uint8_t* ref, int32_t* out, const MeGeom& g, int threads, size_t smem,
+                    cudaStream_t st) {
+	auto kern = full_me_kernel<B, G>;
 	if (smem > 48 * 1024) UMI_TRY(umi::cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                                                                 (int)smem), "cudaFuncSetAttribute"));
 	// Without this the driver may pick a small shared-memory carveout and
@@ -629,7 +607,7 @@ umi_status launch_g(const uint8_t* cur, const uint8_t* ref, const int32_t* cente
 	UMI_TRY(umi::cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
 	                                              (int)cudaSharedmemCarveoutMaxShared), "cudaFuncSetAttribute"));
 	const int grid = (g.slots + g.m - 1) / g.m;
-	kern<<<grid, threads, smem, st>>>(cur, ref, centers, out, g);
+	kern<<<grid, threads, smem, st>>>(cur, ref, out, g);
 	return umi::launch_status("full_me_kernel");
 }
 
@@ -664,14 +642,14 @@ umi_status launch_pipe_b(int G, const uint8_t* cur, const uint8_t* ref, const in
 	}
 }
 
-template <int B, bool V>
-umi_status launch_b(int G, const uint8_t* cur, const uint8_t* ref, const int32_t* centers, int32_t* out,
-                    const MeGeom& g, int threads, size_t smem, cudaStream_t st) {
+template <int B>
+umi_status launch_b(int G, const uint8_t* cur, const uint8_t* ref, int32_t* out, const MeGeom& g, int threads, size_t smem,
+                    cudaStream_t st) {
 	switch (G) {
-		case 5: return launch_g<B, 5, V>(cur, ref, centers, out, g, threads, smem, st);
-		case 9: return launch_g<B, 9, V>(cur, ref, centers, out, g, threads, smem, st);
-		case 13: return launch_g<B, 13, V>(cur, ref, centers, out, g, threads, smem, st);
-		default: return launch_g<B, 15, V>(cur, ref, centers, out, g, threads, smem, st);
+		case 5: return launch_g<B, 5>(cur, ref, out, g, threads, smem, st);
+		case 9: return launch_g<B, 9>(cur, ref, out, g, threads, smem, st);
+		case 13: return launch_g<B, 13>(cur, ref, out, g, threads, smem, st);
+		default: return launch_g<B, 15>(cur, ref, out, g, threads, smem, st);
 	}
 }
 
@@ -704,6 +682,18 @@ umi_status full_me_common(const uint8_t* cur, const uint8_t* ref, int32_t h, int
 	if (!volume && b == 16) {
 		const umi_status rc = umi::full_me_elim(cur, ref, h, w, r, centers, out, list, list_count, max_slots,
 		                                        umi::as_stream(stream));
+		return rc == UMI_OK ? umi::ok() : rc;
+	}
+	// 8x8 blocks at their own places go in strips.  A small frame has too few of
+	// them for the GPU; there the general kernel, one CTA for one or two blocks,
+	// is faster once a block's displacements fill it (240 blocks, +-16: 5.0 us
+	// and 6.6 in strips, 660 blocks 8.3 and 6.3; 240 blocks, +-7: 14.8 and 4.6).
+	int dev = 0, sms = 0;
+	UMI_TRY(umi::cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
+	UMI_TRY(umi::cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"));
+	const bool few = r <= 8 ? g.nblk < 4 : g.nblk <= (r < 16 ? 5 : 3) * sms;
+	if (!volume && !list && !centers && !few) {
+		const umi_status rc = umi::full_me_8(cur, ref, h, w, r, out, umi::as_stream(stream));
 		return rc == UMI_OK ? umi::ok() : rc;
 	}
 	g.win_words = g.win_need;
@@ -740,16 +730,10 @@ umi_status full_me_common(const uint8_t* cur, const uint8_t* ref, int32_t h, int
 	const size_t smem = (size_t)m * g.mb_stride * 4;
 	const cudaStream_t st = umi::as_stream(stream);
 	umi_status rc;
-	if (!volume && 2 * smem <= 200 * 1024) {  // double-buffered persistent search
-		const int tp = threads_for(m * g.tasks_pipe);
-		rc = b == 16 ? launch_pipe_b<16>(G, cur, ref, centers, out, g, tp, 2 * smem, st)
-		             : launch_pipe_b<8>(G, cur, ref, centers, out, g, tp, 2 * smem, st);
-	} else if (b == 16)
-		rc = volume ? launch_b<16, true>(G, cur, ref, centers, out, g, threads, smem, st)
-		            : launch_b<16, false>(G, cur, ref, centers, out, g, threads, smem, st);
+	if (!volume)  // 8x8 blocks: at most 160 KB of the two buffers (+-64)
+		rc = launch_pipe_b<8>(G, cur, ref, centers, out, g, threads_for(m * g.tasks_pipe), 2 * smem, st);
 	else
-		rc = volume ? launch_b<8, true>(G, cur, ref, centers, out, g, threads, smem, st)
-		            : launch_b<8, false>(G, cur, ref, centers, out, g, threads, smem, st);
+		rc = b == 16 ? launch_b<16>(G, cur, ref, out, g, threads, smem, st) : launch_b<8>(G, cur, ref, out, g, threads, smem, st);
 	return rc == UMI_OK ? umi::ok() : rc;
 }
 
