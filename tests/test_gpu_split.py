@@ -153,3 +153,22 @@ def test_gemm_f32_f16x3_workspace_sizes(umi, orc, dev, M, N, K):
     assert _scaled_err(got[0], orc.gemm_f64(a, b, b_is_nk=True), orc.gemm_f64(np.abs(a), np.abs(b), b_is_nk=True)) <= TOL
     with pytest.raises(umi.UmiError):
         umi.gemm_f32_f16x3(A, B, workspace=torch.empty(plain - 256, dtype=torch.uint8, device=dev))
+
+
+# more tiles than SMs, so that accumulators are reused from tile to tile: one
+# chunk per tile (two correction accumulators in turn), an odd and an even
+# number of chunks (the chunks' order alternates across tiles), a short last one
+@pytest.mark.parametrize("K,chunk", [(64, 2), (128, 2), (136, 3), (192, 1), (200, 2), (256, 2), (328, 2)])
+def test_gemm_f32_f16x3_accumulator_reuse(umi, orc, dev, K, chunk):
+    import torch
+    M, N = 2500, 2090
+    g = np.random.default_rng(K + chunk)
+    a, b = g.standard_normal((M, K)).astype(np.float32), g.standard_normal((N, K)).astype(np.float32)
+    err = torch.zeros(1, dtype=torch.int32, device=dev)
+    got = umi.gemm_f32_f16x3(torch.from_numpy(a).to(dev), torch.from_numpy(b).to(dev), chunk=chunk, err=err).cpu().numpy()
+    assert int(err.item()) == 0
+    assert np.isfinite(got).all()
+    rows = np.unique(np.concatenate([np.arange(0, M, 61), [127, 128, M - 1]]))
+    want = orc.gemm_f64(a[rows], b, b_is_nk=True)
+    scale = orc.gemm_f64(np.abs(a[rows]), np.abs(b), b_is_nk=True)
+    assert _scaled_err(got[rows], want, scale) <= TOL
