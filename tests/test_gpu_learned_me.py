@@ -177,6 +177,28 @@ def test_menet_gradient_tiles(umi, dev, h, w):
         assert np.abs(grads[a:b] - want[a:b]).max() <= 1e-4 * (np.abs(want[a:b]).max() + 1e-12), (a, b)
 
 
+@pytest.mark.parametrize("shift", [-40, 0, 40])
+def test_menet_gradient_range(umi, dev, shift):
+    """Gradients between the layers as exact sums of three bf16 parts: the same
+    relative accuracy when they are 2^40 times smaller or larger (scaled head
+    weights; targets and predictions far apart keep the smooth-L1 slopes at +-1)."""
+    h, w = 48, 272
+    g = np.random.default_rng(h + w)
+    cur = g.integers(0, 256, (h, w), dtype=np.uint8)
+    ref = g.integers(0, 256, (h, w), dtype=np.uint8)
+    p = _params(3)
+    layers, wh, bh, _ = menet.layout()
+    p[wh:bh] *= 2.0 ** shift
+    tgt = g.choice([-4000, 4000], ((h // 16) * (w // 16), 2)).astype(np.int32)
+    net = umi.MeNet(h, w, device=dev, params=p)
+    net.forward(_t(cur, dev), _t(ref, dev))
+    grads = net.backward(_t(tgt, dev)).cpu().numpy().astype(np.float64)
+    _, want = menet.loss_and_grad(p, cur, ref, tgt, bf16=True)
+    n = wh  # the convolution layers' weights and biases
+    assert np.isfinite(grads).all()
+    assert np.linalg.norm(grads[:n] - want[:n]) <= 1e-5 * np.linalg.norm(want[:n])
+
+
 def test_menet_rejects_bad_frames(umi, dev):
     import torch
     assert umi.lib().umi_menet_workspace_bytes(100, 64) == 0

@@ -654,19 +654,8 @@ struct MenetRun {
 	__device__ static uint64_t desc_a(uint32_t strip, int row) { return desc_kmajor_sw64(strip + 64u * (uint32_t)row); }
 	__device__ static uint64_t desc_b(uint32_t slice) { return desc_kmajor_sw64(slice); }
 	__device__ static uint32_t strip_bytes(const Args& g) { return (uint32_t)(BM + 2 * g.dil) * KT * 2; }
-	// classes c = y mod d in order, y ascending within a class: classes
-	// 0 .. rm-1 hold q+1 rows, the others q (q = h / d, rm = h mod d)
 	__device__ static void row_of(const Args& g, int pos, int& y, int& class_end) {
-		const int d = g.dil, q = g.h / d, rm = g.h - q * d, big = rm * (q + 1);
-		if (pos < big) {
-			const int c = pos / (q + 1), k = pos - c * (q + 1);
-			y = c + k * d;
-			class_end = (c + 1) * (q + 1);
-		} else {
-			const int p2 = pos - big, c = p2 / q, k = p2 - c * q;
-			y = rm + c + k * d;
-			class_end = big + (c + 1) * q;
-		}
+		umi_roll::row_of(g.h, g.dil, pos, y, class_end);
 	}
 	__device__ static void load_strip(const CUtensorMap* ta, const Args& g, int blk, int row, void* dst, uint64_t* bar) {
 		tma_load_4d(dst, ta, bar, 0, blk * BM - g.dil, row, 0);

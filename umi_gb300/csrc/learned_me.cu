@@ -25,6 +25,10 @@
 namespace umi {
 umi_status menet_conv_tc(const void* in, void* out, const void* wpack, const float* bias, int h, int w, int dil,
                          int* err, cudaStream_t st);
+// The layers' data gradient on the tensor cores at fp32 accuracy (menet_parts.cu).
+umi_status menet_to_parts(const float* in, void* parts, int P, cudaStream_t st);
+umi_status menet_dgrad(const void* parts, const void* wpack, const float* mask, float* out, void* out_parts, int h, int w,
+                       int dil, int* err, cudaStream_t st);
 }
 
 namespace {
@@ -55,6 +59,7 @@ struct Layout {
 struct Work {
 	int H4, W4, P, nbx, nby, nblk;
 	size_t x0, act[NL], dA[2], wf[NL], wt[NL], pred, centers, list, count, alist, amv, wpart, hpart;
+	size_t parts[2];         // training: gradients as bf16 parts (menet_parts.cu)
 	size_t nhwc[2], wtc[NL], err;  // tensor-core inference: bf16 (H4, W4, 32) activations, packed weights
 	size_t bytes;
 	Work(int h, int w) {
@@ -65,9 +70,10 @@ struct Work {
 		x0 = take(sizeof(float) * 2 * P);
 		for (int l = 0; l < NL; ++l) act[l] = take(sizeof(float) * CH * P);
 		for (int i = 0; i < 2; ++i) dA[i] = take(sizeof(float) * CH * P);
-		// training weights (menet_train.cuh): layer 0 once, the others every value twice
+		// training weights (menet_train.cuh): fp32 for the forward layers (after
+		// the first every value twice), bf16 for the data gradient
 		for (int l = 0; l < NL; ++l) wf[l] = take(sizeof(float) * (l ? 2 : 1) * CH * CIN[l] * 9);
-		for (int l = 0; l < NL; ++l) wt[l] = l ? take(sizeof(float) * 2 * CH * CIN[l] * 9) : 0;
+		for (int l = 0; l < NL; ++l) wt[l] = l ? take(2 * CH * CIN[l] * 9) : 0;
 		pred = take(sizeof(float) * 2 * nblk);
 		centers = take(sizeof(int32_t) * 2 * nblk);
 		list = take(sizeof(int32_t) * nblk);
@@ -76,6 +82,7 @@ struct Work {
 		amv = take(sizeof(int32_t) * 3 * nblk);
 		wpart = take(sizeof(float) * (size_t)menet_train::PARTS * (CH * CH * 9 + CH));
 		hpart = take(sizeof(float) * (size_t)menet_train::HEAD_PARTS * (2 * HEADF + 3));
+		for (int i = 0; i < 2; ++i) parts[i] = take((size_t)P * 3 * CH * 2);
 		for (int i = 0; i < 2; ++i) nhwc[i] = take((size_t)P * 64);
 		for (int l = 0; l < NL; ++l) wtc[l] = take(2 * CH * 9 * CH);
 		err = take(sizeof(int32_t));
@@ -359,25 +366,22 @@ umi_status check_frame(int h, int w) {
 int grid_for(size_t n) { return (int)std::min<size_t>((n + NT - 1) / NT, 4096); }
 
 template <int DIL>
-umi_status conv_dil(const float* in, const float* w, const float* bias, float* out, const float* mask, const Work& K,
-                    int relu, cudaStream_t st) {
+umi_status conv_dil(const float* in, const float* w, const float* bias, float* out, const Work& K, cudaStream_t st) {
 	auto kern = menet_train::conv_kernel<DIL>;
 	constexpr int SMEM = (int)menet_train::ConvTile<DIL>::smem;
 	UMI_TRY(umi::cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM),
 	                         "cudaFuncSetAttribute"));
-	kern<<<dim3(umi::ceil_div(K.W4, 32), umi::ceil_div(K.H4, 16)), NT, SMEM, st>>>(in, w, bias, out, mask, K.H4, K.W4,
-	                                                                             relu);
+	kern<<<dim3(umi::ceil_div(K.W4, 32), umi::ceil_div(K.H4, 16)), NT, SMEM, st>>>(in, w, bias, out, K.H4, K.W4);
 	return umi::launch_status("conv_kernel");
 }
 
-// Layer l = 1, 2, 3 (dilations 2, 4, 8): forward, or the data gradient with
-// the transposed, flipped weights.
-umi_status conv_layer(int l, const float* in, const float* w, const float* bias, float* out, const float* mask,
-                      const Work& K, int relu, cudaStream_t st) {
+// Layer l = 1, 2, 3 (dilations 2, 4, 8), forward.
+umi_status conv_layer(int l, const float* in, const float* w, const float* bias, float* out, const Work& K,
+                      cudaStream_t st) {
 	static_assert(DIL[1] == 2 && DIL[2] == 4 && DIL[3] == 8, "one instance per layer");
-	if (l == 1) return conv_dil<DIL[1]>(in, w, bias, out, mask, K, relu, st);
-	if (l == 2) return conv_dil<DIL[2]>(in, w, bias, out, mask, K, relu, st);
-	return conv_dil<DIL[3]>(in, w, bias, out, mask, K, relu, st);
+	if (l == 1) return conv_dil<DIL[1]>(in, w, bias, out, K, st);
+	if (l == 2) return conv_dil<DIL[2]>(in, w, bias, out, K, st);
+	return conv_dil<DIL[3]>(in, w, bias, out, K, st);
 }
 
 template <int DIL>
@@ -407,16 +411,16 @@ umi_status forward(const uint8_t* cur, const uint8_t* ref, int h, int w, const f
 	for (int l = 0; l < NL; ++l) {
 		pk.w[l] = params + L.w[l];
 		pk.fwd[l] = K.at<float>(ws, K.wf[l]);
-		pk.bwd[l] = l ? K.at<float>(ws, K.wt[l]) : nullptr;
+		pk.bwd[l] = l ? K.at<__nv_bfloat16>(ws, K.wt[l]) : nullptr;
 	}
 	menet_train::pack_weights_kernel<<<dim3(grid_for(CH * CH * 9), NL), NT, 0, st>>>(pk);
 	UMI_TRY(umi::launch_status("pack_weights_kernel"));
 	menet_train::conv_first_kernel<<<umi::ceil_div(K.P / 4, NT), NT, 0, st>>>(
-		K.at<float>(ws, K.x0), pk.fwd[0], params + L.b[0], K.at<float>(ws, K.act[0]), K.H4, K.W4);
+		K.at<float>(ws, K.x0), K.at<float>(ws, K.wf[0]), params + L.b[0], K.at<float>(ws, K.act[0]), K.H4, K.W4);
 	UMI_TRY(umi::launch_status("conv_first_kernel"));
 	for (int l = 1; l < NL; ++l)
-		UMI_TRY(conv_layer(l, K.at<float>(ws, K.act[l - 1]), pk.fwd[l], params + L.b[l], K.at<float>(ws, K.act[l]),
-		                   nullptr, K, 1, st));
+		UMI_TRY(conv_layer(l, K.at<float>(ws, K.act[l - 1]), K.at<float>(ws, K.wf[l]), params + L.b[l],
+		                   K.at<float>(ws, K.act[l]), K, st));
 	menet_train::head_fwd_kernel<<<dim3(umi::ceil_div(K.nbx, 64), K.nby), NT, 0, st>>>(
 		K.at<float>(ws, K.act[NL - 1]), params + L.wh, params + L.bh, K.at<float>(ws, K.pred), K.H4, K.W4, K.nbx);
 	return umi::launch_status("head_fwd_kernel");
@@ -509,6 +513,8 @@ extern "C" umi_status umi_menet_backward(const int32_t* target, int32_t target_s
 	                                                K.at<float>(ws, K.hpart), K.H4, K.W4, K.nbx, K.nblk, htx, htiles);
 	UMI_TRY(umi::launch_status("head_bwd_kernel"));
 	UMI_TRY(reduce_rows(K.at<float>(ws, K.hpart), grads + L.wh, loss, nh, 2 * HEADF + 3, 2 * HEADF + 2, st));
+	void *din = K.at<void>(ws, K.parts[0]), *dout = K.at<void>(ws, K.parts[1]);
+	UMI_TRY(umi::menet_to_parts(dcur, din, K.P, st));
 	const int units = umi::ceil_div(K.W4, 32) * K.H4, per = umi::ceil_div(units, menet_train::PARTS);
 	const int grid = umi::ceil_div(units, per);
 	float* part = K.at<float>(ws, K.wpart);
@@ -525,8 +531,10 @@ extern "C" umi_status umi_menet_backward(const int32_t* target, int32_t target_s
 		// grads[w_l], then grads[b_l] right after it (same layout as the partial rows)
 		UMI_TRY(reduce_rows(part, grads + L.w[l], nullptr, grid, m, m, st));
 		if (l > 0) {  // data gradient, masked by ReLU(a_{l-1})
-			UMI_TRY(conv_layer(l, dcur, K.at<float>(ws, K.wt[l]), nullptr, dnext, K.at<float>(ws, K.act[l - 1]), K, 0, st));
+			UMI_TRY(umi::menet_dgrad(din, K.at<void>(ws, K.wt[l]), K.at<float>(ws, K.act[l - 1]), dnext,
+			                         l > 1 ? dout : nullptr, K.H4, K.W4, DIL[l], K.at<int32_t>(ws, K.err), st));
 			std::swap(dcur, dnext);
+			std::swap(din, dout);
 		}
 	}
 	return umi::ok();

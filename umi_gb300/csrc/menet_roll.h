@@ -23,7 +23,10 @@ namespace umi_roll {
 
 constexpr int kSlots = 16;  // 32-column accumulators: all 512 TMEM columns
 
-UMI_ROLL_HD int slot(int r) { return kSlots - 1 - (r & (kSlots - 1)); }
+template <int SLOTS = kSlots>
+UMI_ROLL_HD int slot(int r) {
+	return SLOTS - 1 - r % SLOTS;
+}
 
 struct Step {
 	int lo, hi;  // filter rows reading strip m
@@ -31,14 +34,31 @@ struct Step {
 	int c1;      // blocks before the ring wraps (cnt = hi - lo + 1 in all)
 };
 
+template <int SLOTS = kSlots>
 UMI_ROLL_HD Step step(int m, int rows, int r0) {
 	Step s;
 	s.lo = m - rows + 1 > 0 ? m - rows + 1 : 0;
 	s.hi = m < 2 ? m : 2;
-	s.first = slot(r0 + m - s.lo);
+	s.first = slot<SLOTS>(r0 + m - s.lo);
 	const int cnt = s.hi - s.lo + 1;
-	s.c1 = cnt < kSlots - s.first ? cnt : kSlots - s.first;
+	s.c1 = cnt < SLOTS - s.first ? cnt : SLOTS - s.first;
 	return s;
+}
+
+// Row of position pos in a block's order, and the end of its dilation class:
+// classes c = y mod d in order, y ascending within a class; classes
+// 0 .. rm-1 hold q+1 rows, the others q (q = h / d, rm = h mod d).
+UMI_ROLL_HD void row_of(int h, int d, int pos, int& y, int& class_end) {
+	const int q = h / d, rm = h - q * d, big = rm * (q + 1);
+	if (pos < big) {
+		const int c = pos / (q + 1), k = pos - c * (q + 1);
+		y = c + k * d;
+		class_end = (c + 1) * (q + 1);
+	} else {
+		const int p2 = pos - big, c = p2 / q, k = p2 - c * q;
+		y = rm + c + k * d;
+		class_end = big + (c + 1) * q;
+	}
 }
 
 }  // namespace umi_roll

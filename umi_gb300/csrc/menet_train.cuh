@@ -67,28 +67,29 @@ template <int DIL> struct Strip {
 	static constexpr int TAP0 = (HALO - DIL) / 2;  // pair of tap column 0; the next ones DIL / 2 pairs on
 };
 
-// ---- fp32 weights of the 32 -> 32 layers, rounded to bf16, every value twice
-// (the constant operand of fma2): fwd[ci][tap][co][2], and for the data
-// gradient transposed and flipped, bwd[co][8 - tap][ci][2].  Layer 0 keeps
-// plain values [ci][tap][co].
+// ---- weights rounded to bf16.  Forward in fp32, fwd[ci][tap][co], after layer
+// 0 every value twice (the constant operand of fma2); for the data gradient of
+// the 32 -> 32 layers transposed and flipped, as K-major bf16 matrices
+// bwd[ci][8 - tap][co] (menet_parts.cu).
 struct Pack {
 	const float* w[4];
 	float* fwd[4];
-	float* bwd[4];
+	__nv_bfloat16* bwd[4];
 };
 __global__ void pack_weights_kernel(const Pack p) {
 	const int l = blockIdx.y, cin = l == 0 ? 2 : CH;
 	const float* w = l == 0 ? p.w[0] : l == 1 ? p.w[1] : l == 2 ? p.w[2] : p.w[3];
 	float* fwd = l == 0 ? p.fwd[0] : l == 1 ? p.fwd[1] : l == 2 ? p.fwd[2] : p.fwd[3];
-	float* bwd = l == 1 ? p.bwd[1] : l == 2 ? p.bwd[2] : p.bwd[3];
+	__nv_bfloat16* bwd = l == 1 ? p.bwd[1] : l == 2 ? p.bwd[2] : p.bwd[3];
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < CH * cin * 9; i += gridDim.x * blockDim.x) {
 		const int co = i / (cin * 9), r = i - co * cin * 9, ci = r / 9, tap = r - ci * 9;
-		const float v = __bfloat162float(__float2bfloat16_rn(w[i]));
+		const __nv_bfloat16 b = __float2bfloat16_rn(w[i]);
+		const float v = __bfloat162float(b);
 		if (l == 0) {
 			fwd[r * CH + co] = v;
 		} else {
 			reinterpret_cast<float2*>(fwd)[r * CH + co] = make_float2(v, v);
-			reinterpret_cast<float2*>(bwd)[(co * 9 + 8 - tap) * CH + ci] = make_float2(v, v);
+			bwd[(ci * 9 + 8 - tap) * CH + co] = b;
 		}
 	}
 }
@@ -156,10 +157,9 @@ __global__ void __launch_bounds__(NT) conv_first_kernel(const float* __restrict_
 	}
 }
 
-// ---- layers 2-4, forward and data gradient (32 -> 32 channels).
-//   out[co][p] = act( bias[co] + sum_{ci,tap} w[ci][tap][co] in[ci][p + DIL off(tap)] ),
-// zero outside the image; ReLU when relu, zeroed where !(mask > 0) when mask
-// is given.  CTA: 32 x 16 pixels x 32 channels; a warp owns 8 channels and 8
+// ---- layers 2-4, forward (32 -> 32 channels).
+//   out[co][p] = relu( bias[co] + sum_{ci,tap} w[ci][tap][co] in[ci][p + DIL off(tap)] ),
+// zero outside the image.  CTA: 32 x 16 pixels x 32 channels; a warp owns 8 channels and 8
 // rows, a thread 8 adjacent pixels (four pairs) x 8 channels.  Per input
 // channel and tap row it reads 4-6 16-byte pieces of its pixel row and 12 of
 // doubled weights (one address per warp) for 96 fma2.  Two input channels per
@@ -173,8 +173,8 @@ template <int DIL> struct ConvTile : Strip<DIL> {
 
 template <int DIL>
 __global__ void __launch_bounds__(NT, 2) conv_kernel(const float* __restrict__ in, const float* __restrict__ wdup,
-                                                     const float* __restrict__ bias, float* __restrict__ out,
-                                                     const float* __restrict__ mask, int H, int W, int relu) {
+                                                     const float* __restrict__ bias, float* __restrict__ out, int H,
+                                                     int W) {
 	using T = ConvTile<DIL>;
 	constexpr int TH = T::TH, TWP = T::TWP, Q = T::Q, STG = T::ACT + T::WST;
 	constexpr int NQ = (T::TAP0 * 2 + 2 * DIL + 8 + 3) / 4;  // pieces of a row a thread reads
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(NT, 2) conv_kernel(const float* __restrict__ i
 	uint64_t acc[8][4];  // [channel][pixel pair]
 #pragma unroll
 	for (int c = 0; c < 8; ++c) {
-		const float b = bias ? __ldg(bias + 8 * cg + c) : 0.0f;
+		const float b = __ldg(bias + 8 * cg + c);
 #pragma unroll
 		for (int p = 0; p < 4; ++p) acc[c][p] = pair(b, b);
 	}
@@ -248,16 +248,8 @@ __global__ void __launch_bounds__(NT, 2) conv_kernel(const float* __restrict__ i
 #pragma unroll
 		for (int c = 0; c < 8; ++c) {
 			const float2 l = unpair(acc[c][2 * h]), r = unpair(acc[c][2 * h + 1]);
-			float4 o = make_float4(l.x, l.y, r.x, r.y);
 			const size_t p = (size_t)(8 * cg + c) * P + (size_t)y * W + x;
-			if (relu) o = make_float4(fmaxf(o.x, 0.f), fmaxf(o.y, 0.f), fmaxf(o.z, 0.f), fmaxf(o.w, 0.f));
-			if (mask) {
-				const float4 m = __ldg(reinterpret_cast<const float4*>(mask + p));
-				if (!(m.x > 0.0f)) o.x = 0.0f;
-				if (!(m.y > 0.0f)) o.y = 0.0f;
-				if (!(m.z > 0.0f)) o.z = 0.0f;
-				if (!(m.w > 0.0f)) o.w = 0.0f;
-			}
+			const float4 o = make_float4(fmaxf(l.x, 0.f), fmaxf(l.y, 0.f), fmaxf(r.x, 0.f), fmaxf(r.y, 0.f));
 			*reinterpret_cast<float4*>(out + p) = o;
 		}
 	}
