@@ -157,6 +157,15 @@ typedef enum umi_strategy {
 umi_status umi_launch(const umi_plan* plan, int32_t strategy, const void* const* in, const void* pad,
                       void* const* out, const void* user_const, size_t uc_bytes, void* stream);
 
+/* Separable window sum of an (h, w) float image, k <= UMI_SEPARABLE_MAX_TAPS
+ * weights (device) across, then down, centred, edges replicated: the result
+ * (and, in tmp, if not NULL, the first pass) of two umi_launch calls of
+ * UMI_STRATEGY_WEIGHTED_SUM_F32 with init 0, in one launch.  in, tmp and out
+ * must not overlap. */
+#define UMI_SEPARABLE_MAX_TAPS 31
+umi_status umi_separable_f32(const float* in, const float* weights, int32_t k, int32_t h, int32_t w, float* tmp,
+                             float* out, void* stream);
+
 /* ------------------------------------------------------------------ */
 /* specialised kernels                                                 */
 /* ------------------------------------------------------------------ */

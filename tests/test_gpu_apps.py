@@ -70,3 +70,31 @@ def test_gaussian(umi, dev, h, w, sigma):
     want = sum(k[i] * hz[i:i + h, :] for i in range(k.size))
     got = apps.gaussian(_t(x, dev), sigma).cpu().numpy()
     assert np.max(np.abs(got - want) / np.maximum(np.abs(want), 1e-3)) <= 1e-5
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (5, 3), (31, 127), (32, 128), (33, 129), (97, 260), (70, 514)])
+@pytest.mark.parametrize("radius", [0, 1, 3, 4, 6, 15, 16])
+def test_gaussian_one_launch_equals_two(umi, dev, h, w, radius):
+    """The one-launch blur (up to 31 weights) gives the bits of the two window
+    sums, also in tmp; overlapping buffers and wider windows take two."""
+    import torch
+    from umi_gb300 import apps
+    g = torch.Generator(device="cpu").manual_seed(h * 1000 + w + radius)
+    x = torch.randn(h, w, generator=g)
+    x[0, 0], x[h // 2, w // 2], x[h - 1, w - 1] = float("inf"), -0.0, 1e30
+    x = x.to(dev)
+    wt = torch.from_numpy(apps.gaussian_kernel(2.0, radius)).to(dev)
+    across, down = apps._gaussian_plans(h, w, 2 * radius + 1)
+    tmp, want = torch.empty_like(x), torch.empty_like(x)
+    across((x, wt), (tmp,))
+    down((tmp, wt), (want,))
+    same = lambda a, b: torch.equal(a.view(torch.int32), b.view(torch.int32))  # noqa: E731
+    assert same(apps.gaussian(x, 2.0, radius=radius), want)
+    flat = torch.full((2, h * w + 17), -7.0, device=dev)
+    o, t = flat[0, 1:1 + h * w].view(h, w), flat[1, 4:4 + h * w].view(h, w)  # out one word past a boundary
+    apps.gaussian(x, 2.0, radius=radius, out=o, tmp=t)
+    assert same(o, want) and same(t, tmp)
+    assert (flat[0, 0] == -7) and (flat[0, 1 + h * w:] == -7).all() and (flat[1, 4 + h * w:] == -7).all()
+    y = x.clone()
+    apps.gaussian(y, 2.0, radius=radius, out=y)
+    assert same(y, want)

@@ -61,6 +61,7 @@ SIGNATURES = {
     "umi_batch_run_fused": ([_vp, _i32, _vp], ctypes.c_int),
     "umi_batch_graph_add_fused": ([_vp, _vp, _i32], ctypes.c_int),
     "umi_batch_graph_destroy": ([_vp], None),
+    "umi_separable_f32": ([_vp, _vp, _i32, _i32, _i32, _vp, _vp, _vp], ctypes.c_int),
     "umi_filter3x3_f32": ([_vp, _vp, _i32, _i32, _vp, _f32, _vp], ctypes.c_int),
     "umi_filter3x3_f32_tma": ([_vp, _vp, _i32, _i32, _vp, _vp], ctypes.c_int),
     "umi_iimg_u8_i32_workspace_bytes": ([_i32, _i32], _sz),

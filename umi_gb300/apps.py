@@ -11,7 +11,8 @@ built-in strategy (no specialised kernel):
   integral image with weights +1 -1 -1 +1 (WEIGHTED_SUM_I32 over a 2 x 2
   accumulation view of stride 2r+1, coordinates clamped).
 * ``gaussian``: separable Gaussian blur, a horizontal then a vertical pass
-  of WEIGHTED_SUM_F32 with the normalised 1-D kernel; edges replicated.
+  of WEIGHTED_SUM_F32 with the normalised 1-D kernel; edges replicated.  Up
+  to 31 weights both passes are one launch (``umi_separable_f32``, same bits).
 * ``dilate`` / ``erode``: grey-level max / min over (2r+1)^2 windows
   (MAX_I32 / MIN_I32); edges replicated.
 
@@ -168,6 +169,16 @@ def _gaussian_kernel(sigma: float, radius: int | None) -> np.ndarray:
     return (k / k.sum()).astype(np.float32)
 
 
+def _one_launch(img, tmp, out, k):
+    """Whether both passes can go in one launch: few enough weights, and no
+    buffer overlaps another (each pass alone may then write what it has read)."""
+    if k > 31 or not 0 < img.shape[0] <= 1 << 20 or img.shape[1] == 0:
+        return False
+    n = 4 * img.shape[0] * img.shape[1]
+    at = [t.data_ptr() for t in (img, tmp, out) if t is not None]
+    return all(abs(a - b) >= n for i, a in enumerate(at) for b in at[:i])
+
+
 def gaussian(img, sigma: float, radius: int | None = None, out=None, tmp=None, stream=None):
     """Separable Gaussian blur of a float32 image (edges replicated)."""
     import torch
@@ -176,10 +187,15 @@ def gaussian(img, sigma: float, radius: int | None = None, out=None, tmp=None, s
     k = kern.size
     dev = img.device
     wt = _const(dev, ("gauss", float(sigma), k), lambda: kern)
-    if tmp is None:
-        tmp = torch.empty((h, w), dtype=torch.float32, device=dev)
     if out is None:
         out = torch.empty((h, w), dtype=torch.float32, device=dev)
+    if _one_launch(img, tmp, out, k):
+        U._check_memories(U.STRATEGY_WEIGHTED_SUM_F32, (img, wt), (out,) if tmp is None else (tmp, out))
+        U.check(U.lib().umi_separable_f32(U._ptr(img), U._ptr(wt), k, h, w, U._ptr(tmp), U._ptr(out),
+                                          U._stream_ptr(stream)), "umi_separable_f32")
+        return out
+    if tmp is None:
+        tmp = torch.empty((h, w), dtype=torch.float32, device=dev)
     across, down = _gaussian_plans(h, w, k)
     across((img, wt), (tmp,), stream)
     down((tmp, wt), (out,), stream)

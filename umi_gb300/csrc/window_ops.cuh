@@ -117,6 +117,35 @@ __device__ __forceinline__ void copy4(void* dst, const void* src) {
 	asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
+// rows x tw elements of im from (ys, xs) by cp.async (the caller waits).
+template <class T>
+__device__ __forceinline__ void stage_tile(const Image<T>& im, T* tile, int tw, int rows, int xs, int ys, int warp,
+                                           int lane) {
+	if (xs >= 0 && xs + tw <= im.w && ys >= 0 && ys + rows <= im.h) {
+		const T* src = im.p + (size_t)(ys + warp) * im.w + xs + lane;
+		T* dst = tile + warp * tw + lane;
+		for (int r = warp; r < rows; r += NT / 32) {
+#pragma unroll
+			for (int c = 0; c < TX; c += 32) copy4(dst + c, src + c);
+			for (int c = TX; c < tw - lane; c += 32) copy4(dst + c, src + c);
+			src += (size_t)(NT / 32) * im.w;
+			dst += (NT / 32) * tw;
+		}
+	} else {
+		for (int r = warp; r < rows; r += NT / 32) {
+			const int y = ys + r, cy = min(max(y, 0), im.h - 1);
+			const bool yout = im.pad_y && cy != y;
+			const T* row = im.p + (size_t)cy * im.w;
+			T* dst = tile + (size_t)r * tw;
+			for (int c = lane; c < tw; c += 32) {
+				const int x = xs + c, cx = min(max(x, 0), im.w - 1);
+				if (yout || (im.pad_x && cx != x)) dst[c] = im.pad;
+				else copy4(dst + c, row + cx);
+			}
+		}
+	}
+}
+
 // KX: window columns when known at compile time, else 0 (any number, four at a time).
 template <class Op, int KX>
 __global__ void __launch_bounds__(NT) window_kernel(const Args<Op> a) {
@@ -129,29 +158,7 @@ __global__ void __launch_bounds__(NT) window_kernel(const Args<Op> a) {
 	const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, kx = KX ? KX : a.kx, kxp = (kx + 3) & ~3;
 	const Image<T>& im = a.img;
 	const int rows = TY + a.ky - 1, xs = x0 + im.ox, ys = y0 + im.oy;
-	if (xs >= 0 && xs + a.tw <= im.w && ys >= 0 && ys + rows <= im.h) {
-		const T* src = im.p + (size_t)(ys + warp) * im.w + xs + lane;
-		T* dst = tile + warp * a.tw + lane;
-		for (int r = warp; r < rows; r += NT / 32) {
-#pragma unroll
-			for (int c = 0; c < TX; c += 32) copy4(dst + c, src + c);
-			for (int c = TX; c < a.tw - lane; c += 32) copy4(dst + c, src + c);
-			src += (size_t)(NT / 32) * im.w;
-			dst += (NT / 32) * a.tw;
-		}
-	} else {
-		for (int r = warp; r < rows; r += NT / 32) {
-			const int y = ys + r, cy = min(max(y, 0), im.h - 1);
-			const bool yout = im.pad_y && cy != y;
-			const T* row = im.p + (size_t)cy * im.w;
-			T* dst = tile + (size_t)r * a.tw;
-			for (int c = lane; c < a.tw; c += 32) {
-				const int x = xs + c, cx = min(max(x, 0), im.w - 1);
-				if (yout || (im.pad_x && cx != x)) dst[c] = im.pad;
-				else copy4(dst + c, row + cx);
-			}
-		}
-	}
+	stage_tile(im, tile, a.tw, rows, xs, ys, warp, lane);
 	if (Op::kWeights)
 		for (int i = threadIdx.x; i < a.ky * kx; i += NT) {
 			const int ay = i / kx, ax = i - ay * kx;
