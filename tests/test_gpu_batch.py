@@ -270,3 +270,46 @@ def test_batch_fused_rejects(umi, dev):
         umi.batch_run_fused([job, job])  # two jobs of one operator
     with pytest.raises(umi.UmiError):
         umi.batch_run_fused([(umi.OP_BILATERAL, [(x, None, x.clone())], umi.BatchParams(2, 2.0, 0.1, 0, 0), [9])])
+
+
+@pytest.mark.parametrize("lead", [0, 1, 2, 3])
+def test_wfilter_weight_rows_of_any_alignment(umi, orc, dev, lead):
+    """Weight rows staged as 16-byte pieces: tensors that start `lead` words
+    past a 16-byte boundary, widths that shift every row, one pixel, ragged
+    strips of 128; NaN around the weights (nothing outside them is used), alone
+    and in the fused launch before a bilateral of the same images."""
+    import torch
+    sizes = [(1, 1), (3, 1), (7, 3), (61, 127), (5, 128), (62, 129), (4, 256), (9, 259)]
+    xs, ws, want, ims, outs, bil = [], [], [], [], [], []
+    for i, (h, w) in enumerate(sizes):
+        g = np.random.default_rng(100 * lead + i)
+        x = g.standard_normal((h, w)).astype(np.float32)
+        wt = g.standard_normal((h, w, 3, 3)).astype(np.float32)
+        flat = torch.full((wt.size + 8,), float("nan"), device=dev)
+        t = flat[lead:lead + wt.size].view(h, w, 3, 3)
+        t.copy_(torch.from_numpy(wt))
+        ims.append((_t(x, dev), t, torch.full((h, w), -7.0, device=dev)))
+        bil.append((ims[-1][0], None, torch.empty(h, w, device=dev)))
+        xs.append(x)
+        ws.append(wt)
+        want.append(orc.wfilter_pp_f64(x, wt))
+
+    def check(tag):
+        for (x, wt, wv, im) in zip(xs, ws, want, ims):
+            got = im[2].cpu().numpy()
+            assert np.max(np.abs(got - wv) / np.maximum(np.abs(wv), _wf_scale(x, wt))) <= TOL, (tag, x.shape)
+            im[2].fill_(-7.0)
+
+    for v in range(umi.batch_variants(umi.OP_WFILTER_PP)):
+        umi.batch_run(umi.OP_WFILTER_PP, ims, variant=v)
+        check(v)
+    prm = umi.BatchParams(2, 2.0, 0.3, 0, 0)
+    umi.batch_run(umi.OP_BILATERAL, bil, prm)
+    alone = [b[2].clone() for b in bil]
+    for v in range(umi.batch_fused_variants(umi.OP_WFILTER_PP)):
+        for b in bil:
+            b[2].fill_(-7.0)
+        umi.batch_run_fused([(umi.OP_WFILTER_PP, ims, None, [v] * len(ims)), (umi.OP_BILATERAL, bil, prm, None)])
+        check(("fused", v))
+        for b, a in zip(bil, alone):
+            assert torch.allclose(b[2], a, rtol=1e-5, atol=1e-6)

@@ -130,8 +130,14 @@ struct Bilateral {
 
 // ------------------------------------------------------------------ wfilter
 // A warp owns a 128-column strip and RY rows (4 pixels per lane, halo
-// columns by shuffle, every input row loaded once); the 9 weights of 4
-// pixels are 9 float4 loads.
+// columns by shuffle, every input row loaded once).  Bound by the weights, 36
+// of its 44 bytes a pixel: a row's 128 x 9 go through the warp's shared memory
+// by 16-byte cp.async, coalesced for every alignment, the next row's under
+// this one's arithmetic.  Loaded straight from global memory each of a lane's
+// 9 (36 where a row is not aligned) loads touched 32 lines, which the L1 had to
+// keep until the last of them; beside the cost volume's 222 KB it could not.
+// Six uneven images, 6.2 M pixels: 93 -> 65 us alone, 1022 -> 915 in the launch
+// with the cost volume and the bilateral; 386 x 439: 16.3 -> 8.9 and 74 -> 35.
 struct NoParams {};
 
 __device__ __forceinline__ float4 row4(const Img& im, int y, int x) {
@@ -150,15 +156,59 @@ template <int RY, int NTH = NT>
 struct WFilter {
 	static constexpr int WARPS = NTH / 32;
 	static constexpr int TH = WARPS * RY;
-	static constexpr size_t smem = 0;
+	static constexpr int ROW = 128 * 9 + 4;  // words of a staged row: up to 3 before its first weight
+	static constexpr size_t smem = sizeof(float) * WARPS * 2 * ROW;
 	static int tiles_x(int w) { return umi::ceil_div(w, 128); }
 	static int tiles(int h, int w) { return tiles_x(w) * umi::ceil_div(h, TH); }
-	__device__ static void tile(const Img& im, int t, const NoParams&, float*) {
+	// The weights of n pixels from (y, x0) to buf, as the 16-byte pieces that
+	// hold them; returns the words before the first one.
+	__device__ static int stage(const Img& im, int y, int x0, int n, float* buf, int lane) {
+		const size_t first = ((size_t)y * im.w + x0) * 9, total = (size_t)im.h * im.w * 9;
+		const int lead = (int)(reinterpret_cast<uintptr_t>(im.aux + first) >> 2) & 3;
+		const unsigned d = (unsigned)__cvta_generic_to_shared(buf);
+		for (int j = 4 * lane; j < lead + 9 * n; j += 128) {
+			const int64_t o = (int64_t)first - lead + j;  // of this piece in the weights
+			if (o >= 0 && o + 4 <= (int64_t)total) {
+				asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 4 * j), "l"(im.aux + o) : "memory");
+			} else {  // the tensor's ends
+				for (int k = 0; k < 4; ++k)
+					if (o + k >= 0 && o + k < (int64_t)total)
+						asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * (j + k)), "l"(im.aux + o + k)
+						             : "memory");
+			}
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+		return lead;
+	}
+	// Four pixels of one row: LEAD words lie before the staged weights.
+	template <int LEAD>
+	__device__ static void pixels(const float* w, const float (&r)[RY + 2][6], int i, float (&o)[4]) {
+		float q[40];
+#pragma unroll
+		for (int k = 0; k < (LEAD ? 10 : 9); ++k) {
+			const float4 v = *reinterpret_cast<const float4*>(w + 4 * k);
+			q[4 * k] = v.x; q[4 * k + 1] = v.y; q[4 * k + 2] = v.z; q[4 * k + 3] = v.w;
+		}
+#pragma unroll
+		for (int px = 0; px < 4; ++px) {
+			float s = 0.0f;
+#pragma unroll
+			for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+				for (int dx = 0; dx < 3; ++dx) s = fmaf(q[LEAD + 9 * px + 3 * dy + dx], r[i + dy][px + dx], s);
+			o[px] = s;
+		}
+	}
+	// Waits for every cp.async of the thread, also those issued before the tile.
+	__device__ static void tile(const Img& im, int t, const NoParams&, float* sm) {
 		const int ty = t / im.tiles_x, tx = t - ty * im.tiles_x;
 		const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 		const int x0 = tx * 128, x = x0 + 4 * lane;
 		const int y0 = ty * TH + warp * RY;
 		if (y0 >= im.h) return;  // no barrier in this operator
+		const int n = min(128, im.w - x0);
+		float* buf = sm + warp * 2 * ROW;
+		int lead = stage(im, y0, x0, n, buf, lane);
 		float r[RY + 2][6];
 #pragma unroll
 		for (int i = 0; i < RY + 2; ++i) {
@@ -175,28 +225,21 @@ struct WFilter {
 		for (int i = 0; i < RY; ++i) {
 			const int y = y0 + i;
 			if (y >= im.h) break;
-			float wv[36];
-			const float* wp = im.aux + ((size_t)y * im.w + x) * 9;
-			if (im.vec && x + 3 < im.w) {
-#pragma unroll
-				for (int k = 0; k < 9; ++k) {
-					const float4 q = __ldg(reinterpret_cast<const float4*>(wp) + k);
-					wv[4 * k] = q.x; wv[4 * k + 1] = q.y; wv[4 * k + 2] = q.z; wv[4 * k + 3] = q.w;
-				}
+			const int l = lead;
+			if (i + 1 < RY && y + 1 < im.h) {
+				lead = stage(im, y + 1, x0, n, buf + ((i + 1) & 1) * ROW, lane);
+				asm volatile("cp.async.wait_group 1;" ::: "memory");
 			} else {
-#pragma unroll
-				for (int k = 0; k < 36; ++k) wv[k] = (x + k / 9 < im.w) ? __ldg(wp + k) : 0.f;
+				asm volatile("cp.async.wait_group 0;" ::: "memory");
 			}
+			__syncwarp();
+			const float* w = buf + (i & 1) * ROW + 36 * lane;
 			float o[4];
-#pragma unroll
-			for (int px = 0; px < 4; ++px) {
-				float s = 0.0f;
-#pragma unroll
-				for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-					for (int dx = 0; dx < 3; ++dx) s = fmaf(wv[9 * px + 3 * dy + dx], r[i + dy][px + dx], s);
-				o[px] = s;
-			}
+			if (l == 0) pixels<0>(w, r, i, o);
+			else if (l == 1) pixels<1>(w, r, i, o);
+			else if (l == 2) pixels<2>(w, r, i, o);
+			else pixels<3>(w, r, i, o);
+			__syncwarp();  // every lane has read the buffer that the next row's copies fill
 			float* dst = im.out + (size_t)y * im.w + x;
 			if (im.vec && x + 3 < im.w) {
 				*reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
@@ -726,6 +769,7 @@ using FWf0 = WFilter<4, FNT>;
 using FWf1 = WFilter<2, FNT>;
 using FWf2 = WFilter<1, FNT>;
 constexpr size_t kFusedSimtSmem = sizeof(float) * (96 + 6) * (60 + 6);  // one halo buffer, any bilateral variant at r <= 3
+constexpr size_t kFusedFilterSmem = std::max(2 * kFusedSimtSmem, FWf0::smem);
 
 template <int R>
 __global__ void __launch_bounds__(FNT, 1)
@@ -747,6 +791,7 @@ batch_fused_kernel(const Table cv, const cvtc::Params cvp, const Table q, const 
 	};
 	int buf = 0;
 	bool staged = false;  // the current tile's halo is already in sm[buf]
+	bool weights = false;  // the tile before was the per-pixel-weight filter's, whose warps each go on by themselves
 	for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
 		const int i = find_image(q, tile);
 		const Img& im = q.img[i];
@@ -758,8 +803,11 @@ batch_fused_kernel(const Table cv, const cvtc::Params cvp, const Table q, const 
 				default: FWf2::tile(im, lt, NoParams{}, sm); break;
 			}
 			staged = false;
+			weights = true;
 			continue;
 		}
+		if (weights) __syncthreads();  // their shared memory becomes the halo buffers
+		weights = false;
 		float* cur = sm + buf * BUFW;
 		if (!staged) stage(im, lt, cur);
 		const int next = tile + (int)gridDim.x;
@@ -835,8 +883,8 @@ template <int R>
 umi_status launch_fused_r(const Table& cv, const cvtc::Params& cvp, const Table& q, const BilParams& bp, cudaStream_t st) {
 	auto kern = batch_fused_kernel<R>;
 	const bool has_cv = cv.start[cv.n] > 0;
-	const size_t smem = has_cv ? cvtc::SMEM : 2 * kFusedSimtSmem;
-	static_assert(2 * kFusedSimtSmem <= cvtc::SMEM, "two halo buffers fit the cost volume's shared memory");
+	const size_t smem = has_cv ? cvtc::SMEM : kFusedFilterSmem;
+	static_assert(kFusedFilterSmem <= cvtc::SMEM, "the filters fit the cost volume's shared memory");
 	UMI_TRY(umi::cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cvtc::SMEM),
 	                         "cudaFuncSetAttribute"));
 	int dev = 0, sms = 0;
