@@ -78,3 +78,27 @@ def test_elim_list_and_centers(umi, orc, dev, h, w, r):
                    for dy in range(centers[i, 0] - r, centers[i, 0] + r + 1)
                    for dx in range(centers[i, 1] - r, centers[i, 1] + r + 1))
         assert tuple(got[i]) == (best[1], best[2], best[0]), i
+
+
+@pytest.mark.parametrize("r", [33, 34, 64])
+@pytest.mark.parametrize("n", [1, 150, 153, 400])
+def test_list_of_any_length(umi, orc, dev, r, n):
+    """Lists with wide windows: up to one block per SM every thread of a CTA
+    serves one block, beyond that two teams share the CTA; the length is read on
+    the GPU.  Blocks that are not listed keep what they held."""
+    import torch
+    g = np.random.default_rng(r + n)
+    h, w = 16 * 21, 16 * 20
+    cur, ref = _scene(g, h, w, 40)
+    nblk = (h // 16) * (w // 16)
+    blocks = g.permutation(nblk)[:n].astype(np.int32)
+    want = orc.full_me_u8(cur, ref, 16, r, blocks=blocks)
+    padded = np.full(nblk, -5, np.int32)
+    padded[:n] = blocks
+    mv = torch.full((nblk, 3), -99, dtype=torch.int32, device=dev)
+    umi.full_me_u8_list(_t(cur, dev), _t(ref, dev), torch.from_numpy(padded).to(dev),
+                        torch.tensor([n], dtype=torch.int32, device=dev), mv, 16, r)
+    got = mv.cpu().numpy()
+    assert np.array_equal(got[blocks], want)
+    rest = np.setdiff1d(np.arange(nblk), blocks)
+    assert (got[rest] == -99).all()

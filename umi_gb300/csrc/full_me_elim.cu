@@ -119,7 +119,7 @@ struct ElimArgs {
 	int nchunk;                 // threads per column, two passes of RC rows each (one when nd <= RC)
 	int wrows, wwords, sw;      // window: rows, words per row, row stride in words (an odd number of 16-byte pieces)
 	int qrows, ncols, spw;      // cells: rows, columns; row pieces a warp forms at a time
-	int pieces, piece_rows;     // 16-byte pieces per window row; window rows loaded at a time
+	int pieces;                 // 16-byte pieces per window row
 	int limit;                  // survivors a block may keep before it is searched exhaustively
 	int cur_words;              // cur's rows are 4-byte aligned
 	int ref_pieces;             // ref's rows are 16-byte aligned
@@ -129,6 +129,7 @@ struct ElimArgs {
 	uint32_t mul16, mul64k;     // 16 and 2^16 (runtime values: the keys stay multiply-adds, off the ALU pipe)
 	// shared memory offsets in words
 	int copy, o_copy;           // stride and start of the shifted windows (over the cell words)
+	int team_words;             // shared memory of a team
 	int o_q, o_blk, o_cell, o_list;
 };
 
@@ -244,12 +245,12 @@ __device__ __forceinline__ Run run_of(const ElimArgs& a, int unit) {
 // A run's window and blocks into shared memory, cp.async where the source is
 // aligned (words past the last block's window are loaded but not used).
 __device__ __forceinline__ void load_run(const ElimArgs& a, const Run& u, uint32_t* win, uint32_t* blkw, int row0,
-                                         int piece) {
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+                                         int piece, int piece_rows, int tid, int nt) {
+	const int warp = tid >> 5, lane = tid & 31, nwarps = nt >> 5;
 	const int gy0 = 16 * u.by + u.cy - a.r, gx0 = 16 * u.bx0 + u.cx - a.r;
 	if (a.ref_pieces && (gx0 & 15) == 0 && gx0 >= 0 && gx0 + 16 * a.pieces <= a.w) {
 		const uint8_t* src = a.ref + gx0 + 16 * piece;
-		for (int row = row0; row < a.wrows; row += a.piece_rows)
+		for (int row = row0; row < a.wrows; row += piece_rows)
 			copy16(win + row * a.sw + 4 * piece, src + (size_t)min(max(gy0 + row, 0), a.h - 1) * a.w);
 	} else {
 		const size_t total = (size_t)a.h * a.w;
@@ -274,13 +275,13 @@ __device__ __forceinline__ void load_run(const ElimArgs& a, const Run& u, uint32
 		}
 	}
 	if (a.cur_pieces) {
-		for (int i = tid; i < 16 * u.nb; i += blockDim.x) {
+		for (int i = tid; i < 16 * u.nb; i += nt) {
 			const int b = i >> 4, row = i & 15;
 			copy16(blkw + 4 * i, a.cur + (size_t)(16 * u.by + row) * a.w + 16 * (u.bx0 + b));
 		}
 		return;
 	}
-	for (int i = tid; i < 64 * u.nb; i += blockDim.x) {
+	for (int i = tid; i < 64 * u.nb; i += nt) {
 		const int b = i >> 6, row = (i >> 2) & 15, k = i & 3;
 		const size_t off = (size_t)(16 * u.by + row) * a.w;
 		const int gx = 16 * (u.bx0 + b) + 4 * k;
@@ -358,21 +359,38 @@ __device__ __forceinline__ void form_cells(const ElimArgs& a, const uint32_t* __
 	}
 }
 
-// MINB: CTAs per SM (three at 72 registers; two where shared memory holds no more).
-template <int MINB>
-__global__ void __launch_bounds__(MAXT, MINB) full_me_elim_kernel(const ElimArgs a) {
-	extern __shared__ __align__(16) uint32_t sm[];
-	__shared__ uint32_t seed[MAXNB], best[MAXNB];
-	__shared__ int cnt[MAXNB], total_cnt;
+// MINB: CTAs per SM (three at 72 registers; two where shared memory holds no
+// more).  HALVES: a list of blocks with windows of more than 66 rows, whose
+// length only the GPU knows.  One CTA per SM takes a block with all its threads
+// if the list has no more blocks than there are CTAs, and otherwise works as two
+// teams with a block each, of half the threads and shared memory, that never
+// wait for one another.  (A fallback list of 130 blocks at 1080p, +-64, most of
+// them hard: the pass around it 79 us with two CTAs per SM, 68 so; 28 000 blocks
+// at 4K: the pass 1.17 ms with all threads on each block, 0.91 so.)
+template <int MINB, bool HALVES>
+__global__ void __launch_bounds__(HALVES ? 2 * MAXT : MAXT, MINB) full_me_elim_kernel(const ElimArgs a) {
+	extern __shared__ __align__(16) uint32_t smem[];
+	__shared__ uint32_t seeds[2][MAXNB], bests[2][MAXNB];
+	__shared__ int cnts[2][MAXNB], totals[2];
+	int units = a.units;
+	if (a.list) units = min(units, *a.list_count);
+	const bool teams = HALVES && units > (int)gridDim.x;
+	const int team = teams ? (int)threadIdx.x / MAXT : 0, nteams = teams ? 2 : 1;
+	const int tid = (int)threadIdx.x - team * MAXT, nt = teams ? MAXT : (int)blockDim.x;
+	const int warp = tid >> 5, lane = tid & 31, nwarps = nt >> 5;
+	auto sync = [&] {  // the threads of this team
+		if (HALVES) asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(nt) : "memory");
+		else __syncthreads();
+	};
+	uint32_t *seed = seeds[team], *best = bests[team];
+	int *cnt = cnts[team], &total_cnt = totals[team];
+	uint32_t* sm = smem + team * a.team_words;
 	uint32_t* win = sm;              // [wrows][sw]
 	uint32_t* q = sm + a.o_q;        // [max(nd, RC) + 12][QS]: cell words
 	uint32_t* blkw = sm + a.o_blk;   // [nb][16][4]
 	uint32_t* cell = sm + a.o_cell;  // [nb][4]
 	uint32_t* list = sm + a.o_list;  // [nb * limit]: block, row, column
-	const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31, nwarps = nt >> 5;
 	const int nd = a.nd, r = a.r;
-	int units = a.units;
-	if (a.list) units = min(units, *a.list_count);
 	// this thread's column of the bound and its rows: two passes from iy0, the
 	// second one ending with row iy1 + RC - 1 (passes and threads overlap where
 	// the rows do not divide)
@@ -381,11 +399,11 @@ __global__ void __launch_bounds__(MAXT, MINB) full_me_elim_kernel(const ElimArgs
 	const int wb0 = a.div_task(tid - lane), wb1 = a.div_task(tid - lane + 31);  // the blocks of this warp's columns
 	const int gl = a.div_spw(lane), seg = lane - gl * a.spw;
 	const int prow = a.div_piece(tid), piece = tid - prow * a.pieces;
-	const int row0 = prow < a.piece_rows ? prow : a.wrows;
+	const int piece_rows = nt / a.pieces, row0 = prow < piece_rows ? prow : a.wrows;
 
-	for (int unit = blockIdx.x; unit < units; unit += gridDim.x) {
+	for (int unit = blockIdx.x * nteams + team; unit < units; unit += gridDim.x * nteams) {
 		const Run u = run_of(a, unit);
-		load_run(a, u, win, blkw, row0, piece);
+		load_run(a, u, win, blkw, row0, piece, piece_rows, tid, nt);
 		if (tid < MAXNB) {
 			seed[tid] = 0xffffffffu;
 			best[tid] = 0xffffffffu;
@@ -393,7 +411,7 @@ __global__ void __launch_bounds__(MAXT, MINB) full_me_elim_kernel(const ElimArgs
 		}
 		if (tid == 0) total_cnt = 0;
 		asm volatile("cp.async.wait_all;" ::: "memory");
-		__syncthreads();
+		sync();
 		// ---- 1. cells: cur's, by every warp for the scale; then the window's
 		uint32_t sums[NC], mn = 0xffffffffu, mx = 0;
 #pragma unroll
@@ -423,7 +441,7 @@ __global__ void __launch_bounds__(MAXT, MINB) full_me_elim_kernel(const ElimArgs
 		// lane = (group gl of 16 columns, piece `seg` of CR rows)
 		for (int s0 = warp * a.spw; s0 * CR < a.qrows; s0 += nwarps * a.spw)
 			form_cells(a, win, q, (s0 + seg) * CR, min(gl, a.pieces - 1), gl < a.pieces ? a.ncols - 16 * gl : 0, lo, sh);
-		__syncthreads();
+		sync();
 		// ---- 2. bound
 		const bool task = tb < u.nb;
 		uint32_t p0[16], p1[16], l0 = 0, l1 = 0, k0 = 0xffffffffu, k1 = 0xffffffffu;
@@ -444,7 +462,7 @@ __global__ void __launch_bounds__(MAXT, MINB) full_me_elim_kernel(const ElimArgs
 		} else if (task) {
 			atomicMin(&seed[tb], key);
 		}
-		__syncthreads();
+		sync();
 		uint32_t T = 0;
 		for (int b = wb0; b <= min(wb1, u.nb - 1); ++b) {
 			const uint32_t idx = seed[b] & 0x7fffu;
@@ -481,7 +499,7 @@ __global__ void __launch_bounds__(MAXT, MINB) full_me_elim_kernel(const ElimArgs
 				for (; m1; m1 &= m1 - 1) *dst++ = e + ((uint32_t)(iy1 + __ffs((int)m1) - 1) << 8);
 			}
 		}
-		__syncthreads();
+		sync();
 		// ---- 5. exact sums
 		int hard = 0;
 		for (int b = 0; b < u.nb; ++b) hard |= (cnt[b] > a.limit) << b;
@@ -517,7 +535,7 @@ __global__ void __launch_bounds__(MAXT, MINB) full_me_elim_kernel(const ElimArgs
 #pragma unroll
 				for (int k = 1; k < 4; ++k) copies[(k - 1) * a.copy + i] = __funnelshift_r(x, y, 8 * k);
 			}
-			__syncthreads();
+			sync();
 			const int ng = (nd + BG - 1) / BG, tasks = nd * ng, all = __popc(hard) * tasks;
 			for (int t0 = tid - lane; t0 < all; t0 += nt) {  // warp-uniform
 				const int t = min(t0 + lane, all - 1);       // lanes past the end repeat the last task
@@ -536,7 +554,7 @@ __global__ void __launch_bounds__(MAXT, MINB) full_me_elim_kernel(const ElimArgs
 				}
 			}
 		}
-		__syncthreads();
+		sync();
 		if (tid < u.nb) {
 			const uint32_t key = best[tid];
 			const int idx = (int)(key & 0x7fffu), iy = a.div_nd(idx);
@@ -545,13 +563,13 @@ __global__ void __launch_bounds__(MAXT, MINB) full_me_elim_kernel(const ElimArgs
 			o[1] = u.cx + (idx - iy * nd) - r;
 			o[2] = (int32_t)(key >> 15);
 		}
-		__syncthreads();  // a list's next block overwrites the keys and the window
+		sync();  // a list's next block overwrites the keys and the window
 	}
 }
 
-template <int MINB>
+template <int MINB, bool HALVES>
 umi_status launch(const ElimArgs& a, int threads, size_t smem, int sms, cudaStream_t st) {
-	auto kern = full_me_elim_kernel<MINB>;
+	auto kern = full_me_elim_kernel<MINB, HALVES>;
 	UMI_TRY(umi::cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
 	                         "cudaFuncSetAttribute"));
 	// a list's length is known on the GPU only: CTAs that fill it once take its blocks in turn
@@ -607,8 +625,8 @@ umi_status full_me_elim(const uint8_t* cur, const uint8_t* ref, int h, int w, in
 	a.div_piece = SmallDiv::by(a.pieces);
 	a.div_spw = SmallDiv::by(a.spw);
 	auto up4 = [](int n) { return (n + 3) & ~3; };
-	const int threads = ceil_div(a.nb * per_b, 32) * 32;
-	a.piece_rows = threads / a.pieces;
+	const bool halves = list && a.nd > 2 * RC;
+	const int threads = halves ? 2 * MAXT : ceil_div(a.nb * per_b, 32) * 32;
 	a.o_q = up4(a.wrows * a.sw + 4);
 	// the exhaustive search's copies: 8, 16, 24 banks from the window; its last
 	// row group reads up to BG - 1 rows past a window's end
@@ -617,8 +635,10 @@ umi_status full_me_elim(const uint8_t* cur, const uint8_t* ref, int h, int w, in
 	a.o_blk = up4(std::max(a.o_q + (std::max(a.nd, RC) + 12) * QS, a.o_copy + 3 * a.copy + (BG - 1) * a.sw));
 	a.o_cell = a.o_blk + 64 * a.nb;
 	a.o_list = a.o_cell + 4 * a.nb;
-	const size_t smem = 4 * (size_t)(a.o_list + a.nb * a.limit);
-	return smem > kSmemThree ? launch<2>(a, threads, smem, sms, st) : launch<3>(a, threads, smem, sms, st);
+	a.team_words = up4(a.o_list + a.nb * a.limit);
+	const size_t smem = 4 * (size_t)a.team_words;
+	if (halves) return launch<1, true>(a, threads, 2 * smem, sms, st);
+	return smem > kSmemThree ? launch<2, false>(a, threads, smem, sms, st) : launch<3, false>(a, threads, smem, sms, st);
 }
 
 }  // namespace umi
