@@ -1023,7 +1023,7 @@ class Apps1080p:
 
     def config(self):
         return {"workload": self.name, "frame": f"{self.W}x{self.H}", "ops": "census r2, dilate r1, box r7 "
-                "(integral image + 4 corner reads), gaussian sigma 2 (13 taps, two passes)",
+                "(integral image + 4 corner reads), gaussian sigma 2 (13 taps, two passes in one launch)",
                 "bytes_per_px": self.BYTES, "l2": "4 frame sets rotated (> L2)",
                 "streams": "census + dilate | box | gaussian, joined every step"}
 
@@ -1048,8 +1048,8 @@ class Apps1080p:
         self.J = [torch.zeros((self.H + 1, self.W + 1), dtype=torch.int32, device=dev) for _ in range(self.n_rot)]
         self.ws = torch.empty(U.iimg_workspace_bytes(self.H, self.W), dtype=torch.uint8, device=dev)
         self.h_out = torch.empty((self.H, self.W), dtype=torch.int32).pin_memory()
-        # census + dilate + (iimg 2 kernels + J copy + box) + gaussian 2
-        self.launches_per_step = 1 + 1 + 4 + 2
+        # census + dilate + (iimg 2 kernels + corners) + gaussian
+        self.launches_per_step = 1 + 1 + 3 + 1
         self.s1, self.s2 = torch.cuda.Stream(device=dev), torch.cuda.Stream(device=dev)
         for k in range(self.n_rot):  # constants made before any graph capture
             self.step(k)

@@ -199,6 +199,14 @@ size_t umi_iimg_u8_i32_workspace_bytes(int32_t h, int32_t w);
 umi_status umi_iimg_u8_i32(const uint8_t* in, int32_t* out, int32_t h, int32_t w, void* workspace,
                            size_t workspace_bytes, void* stream);
 
+/* Sums of a uint8 image over (2 radius + 1)^2 windows clipped to the image,
+ * radius 0..2^20: the integral image to ii, then every window's four corners
+ * from it.  J, if not NULL, receives the (h+1, w+1) integral image's interior
+ * (rows and columns from 1; its first row and column are left alone).
+ * Workspace as umi_iimg_u8_i32.  out must not overlap ii or J, nor ii J. */
+umi_status umi_box_sum_u8(const uint8_t* in, int32_t h, int32_t w, int32_t radius, int32_t* ii, int32_t* J, int32_t* out,
+                          void* workspace, size_t workspace_bytes, void* stream);
+
 /* The same integral image for callers that cannot allocate device memory
  * (no allocator to take a workspace from, or a context where cudaMalloc is
  * not allowed).  No counterpart in the reference.  The tile sums go to a

@@ -98,3 +98,30 @@ def test_gaussian_one_launch_equals_two(umi, dev, h, w, radius):
     y = x.clone()
     apps.gaussian(y, 2.0, radius=radius, out=y)
     assert same(y, want)
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (2, 5), (8, 127), (9, 129), (70, 300), (33, 2100)])
+@pytest.mark.parametrize("r", [0, 1, 7, 40, 5000])
+def test_box_sum_reads_corners_or_j(umi, dev, h, w, r):
+    """Corners straight from the integral image, with and without J, equal the
+    clipped sums; J's interior is filled, nothing outside the buffers written;
+    overlapping buffers take the way through J."""
+    import torch
+    from umi_gb300 import apps
+    x = np.random.default_rng(h * 7 + w + r).integers(0, 256, (h, w), dtype=np.uint8)
+    c = np.pad(x.astype(np.int64).cumsum(0).cumsum(1), ((1, 0), (1, 0)))
+    y0, y1 = np.maximum(np.arange(h) - r, 0), np.minimum(np.arange(h) + r + 1, h)
+    x0, x1 = np.maximum(np.arange(w) - r, 0), np.minimum(np.arange(w) + r + 1, w)
+    want = c[y1][:, x1] - c[y1][:, x0] - c[y0][:, x1] + c[y0][:, x0]
+    xd = _t(x, dev)
+    assert apps._box_direct(xd, r, None, None, None) == (r <= 1 << 20)
+    assert np.array_equal(apps.box_sum(xd, r).cpu().numpy(), want)
+    flat = torch.full((3, (h + 1) * (w + 1) + 16), -7, dtype=torch.int32, device=dev)
+    o, ii, J = flat[0, :h * w].view(h, w), flat[1, :h * w].view(h, w), flat[2, :(h + 1) * (w + 1)].view(h + 1, w + 1)
+    J.zero_()
+    assert apps._box_direct(xd, r, o, J, ii) and not apps._box_direct(xd, r, ii, J, ii)
+    got = apps.box_sum(xd, r, out=o, J=J, ii=ii)
+    assert got is o and np.array_equal(o.cpu().numpy(), want)
+    assert np.array_equal(J.cpu().numpy(), c) and np.array_equal(ii.cpu().numpy(), c[1:, 1:])
+    assert (flat[0, h * w:] == -7).all() and (flat[1, h * w:] == -7).all() and (flat[2, (h + 1) * (w + 1):] == -7).all()
+    assert np.array_equal(apps.box_sum(xd, r, out=ii, J=J, ii=ii).cpu().numpy(), want)

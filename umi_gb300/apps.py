@@ -9,7 +9,9 @@ built-in strategy (no specialised kernel):
 * ``box_sum``: sums over (2r+1)^2 windows clipped to the image, from the
   integral image (``iimg_u8_i32``): four corner reads of the zero-bordered
   integral image with weights +1 -1 -1 +1 (WEIGHTED_SUM_I32 over a 2 x 2
-  accumulation view of stride 2r+1, coordinates clamped).
+  accumulation view of stride 2r+1, coordinates clamped); buffers that do
+  not overlap take the same sums straight from the integral image
+  (``umi_box_sum_u8``).
 * ``gaussian``: separable Gaussian blur, a horizontal then a vertical pass
   of WEIGHTED_SUM_F32 with the normalised 1-D kernel; edges replicated.  Up
   to 31 weights both passes are one launch (``umi_separable_f32``, same bits).
@@ -137,6 +139,20 @@ def erode(img, radius: int = 1, out=None, stream=None):
     return _extremum(img, radius, U.STRATEGY_MIN_I32, (1 << 31) - 1, out, stream)
 
 
+def _box_direct(img, radius, out, J, ii):
+    """Whether the windows' corners can be read straight from the integral
+    image: buffers of its shape that do not overlap (through J, each step had
+    read its input before the next one wrote)."""
+    h, w = img.shape
+    if not (0 < h <= 500000 and 0 < w and isinstance(radius, int) and 0 <= radius <= 1 << 20):
+        return False
+    if (J is not None and tuple(J.shape) != (h + 1, w + 1)) or any(
+            t is not None and tuple(t.shape) != (h, w) for t in (out, ii)):
+        return False
+    at = sorted((t.data_ptr(), t.numel()) for t in (out, J, ii) if t is not None)
+    return all(a + 4 * n <= b for (a, n), (b, _) in zip(at, at[1:]))
+
+
 def box_sum(img_u8, radius: int, out=None, J=None, ii=None, workspace=None, stream=None):
     """Sums of a uint8 image over (2 radius + 1)^2 windows clipped to the
     image (int32), from its integral image.  J ((h+1, w+1) int32, first row
@@ -145,6 +161,18 @@ def box_sum(img_u8, radius: int, out=None, J=None, ii=None, workspace=None, stre
     import torch
     h, w = img_u8.shape
     dev = img_u8.device
+    if _box_direct(img_u8, radius, out, J, ii):
+        U._need(img_u8, torch.uint8, "inp")
+        ii = torch.empty((h, w), dtype=torch.int32, device=dev) if ii is None else ii
+        out = torch.empty((h, w), dtype=torch.int32, device=dev) if out is None else out
+        for name, t in (("out", ii), ("memory 0", J), ("memory 2", out)):
+            if t is not None:
+                U._need(t, torch.int32, name)
+        if workspace is None:
+            workspace = torch.empty(max(U.iimg_workspace_bytes(h, w), 16), dtype=torch.uint8, device=dev)
+        U.check(U.lib().umi_box_sum_u8(U._ptr(img_u8), h, w, radius, U._ptr(ii), U._ptr(J), U._ptr(out),
+                                       U._ptr(workspace), workspace.numel(), U._stream_ptr(stream)), "umi_box_sum_u8")
+        return out
     if J is None:
         J = torch.zeros((h + 1, w + 1), dtype=torch.int32, device=dev)  # J[y][x] = sum of img[:y, :x]
     J[1:, 1:] = U.iimg_u8_i32(img_u8, out=ii, workspace=workspace, stream=stream)
