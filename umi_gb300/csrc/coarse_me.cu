@@ -115,7 +115,8 @@ __device__ __forceinline__ uint32_t pack_cells(const uint32_t (&s)[4]) {
 // owns one word of cur's cells.
 __global__ void __launch_bounds__(NT) coarse_cells_kernel(const uint8_t* __restrict__ cur, const uint8_t* __restrict__ ref,
                                                           CoarseGeom g, bool words, uint32_t* __restrict__ cells,
-                                                          uint32_t* __restrict__ planes) {
+                                                          uint32_t* __restrict__ planes, const umi::MeZero zero) {
+	zero.run();
 	const int pww = g.pw / 4;
 	const int nplane = g.pr * pww, n = nplane + 4 * g.nblk;  // < 2^31: frames up to 2^30 pixels
 	const size_t plane_words = (size_t)nplane;
@@ -328,13 +329,14 @@ umi_status check_frame(int h, int w) {
 }
 
 umi_status centers_impl(const uint8_t* cur, const uint8_t* ref, int h, int w, int range, int32_t* centers, void* ws,
-                        cudaStream_t st) {
+                        const umi::MeZero& zero, cudaStream_t st) {
 	const CoarseGeom g(h, w);
 	const CoarseWork K(g);
 	const bool words = umi::aligned(cur, 4) && umi::aligned(ref, 4);
 	const size_t items = (size_t)g.pr * (g.pw / 4) + 4 * (size_t)g.nblk;
 	const int grid = (int)std::min<size_t>((items + NT - 1) / NT, 152 * 16);
-	coarse_cells_kernel<<<grid, NT, 0, st>>>(cur, ref, g, words, K.at<uint32_t>(ws, K.cells), K.at<uint32_t>(ws, K.planes));
+	coarse_cells_kernel<<<grid, NT, 0, st>>>(cur, ref, g, words, K.at<uint32_t>(ws, K.cells), K.at<uint32_t>(ws, K.planes),
+	                                       zero);
 	UMI_TRY(umi::launch_status("coarse_cells_kernel"));
 	auto kern = range == 60 ? coarse_search_kernel<30> : coarse_search_kernel<-1>;
 	const int runs = (g.nby + NBK - 1) / NBK * g.nbx;
@@ -365,7 +367,7 @@ extern "C" umi_status umi_me_coarse_centers_u8(const uint8_t* cur, const uint8_t
 	if (!centers) return umi::fail(UMI_ERR_INVALID_ARG, "coarse ME: null pointer");
 	if (range < 0 || range > 62 || range % 2)
 		return umi::fail(UMI_ERR_UNSUPPORTED, "coarse ME: range %d (even, 0..62)", range);
-	UMI_TRY(centers_impl(cur, ref, h, w, range, centers, workspace, umi::as_stream(stream)));
+	UMI_TRY(centers_impl(cur, ref, h, w, range, centers, workspace, umi::MeZero{}, umi::as_stream(stream)));
 	return umi::ok();
 }
 
@@ -385,7 +387,7 @@ extern "C" umi_status umi_me_coarse_u8(const uint8_t* cur, const uint8_t* ref, i
 	umi::MeAudit audit;  // the audited blocks' exhaustive search runs beside the proposal and the refine
 	UMI_TRY(umi::me_audit_begin(cur, ref, h, w, full_r, audit_stride, fb, st, &audit));
 	int32_t* centers = K.at<int32_t>(workspace, K.centers);
-	UMI_TRY(centers_impl(cur, ref, h, w, (full_r - refine_r) & ~1, centers, workspace, st));
+	UMI_TRY(centers_impl(cur, ref, h, w, (full_r - refine_r) & ~1, centers, workspace, umi::MeZero{fb.count, audit_sums}, st));
 	return umi::me_refine_fallback_finish(cur, ref, h, w, centers, refine_r, full_r, sad_threshold, audit_stride, mv,
 	                                      audit_sums, n_fallback, fb, audit, st);
 }

@@ -121,7 +121,9 @@ __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, 
 }
 
 // Search centres from the predictions: round(pred * 16), clamped to +-range.
-__global__ void centers_kernel(const float* __restrict__ pred, int32_t* __restrict__ centers, int n, int range) {
+__global__ void centers_kernel(const float* __restrict__ pred, int32_t* __restrict__ centers, int n, int range,
+                               const umi::MeZero zero) {
+	zero.run();
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 2 * n; i += gridDim.x * blockDim.x) {
 		const float v = rintf(pred[i] * 16.0f);
 		centers[i] = (int32_t)fminf(fmaxf(v, (float)-range), (float)range);
@@ -153,7 +155,9 @@ __global__ void flag_kernel(const int32_t* __restrict__ mv, int n, int stride, i
 // audit_sums[1] += exhaustive SAD of the audited blocks, searched in the
 // same list as the fallback blocks.
 __global__ void audit_sum_kernel(const int32_t* __restrict__ mv, int n, int stride,
-                                 unsigned long long* __restrict__ audit_sums) {
+                                 unsigned long long* __restrict__ audit_sums, const int32_t* __restrict__ fallback,
+                                 int32_t* __restrict__ n_fallback) {
+	if (n_fallback && blockIdx.x == 0 && threadIdx.x == 0) *n_fallback = *fallback;
 	const int na = (n + stride - 1) / stride;
 	unsigned long long s = 0;
 	for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x)
@@ -172,7 +176,9 @@ __global__ void audit_list_kernel(int32_t* __restrict__ alist, int32_t* __restri
 // The audited blocks take their exhaustive result (amv) in place of the
 // refined one (mv); audit_sums (if non-null) += (refined SAD, exhaustive SAD).
 __global__ void audit_merge_kernel(int32_t* __restrict__ mv, const int32_t* __restrict__ amv, int n, int stride,
-                                   unsigned long long* __restrict__ audit_sums) {
+                                   unsigned long long* __restrict__ audit_sums, const int32_t* __restrict__ fallback,
+                                   int32_t* __restrict__ n_fallback) {
+	if (n_fallback && blockIdx.x == 0 && threadIdx.x == 0) *n_fallback = *fallback;
 	const int na = (n + stride - 1) / stride;
 	unsigned long long s0 = 0, s1 = 0;
 	for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
@@ -572,7 +578,7 @@ extern "C" umi_status umi_me_learned_u8(const uint8_t* cur, const uint8_t* ref, 
 	UMI_TRY(infer(cur, ref, h, w, params, ws, K.at<int32_t>(ws, K.err), st));
 	int32_t* centers = K.at<int32_t>(ws, K.centers);
 	centers_kernel<<<grid_for(2 * (size_t)K.nblk), NT, 0, st>>>(K.at<float>(ws, K.pred), centers, K.nblk,
-	                                                             full_r - refine_r);
+	                                                             full_r - refine_r, umi::MeZero{fb.count, audit_sums});
 	UMI_TRY(umi::launch_status("centers_kernel"));
 	return umi::me_refine_fallback_finish(cur, ref, h, w, centers, refine_r, full_r, sad_threshold, audit_stride, mv,
 	                                      audit_sums, n_fallback, fb, audit, st);
@@ -672,24 +678,24 @@ umi_status me_refine_fallback_finish(const uint8_t* cur, const uint8_t* ref, int
 	const int nblk = (h / 16) * (w / 16);
 	void* stream = st;
 	UMI_TRY(umi_full_me_u8(cur, ref, h, w, 16, refine_r, centers, mv, stream));
-	UMI_TRY(cuda_status(cudaMemsetAsync(b.count, 0, 2 * sizeof(int32_t), st), "cudaMemsetAsync"));
-	if (audit_sums)
-		UMI_TRY(cuda_status(cudaMemsetAsync(audit_sums, 0, 2 * sizeof(unsigned long long), st), "cudaMemsetAsync"));
 	flag_kernel<<<grid_for(nblk), NT, 0, st>>>(mv, nblk, audit.active ? audit_stride : 0, sad_threshold, audit.combined,
 	                                           b.list, b.count, audit_sums);
 	UMI_TRY(launch_status("flag_kernel"));
 	UMI_TRY(umi_full_me_u8_list(cur, ref, h, w, 16, full_r, nullptr, b.list, b.count, nblk, mv, stream));
 	if (audit.combined && audit_sums) {
-		audit_sum_kernel<<<grid_for(ceil_div(nblk, audit_stride)), NT, 0, st>>>(mv, nblk, audit_stride, audit_sums);
+		audit_sum_kernel<<<grid_for(ceil_div(nblk, audit_stride)), NT, 0, st>>>(mv, nblk, audit_stride, audit_sums,
+		                                                                        b.count + 1, n_fallback);
 		UMI_TRY(launch_status("audit_sum_kernel"));
+		n_fallback = nullptr;  // written
 	} else if (audit.active && !audit.combined) {
 		if (audit.forked) {
 			UMI_TRY(cuda_status(cudaStreamWaitEvent(st, audit.done, 0), "cudaStreamWaitEvent"));
 			audit.joined = true;
 		}
 		audit_merge_kernel<<<grid_for(ceil_div(nblk, audit_stride)), NT, 0, st>>>(mv, b.amv, nblk, audit_stride,
-		                                                                          audit_sums);
+		                                                                          audit_sums, b.count + 1, n_fallback);
 		UMI_TRY(launch_status("audit_merge_kernel"));
+		n_fallback = nullptr;  // written
 	}
 	if (n_fallback)
 		UMI_TRY(cuda_status(cudaMemcpyAsync(n_fallback, b.count + 1, sizeof(int32_t), cudaMemcpyDeviceToDevice, st),

@@ -19,6 +19,21 @@ struct MeFinishBuffers {
 	int32_t* amv;    // 3 nblk: exhaustive results, written at the audited blocks' rows only
 };
 
+// What flag_kernel counts into (the list's length and the fallback blocks, the
+// audit's sums or null), cleared by a kernel of the proposal: two memsets less
+// in the chain of a pass.
+struct MeZero {
+	int32_t* count;
+	unsigned long long* audit_sums;
+#ifdef __CUDACC__
+	__device__ __forceinline__ void run() const {
+		if (blockIdx.x != 0 || threadIdx.x >= 2) return;
+		if (count) count[threadIdx.x] = 0;
+		if (audit_sums) audit_sums[threadIdx.x] = 0;
+	}
+#endif
+};
+
 // The audit's exhaustive search.  An audit of fewer blocks than SMs is
 // `combined`: its blocks join the fallback blocks' list search after the
 // refine (one round holds both).  A larger one is started before the
@@ -59,7 +74,8 @@ umi_status me_audit_begin(const uint8_t* cur, const uint8_t* ref, int h, int w, 
 // searched exhaustively (n_fallback, if non-null, receives their count);
 // then the audited blocks take their exhaustive result and add (refined
 // SAD, exhaustive SAD) to audit_sums[0..1] (if non-null).  The centres must
-// lie within +-(full_r - refine_r).
+// lie within +-(full_r - refine_r), and a kernel before this must have run
+// MeZero{b.count, audit_sums}.
 umi_status me_refine_fallback_finish(const uint8_t* cur, const uint8_t* ref, int h, int w, const int32_t* centers,
                                      int refine_r, int full_r, int32_t sad_threshold, int audit_stride, int32_t* mv,
                                      unsigned long long* audit_sums, int32_t* n_fallback, const MeFinishBuffers& b,
