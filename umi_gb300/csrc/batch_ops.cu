@@ -425,7 +425,8 @@ struct CostVolume {
 // stores take 2900 without the loads, and the loads share the load/store pipe
 // with the stores: 4490 cycles per tile in all (5200 before a tile's loads were
 // issued under the previous tile's stores).  Six uneven images of 256 to 2048
-// pixels a side with 32 channels, all three operators: 1117 -> 1024 us.  Raw rows copied to
+// pixels a side with 32 channels, all three operators: 1117 -> 1024 us (918 with the
+// filter's staged weights).  Raw rows copied to
 // shared memory first (16-byte cp.async, or bulk copies, which issue one lane
 // at a time at about 60 clocks each) and all ten warps on one tile were no
 // faster: 5400, 5400 and 4541.

@@ -1,6 +1,6 @@
 // Kernels of the motion-proposal network's training pass (learned_me.cu):
-// convolution forward / data gradient, weight gradient and head, on fp32
-// planar activations (C, H, W) with W a multiple of 4.
+// convolution forward, weight gradient and head, on fp32 planar activations
+// (C, H, W) with W a multiple of 4.  (The data gradient: menet_parts.cu.)
 //
 // The FP32 pipe bounds the pass (9.6 GFLOP per 32 -> 32 layer and direction at
 // 4K, 0.12 ms at its peak): the kernels keep it fed with packed fp32 pairs
@@ -8,10 +8,11 @@
 // slots) on register tiles of 64-72 accumulators per thread.  Measured at
 // 2160 x 3840 on a GB300, before -> now (before: scalar FMAs, 9-10 shared
 // loads per tap of two pixels or one, one partial row per 4 x 32 pixels):
-// forward and data gradient 0.39-0.45 -> 0.21-0.23 ms a layer (FMA pipe 60-64 %
-// busy, the rest is the last wave of tiles and the barriers), weight gradient
-// 0.92-1.07 -> 0.22-0.24 ms and its reduction 0.37 -> 0.008 ms, head 0.64 ->
-// 0.05 ms; forward + backward 7.5 -> 2.15 ms.
+// forward 0.39-0.45 -> 0.21-0.23 ms a layer (FMA pipe 60-64 % busy, the rest is
+// the last wave of tiles and the barriers), weight gradient 0.92-1.07 ->
+// 0.22-0.24 ms (53-58 %) and its reduction 0.37 -> 0.008 ms, head 0.64 -> 0.05
+// ms; forward + backward 7.5 -> 1.69 ms, the data gradient's part of it on the
+// tensor cores (2.15 with it on this pipe).
 #pragma once
 #include <cuda_bf16.h>
 
