@@ -94,3 +94,24 @@ def test_window_forms(umi, dev, name, k):
     if more.get("block") and name == "CENSUS_I32":
         more = {}  # another order of the bits
     _case(umi, dev, strat, g, P, img, off[0], off[1], win[0], win[1], stride[0], stride[1], mode, **more)
+
+
+@pytest.mark.parametrize("h,w", [(33, 129), (32, 128), (65, 257), (1, 385), (97, 131)])
+def test_window_last_tiles(umi, dev, h, w):
+    """Tiles of which the image fills one row or one column: only what their
+    outputs use is staged."""
+    import torch
+    from umi_gb300 import apps
+    x = np.random.default_rng(h + w).integers(-1000, 1000, (h, w)).astype(np.int32)
+    xd = torch.from_numpy(x).to(dev)
+    for r in (1, 3, 6):
+        p = np.pad(x, r, mode="edge")
+        win = np.stack([p[i:i + h, j:j + w] for i in range(2 * r + 1) for j in range(2 * r + 1)])
+        assert np.array_equal(apps.dilate(xd, r).cpu().numpy(), win.max(0))
+        assert np.array_equal(apps.erode(xd, r).cpu().numpy(), win.min(0))
+    c = np.zeros((h, w), np.uint32)
+    p = np.pad(x, 2, mode="edge")
+    for i in range(5):
+        for j in range(5):
+            c = (c << 1) | (p[i:i + h, j:j + w] < x)
+    assert np.array_equal(apps.census(xd, 2).cpu().numpy().view(np.uint32), c.astype(np.uint32))

@@ -50,7 +50,8 @@ __global__ void __launch_bounds__(NT) separable_kernel(const SepArgs a) {
 	float* ws = mid + rows * TX;       // [k]
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
-	umi_window::stage_tile(a.img, tile, a.tw, rows, x0 + a.img.ox, y0 + a.img.oy, warp, lane);
+	umi_window::stage_tile(a.img, tile, a.tw, rows, x0 + a.img.ox, y0 + a.img.oy, min(TY, a.h - y0) + k - 1,
+	                       min(TX, a.w - x0) + k - 1, warp, lane);
 	for (int i = threadIdx.x; i < k; i += NT) ws[i] = __ldg(a.wts + i);
 	asm volatile("cp.async.wait_all;" ::: "memory");
 	__syncthreads();

@@ -117,10 +117,14 @@ __device__ __forceinline__ void copy4(void* dst, const void* src) {
 	asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-// rows x tw elements of im from (ys, xs) by cp.async (the caller waits).
+// rows x tw elements of im from (ys, xs) by cp.async (the caller waits).  Where
+// the tile leaves the image only the urows x ucols that its outputs use: a tile
+// of one output column would copy the edge pixel to 131 places of every row,
+// one lane after the other (1080 x 1921, dilation 3x3 10.7 -> 6.5 us, 13-tap
+// blur 16.0 -> 10.5).
 template <class T>
-__device__ __forceinline__ void stage_tile(const Image<T>& im, T* tile, int tw, int rows, int xs, int ys, int warp,
-                                           int lane) {
+__device__ __forceinline__ void stage_tile(const Image<T>& im, T* tile, int tw, int rows, int xs, int ys, int urows,
+                                           int ucols, int warp, int lane) {
 	if (xs >= 0 && xs + tw <= im.w && ys >= 0 && ys + rows <= im.h) {
 		const T* src = im.p + (size_t)(ys + warp) * im.w + xs + lane;
 		T* dst = tile + warp * tw + lane;
@@ -132,12 +136,12 @@ __device__ __forceinline__ void stage_tile(const Image<T>& im, T* tile, int tw, 
 			dst += (NT / 32) * tw;
 		}
 	} else {
-		for (int r = warp; r < rows; r += NT / 32) {
+		for (int r = warp; r < urows; r += NT / 32) {
 			const int y = ys + r, cy = min(max(y, 0), im.h - 1);
 			const bool yout = im.pad_y && cy != y;
 			const T* row = im.p + (size_t)cy * im.w;
 			T* dst = tile + (size_t)r * tw;
-			for (int c = lane; c < tw; c += 32) {
+			for (int c = lane; c < ucols; c += 32) {
 				const int x = xs + c, cx = min(max(x, 0), im.w - 1);
 				if (yout || (im.pad_x && cx != x)) dst[c] = im.pad;
 				else copy4(dst + c, row + cx);
@@ -158,7 +162,7 @@ __global__ void __launch_bounds__(NT) window_kernel(const Args<Op> a) {
 	const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, kx = KX ? KX : a.kx, kxp = (kx + 3) & ~3;
 	const Image<T>& im = a.img;
 	const int rows = TY + a.ky - 1, xs = x0 + im.ox, ys = y0 + im.oy;
-	stage_tile(im, tile, a.tw, rows, xs, ys, warp, lane);
+	stage_tile(im, tile, a.tw, rows, xs, ys, min(TY, a.h - y0) + a.ky - 1, min(TX, a.w - x0) + kx - 1, warp, lane);
 	if (Op::kWeights)
 		for (int i = threadIdx.x; i < a.ky * kx; i += NT) {
 			const int ay = i / kx, ax = i - ay * kx;
