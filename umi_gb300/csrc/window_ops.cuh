@@ -329,7 +329,8 @@ constexpr int kMaxTile = 96 * 1024;  // bytes of shared memory for the staged ti
 // Runs the plan if it is a window operator of `Op` (memories: [centre,] image
 // [, weights], output); *done says whether it did.  What is left to the
 // generic kernel: other P or A spaces, a window in several accumulation
-// blocks (another order), outer image dimensions, indices beyond 32 bits.
+// blocks (another order), outer image dimensions, images whose rows or elements
+// are not contiguous, indices beyond 32 bits.
 //
 // 1080p on a GB300, us per launch under ncu (cold caches), generic kernel ->
 // window kernel: census 5x5 51.5 -> 12.9, 3x3 37.8 -> 9.8; dilation 3x3 35.2
@@ -351,6 +352,8 @@ umi_status window_launch(const umi_plan& plan, const UMI::gpu_detail::LinearMaps
 	auto image = [&](int m, Image<T>* im) {
 		const umi_mem_plan& mp = plan.mem[m];
 		if (mp.size[0] < 1 || mp.size[1] < 1 || mp.size[2] < 1 || mp.size[3] < 1) return false;
+		// a plan's row strides may be the caller's own (rows of a pitched image)
+		if (mp.rowstride[3] != 1 || mp.rowstride[2] != mp.size[3]) return false;
 		im->p = static_cast<const T*>(in[m]);
 		im->h = mp.size[2]; im->w = mp.size[3];
 		im->oy = mp.base[2]; im->ox = mp.base[3];
