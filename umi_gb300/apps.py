@@ -61,7 +61,22 @@ def _img(h, w, mode=WRAP, a_view=None, stage=1, out=False):
     return m
 
 
-@functools.lru_cache(maxsize=64, typed=True)
+_PLAIN = (int, float, bool, str, type(None))
+
+
+def _kept(make):
+    """make(...) with its last results kept.  Arguments that are not plain values
+    (an array or a tensor, which its owner may change) are computed anew."""
+    kept = functools.lru_cache(maxsize=64, typed=True)(make)
+
+    @functools.wraps(make)
+    def get(*args):
+        plain = all(type(a) in _PLAIN or isinstance(a, np.generic) for a in args)
+        return (kept if plain else make)(*args)
+    return get
+
+
+@_kept
 def _census_plan(h, w, radius):
     k = 2 * radius + 1
     d = U.make_desc(p=_p(h, w), a=[(1, 1), (1, 1), (k, k), (k, k)],
@@ -69,7 +84,7 @@ def _census_plan(h, w, radius):
     return U.PlannedLaunch(d, U.STRATEGY_CENSUS_I32)
 
 
-@functools.lru_cache(maxsize=64, typed=True)
+@_kept
 def _extremum_plan(h, w, radius, strategy, init):
     k = 2 * radius + 1
     d = U.make_desc(p=_p(h, w), a=[(1, 1), (1, 1), (k, k), (k, k)],
@@ -77,7 +92,7 @@ def _extremum_plan(h, w, radius, strategy, init):
     return U.PlannedLaunch(d, strategy, [init])
 
 
-@functools.lru_cache(maxsize=64, typed=True)
+@_kept
 def _box_plan(h, w, radius):
     k = 2 * radius + 1
     # corner (a_y, a_x) of point (y, x): J[clamp(y - r + a_y k)][clamp(x - r + a_x k)]
@@ -89,7 +104,7 @@ def _box_plan(h, w, radius):
     return U.PlannedLaunch(d, U.STRATEGY_WEIGHTED_SUM_I32, [0])
 
 
-@functools.lru_cache(maxsize=64, typed=True)
+@_kept
 def _gaussian_plans(h, w, k):
     r = k // 2
     dh = U.make_desc(p=_p(h, w), a=[(1, 1), (1, 1), (1, 1), (k, k)],
@@ -189,7 +204,7 @@ def gaussian_kernel(sigma: float, radius: int | None = None) -> np.ndarray:
     return _gaussian_kernel(sigma, radius).copy()
 
 
-@functools.lru_cache(maxsize=64, typed=True)
+@_kept
 def _gaussian_kernel(sigma: float, radius: int | None) -> np.ndarray:
     r = int(math.ceil(3 * sigma)) if radius is None else int(radius)
     t = np.arange(-r, r + 1, dtype=np.float64)
