@@ -18,6 +18,16 @@ umi_status cuda_status(cudaError_t e, const char* what);
 // Checks the launch that was just issued (cudaGetLastError).
 inline umi_status launch_status(const char* what) { return cuda_status(cudaGetLastError(), what); }
 
+// Lets a kernel that takes shared memory by the size of its work use as much as
+// there is (4 KB of the 227 left to its static arrays).  The limit belongs to
+// the function, not to a launch: set to what one launch needs, it would refuse
+// another host thread's larger launch between that one's setting and its launch.
+constexpr int kMaxDynamicShared = 223 * 1024;
+template <class K> umi_status allow_shared(K* kern) {
+	return cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicShared),
+	                   "cudaFuncSetAttribute");
+}
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 template <class T> constexpr T ceil_div(T a, T b) { return (a + b - 1) / b; }
