@@ -146,3 +146,12 @@ def test_iimg_workspace_contract(umi):
     p16 = (p + 15) & ~15
     assert L.umi_iimg_u8_i32(ctypes.c_void_p(p16), ctypes.c_void_p(p16), 1080, 1920, ctypes.c_void_p(p16), 16,
                              None) == 5
+
+
+def test_menet_backward_refuses_a_misaligned_workspace(umi):
+    """Before anything is launched (no GPU is needed to be told)."""
+    L, p = umi.lib(), ctypes.c_void_p(1 << 20)
+    for at in (32, 16, 4, 1):
+        st = L.umi_menet_backward(p, 2, 64, 64, p, p, None, ctypes.c_void_p((1 << 20) + at), 1 << 40, None)
+        assert L.umi_status_string(st) == b"UMI_ERR_INVALID_ARG"
+        assert b"alignment" in L.umi_last_error_string()

@@ -508,6 +508,7 @@ extern "C" umi_status umi_menet_backward(const int32_t* target, int32_t target_s
 	if (!target || !params || !grads || !workspace) return umi::fail(UMI_ERR_INVALID_ARG, "menet_backward: null pointer");
 	const Work K(h, w);
 	if (workspace_bytes < K.bytes) return umi::fail(UMI_ERR_NO_MEMORY, "menet_backward: workspace too small");
+	if (!umi::aligned(workspace, 256)) return umi::fail(UMI_ERR_INVALID_ARG, "menet_backward: workspace alignment");
 	const Layout& L = layout();
 	const cudaStream_t st = umi::as_stream(stream);
 	void* ws = workspace;
