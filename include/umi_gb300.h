@@ -280,9 +280,16 @@ umi_status umi_menet_forward(const uint8_t* cur, const uint8_t* ref, int32_t h, 
  * prediction and target/16 (target: int32 vectors (mv_y, mv_x) per block at
  * target[k*target_stride], target[k*target_stride+1]).  Writes the full
  * gradient (param_count floats) to grads and, when loss is not NULL, the
- * loss (one float, device). */
+ * loss (one float, device).  The data gradients run on the tensor cores, with
+ * bounded waits: where one gave up, the gradients of the layers below are NaN. */
 umi_status umi_menet_backward(const int32_t* target, int32_t target_stride, int32_t h, int32_t w, const float* params,
                               float* grads, float* loss, void* workspace, size_t workspace_bytes, void* stream);
+/* The same; err (device, may be NULL) also receives the error bits of waits
+ * that gave up (0 when all is well), and wait_ns, if not 0, limits the wait for
+ * a finished row (1 s otherwise): the timeout path's test hook. */
+umi_status umi_menet_backward_err(const int32_t* target, int32_t target_stride, int32_t h, int32_t w, const float* params,
+                                  float* grads, float* loss, int32_t* err, unsigned long long wait_ns, void* workspace,
+                                  size_t workspace_bytes, void* stream);
 /* Inference forward pass (the one umi_me_learned_u8 runs): layer 1 on the
  * FP32 pipe, layers 2-4 on the tensor cores (tcgen05, bf16 activations,
  * fp32 accumulation), activations rounded to bf16 after each ReLU; pred (may

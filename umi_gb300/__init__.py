@@ -77,6 +77,7 @@ SIGNATURES = {
     "umi_menet_workspace_bytes": ([_i32, _i32], _sz),
     "umi_menet_forward": ([_vp, _vp, _i32, _i32, _vp, _vp, _vp, _sz, _vp], ctypes.c_int),
     "umi_menet_backward": ([_vp, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _sz, _vp], ctypes.c_int),
+    "umi_menet_backward_err": ([_vp, _i32, _i32, _i32, _vp, _vp, _vp, _vp, ctypes.c_ulonglong, _vp, _sz, _vp], ctypes.c_int),
     "umi_menet_adam": ([_vp, _vp, _vp, _vp, _i32, _f32, _vp], ctypes.c_int),
     "umi_menet_infer": ([_vp, _vp, _i32, _i32, _vp, _vp, _vp, _vp, _sz, _vp], ctypes.c_int),
     "umi_me_learned_u8": ([_vp, _vp, _i32, _i32, _vp, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _sz, _vp],
@@ -476,12 +477,14 @@ class MeNet:
                                     _ptr(self.ws), self.ws.numel(), _stream_ptr(stream)), "umi_menet_infer")
         return pred
 
-    def backward(self, target, stride: int = 2, stream=None):
+    def backward(self, target, stride: int = 2, stream=None, err=None, wait_ns: int = 0):
+        """Gradients of the last forward's loss (umi_menet_backward_err); err: an
+        int32 CUDA word for the bits of device waits that gave up (check_err)."""
         import torch
         _need(target, torch.int32, "target")
-        check(lib().umi_menet_backward(_ptr(target), stride, self.h, self.w, _ptr(self.params), _ptr(self.grads),
-                                       _ptr(self.loss), _ptr(self.ws), self.ws.numel(), _stream_ptr(stream)),
-              "umi_menet_backward")
+        check(lib().umi_menet_backward_err(_ptr(target), stride, self.h, self.w, _ptr(self.params), _ptr(self.grads),
+                                           _ptr(self.loss), _ptr(err), wait_ns, _ptr(self.ws), self.ws.numel(),
+                                           _stream_ptr(stream)), "umi_menet_backward")
         return self.grads
 
     def adam(self, lr: float, stream=None):

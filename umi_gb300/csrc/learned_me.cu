@@ -28,7 +28,7 @@ umi_status menet_conv_tc(const void* in, void* out, const void* wpack, const flo
 // The layers' data gradient on the tensor cores at fp32 accuracy (menet_parts.cu).
 umi_status menet_to_parts(const float* in, void* parts, int P, cudaStream_t st);
 umi_status menet_dgrad(const void* parts, const void* wpack, const float* mask, float* out, void* out_parts, int h, int w,
-                       int dil, int* err, cudaStream_t st);
+                       int dil, int* err, unsigned long long wait_ns, cudaStream_t st);
 }
 
 namespace {
@@ -402,8 +402,9 @@ umi_status wgrad_dil(const float* in, const float* dpre, float* part, const Work
 }
 
 // out[0 .. cols) (and *extra, the column after them) = sums of the partial rows.
-umi_status reduce_rows(const float* part, float* out, float* extra, int n, int m, int cols, cudaStream_t st) {
-	menet_train::reduce_rows_kernel<<<umi::ceil_div(m, 32), NT, 0, st>>>(part, out, extra, n, m, cols);
+umi_status reduce_rows(const float* part, float* out, float* extra, int n, int m, int cols, const int32_t* err,
+                       int32_t* report, cudaStream_t st) {
+	menet_train::reduce_rows_kernel<<<umi::ceil_div(m, 32), NT, 0, st>>>(part, out, extra, n, m, cols, err, report);
 	return umi::launch_status("reduce_rows_kernel");
 }
 
@@ -501,9 +502,10 @@ extern "C" umi_status umi_menet_forward(const uint8_t* cur, const uint8_t* ref, 
 	return umi::ok();
 }
 
-extern "C" umi_status umi_menet_backward(const int32_t* target, int32_t target_stride, int32_t h, int32_t w,
-                                         const float* params, float* grads, float* loss, void* workspace,
-                                         size_t workspace_bytes, void* stream) {
+extern "C" umi_status umi_menet_backward_err(const int32_t* target, int32_t target_stride, int32_t h, int32_t w,
+                                             const float* params, float* grads, float* loss, int32_t* err,
+                                             unsigned long long wait_ns, void* workspace, size_t workspace_bytes,
+                                             void* stream) {
 	UMI_TRY(check_frame(h, w));
 	if (!target || !params || !grads || !workspace) return umi::fail(UMI_ERR_INVALID_ARG, "menet_backward: null pointer");
 	const Work K(h, w);
@@ -514,12 +516,13 @@ extern "C" umi_status umi_menet_backward(const int32_t* target, int32_t target_s
 	void* ws = workspace;
 	float* dcur = K.at<float>(ws, K.dA[0]);
 	float* dnext = K.at<float>(ws, K.dA[1]);
+	int32_t* bits = K.at<int32_t>(ws, K.err);  // of this pass's waits, cleared by its first kernel
 	const int htx = umi::ceil_div(K.nbx, 8), htiles = htx * K.nby, nh = std::min(htiles, menet_train::HEAD_PARTS);
 	menet_train::head_bwd_kernel<<<nh, NT, 0, st>>>(K.at<float>(ws, K.act[NL - 1]), params + L.wh,
 	                                                K.at<float>(ws, K.pred), target, target_stride, dcur,
-	                                                K.at<float>(ws, K.hpart), K.H4, K.W4, K.nbx, K.nblk, htx, htiles);
+	                                                K.at<float>(ws, K.hpart), K.H4, K.W4, K.nbx, K.nblk, htx, htiles, bits);
 	UMI_TRY(umi::launch_status("head_bwd_kernel"));
-	UMI_TRY(reduce_rows(K.at<float>(ws, K.hpart), grads + L.wh, loss, nh, 2 * HEADF + 3, 2 * HEADF + 2, st));
+	UMI_TRY(reduce_rows(K.at<float>(ws, K.hpart), grads + L.wh, loss, nh, 2 * HEADF + 3, 2 * HEADF + 2, bits, nullptr, st));
 	void *din = K.at<void>(ws, K.parts[0]), *dout = K.at<void>(ws, K.parts[1]);
 	UMI_TRY(umi::menet_to_parts(dcur, din, K.P, st));
 	const int units = umi::ceil_div(K.W4, 32) * K.H4, per = umi::ceil_div(units, menet_train::PARTS);
@@ -536,15 +539,22 @@ extern "C" umi_status umi_menet_backward(const int32_t* target, int32_t target_s
 			UMI_TRY(umi::launch_status("wgrad_first_kernel"));
 		}
 		// grads[w_l], then grads[b_l] right after it (same layout as the partial rows)
-		UMI_TRY(reduce_rows(part, grads + L.w[l], nullptr, grid, m, m, st));
+		UMI_TRY(reduce_rows(part, grads + L.w[l], nullptr, grid, m, m, bits, l == 0 ? err : nullptr, st));
 		if (l > 0) {  // data gradient, masked by ReLU(a_{l-1})
 			UMI_TRY(umi::menet_dgrad(din, K.at<void>(ws, K.wt[l]), K.at<float>(ws, K.act[l - 1]), dnext,
-			                         l > 1 ? dout : nullptr, K.H4, K.W4, DIL[l], K.at<int32_t>(ws, K.err), st));
+			                         l > 1 ? dout : nullptr, K.H4, K.W4, DIL[l], bits, wait_ns, st));
 			std::swap(dcur, dnext);
 			std::swap(din, dout);
 		}
 	}
 	return umi::ok();
+}
+
+extern "C" umi_status umi_menet_backward(const int32_t* target, int32_t target_stride, int32_t h, int32_t w,
+                                         const float* params, float* grads, float* loss, void* workspace,
+                                         size_t workspace_bytes, void* stream) {
+	return umi_menet_backward_err(target, target_stride, h, w, params, grads, loss, nullptr, 0, workspace, workspace_bytes,
+	                              stream);
 }
 
 extern "C" umi_status umi_menet_adam(float* params, const float* grads, float* m, float* v, int32_t step, float lr,

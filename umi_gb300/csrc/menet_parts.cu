@@ -60,6 +60,7 @@ struct PartsArgs {
 	uint4* out_parts;    // or null
 	int h, w, dil, xtiles;
 	int* err;
+	unsigned long long acc_wait_ns;  // limit of the epilogue's wait for a finished row (kWaitNs)
 };
 
 // a = p0 + p1 + p2 exactly, each the upper half of an fp32 word; an infinity is its own first part
@@ -250,8 +251,9 @@ __global__ void __launch_bounds__(THREADS, 1)
 		const int qd = warp & 3, grp = (warp - 2) >> 2, P = g.h * g.w;
 		for (int r = grp; t0 + r < t1; r += 2) {
 			const int id = t0 + r, sl = umi_roll::slot<SLOTS>(r);
-			if (!mbar_wait(&accfull[sl], (uint32_t)(r / SLOTS) & 1, abort_flag, g.err, kErrTimeoutAccum)) break;
 			__syncwarp();  // lanes without a pixel skip the stores below
+			if (!mbar_wait_warp(&accfull[sl], (uint32_t)(r / SLOTS) & 1, abort_flag, g.err, kErrTimeoutAccum, g.acc_wait_ns))
+				break;
 			tc_fence_after();
 			const uint32_t acc = tmem + ((uint32_t)(32 * qd) << 16) + 32u * (uint32_t)sl;
 			float v[CH], t[CH];
@@ -303,9 +305,10 @@ umi_status menet_to_parts(const float* in, void* parts, int P, cudaStream_t st) 
 
 // The 3x3 convolution of dilation dil of parts (h, w, 96) with wpack (32, 9*32)
 // bf16 K-major (tap-major, then input channel), zero where !(mask > 0), to out
-// (NCHW fp32) and out_parts (or null).
+// (NCHW fp32) and out_parts (or null).  A wait that gives up leaves rows
+// unwritten and its bit in *err; wait_ns: the epilogue's limit (0: kWaitNs).
 umi_status menet_dgrad(const void* parts, const void* wpack, const float* mask, float* out, void* out_parts, int h, int w,
-                       int dil, int* err, cudaStream_t st) {
+                       int dil, int* err, unsigned long long wait_ns, cudaStream_t st) {
 	if (dil < 1 || dil > MAXD) return fail(UMI_ERR_UNSUPPORTED, "menet gradient: dilation %d", dil);
 	auto enc = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(tma_encode_fn());
 	if (!enc) return fail(UMI_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
@@ -330,7 +333,8 @@ umi_status menet_dgrad(const void* parts, const void* wpack, const float* mask, 
 		                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 		if (rr != CUDA_SUCCESS) return fail(UMI_ERR_CUDA, "menet gradient: weight tensor map (%d)", (int)rr);
 	}
-	const PartsArgs g{mask, out, static_cast<uint4*>(out_parts), h, w, dil, ceil_div(w, BM), err};
+	const PartsArgs g{mask, out, static_cast<uint4*>(out_parts), h, w, dil, ceil_div(w, BM), err,
+	                  wait_ns ? wait_ns : kWaitNs};
 	UMI_TRY(cuda_status(cudaFuncSetAttribute(menet_dgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM),
 	                    "cudaFuncSetAttribute"));
 	int dev = 0, sms = 0;

@@ -495,9 +495,12 @@ __global__ void __launch_bounds__(NT, 2) wgrad_first_kernel(const float* __restr
 
 // out[j] = sum over the n rows of the row-major (n, m) array, j < m - (extra
 // != null), in a fixed order; the last column goes to *extra when given.  A
-// CTA takes 32 columns, its 8 warps every 8th row each.
+// CTA takes 32 columns, its 8 warps every 8th row each.  Where a data gradient
+// that the rows come from is not complete (bits in *err) the sums are NaN, and
+// the bits are added to *report when given.
 __global__ void __launch_bounds__(NT) reduce_rows_kernel(const float* __restrict__ part, float* __restrict__ out,
-                                                         float* __restrict__ extra, int n, int m, int cols) {
+                                                         float* __restrict__ extra, int n, int m, int cols,
+                                                         const int32_t* __restrict__ err, int32_t* __restrict__ report) {
 	__shared__ float red[8][32];
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = blockIdx.x * 32 + lane;
 	float s[4] = {0.f, 0.f, 0.f, 0.f};
@@ -514,6 +517,9 @@ __global__ void __launch_bounds__(NT) reduce_rows_kernel(const float* __restrict
 		float t = 0.0f;
 #pragma unroll
 		for (int k = 0; k < 8; ++k) t += red[k][lane];
+		const int32_t bits = *err;
+		if (bits) t = __int_as_float(0x7fffffff);
+		if (bits && report && j == 0) atomicOr(report, bits);
 		if (j < cols) out[j] = t;
 		else if (extra) *extra = t;
 	}
@@ -563,13 +569,15 @@ __global__ void __launch_bounds__(NT) head_fwd_kernel(const float* __restrict__ 
 __global__ void __launch_bounds__(NT) head_bwd_kernel(const float* __restrict__ a4, const float* __restrict__ wh,
                                                       const float* __restrict__ pred, const int32_t* __restrict__ target,
                                                       int tstride, float* __restrict__ dpre4, float* __restrict__ part,
-                                                      int H4, int W4, int nbx, int nblk, int tiles_x, int tiles) {
+                                                      int H4, int W4, int nbx, int nblk, int tiles_x, int tiles,
+                                                      int32_t* __restrict__ err) {
 	constexpr int RS = 36, CS = 4 * RS;  // row and channel strides of the tile: 16-byte reads and feature reads spread over the banks
 	__shared__ __align__(16) float ws[2 * HEADF];
 	__shared__ __align__(16) float tile[CH * CS];
 	__shared__ float2 sg[8];
 	__shared__ float sl[8];
 	const int tid = threadIdx.x;
+	if (blockIdx.x == 0 && tid == 0) *err = 0;  // the data gradients' error word
 	for (int i = tid; i < 2 * HEADF; i += NT) ws[i] = __bfloat162float(__float2bfloat16_rn(wh[i]));
 	const float inv = 1.0f / (float)nblk;
 	const size_t P = (size_t)H4 * W4;

@@ -98,6 +98,39 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 	return true;
 }
 
+// The same with a limit shorter than try_wait may suspend the thread for (a
+// test's): asks without suspending, and gives up once limit_ns have passed.
+__device__ __forceinline__ bool mbar_poll(uint64_t* bar, uint32_t parity, volatile int* abort, int* err, int code,
+                                          unsigned long long limit_ns) {
+	const unsigned long long t0 = gtimer();
+	for (;;) {
+		uint32_t ok;
+		asm volatile(
+			"{\n\t.reg .pred p;\n\t"
+			"mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+			"selp.u32 %0, 1, 0, p;\n\t}"
+			: "=r"(ok)
+			: "r"(smem_u32(bar)), "r"(parity)
+			: "memory");
+		if (ok) return true;
+		if (*abort) return false;
+		if (gtimer() - t0 + 1 >= limit_ns) {
+			*abort = 1;
+			if (err) atomicOr(err, code);
+			return false;
+		}
+	}
+}
+
+// mbar_wait by a whole warp that goes on to a warp-wide instruction (a TMEM
+// load): the warp gives up if one of its lanes did.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort, int* err, int code,
+                                               unsigned long long limit_ns = kWaitNs) {
+	const bool ok = limit_ns == kWaitNs ? mbar_wait(bar, parity, abort, err, code)
+	                                    : mbar_poll(bar, parity, abort, err, code, limit_ns);
+	return __all_sync(0xffffffffu, ok);
+}
+
 // ---- TMA (tiled tensor loads into shared memory, completion on an mbarrier)
 __device__ __forceinline__ void tma_prefetch(const CUtensorMap* m) {
 	asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

@@ -26,7 +26,7 @@ import time
 
 import numpy as np
 
-from . import MeNet, full_me_u8, full_me_u8_list, init_params, param_count
+from . import MeNet, check_err, full_me_u8, full_me_u8_list, init_params, param_count
 from .workloads import me_pair_cuda
 
 MAGIC = b"UMIMENET"
@@ -111,6 +111,7 @@ def train(pairs: int = 2000, epochs: int = 3, lr: float = 2e-3, h: int = 2160, w
     torch.cuda.synchronize()
     print(json.dumps({"labels_s": round(time.time() - t0, 2), "pairs": pairs}), flush=True)
     total = pairs * epochs
+    err = torch.zeros(1, dtype=torch.int32, device=net.device)
     order = np.random.Generator(np.random.PCG64(seed)).permutation
     t0 = time.time()
     run = 0.0
@@ -121,9 +122,10 @@ def train(pairs: int = 2000, epochs: int = 3, lr: float = 2e-3, h: int = 2160, w
                 break
             cur, ref, _ = me_pair_cuda(TRAIN_SEED0 + int(i), h, w)
             net.forward(cur, ref)
-            net.backward(labels[int(i)], stride=3)
+            net.backward(labels[int(i)], stride=3, err=err)
             net.adam(lr_at(step, total, lr))
             if (step + 1) % log_every == 0:
+                check_err(err, "umi_menet_backward")
                 run = float(net.loss.item())
                 print(json.dumps({"step": step + 1, "epoch": e, "loss": round(run, 5),
                                   "s": round(time.time() - t0, 1)}), flush=True)
