@@ -619,7 +619,7 @@ __device__ __forceinline__ void cv_tc_phase(const Table& t, const cvtc::Params& 
 		for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++i) {
 			const int s = i & 1;
 			const uint32_t use = (uint32_t)(i >> 1);
-			if (!mbar_wait(&accfull[s], use & 1, abort_flag, err, kErrTimeoutAccum)) break;
+			if (!mbar_wait_warp(&accfull[s], use & 1, abort_flag, err, kErrTimeoutAccum)) break;
 			tc_fence_after();
 			const int idx = find_image(t, tile);
 			const Img& im = t.img[idx];

@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 		for (int id = blockIdx.x; id < ntiles; id += gridDim.x, ++i) {
 			const int a = i & 1;
 			const uint32_t use = (uint32_t)(i >> 1);
-			if (!mbar_wait(&accfull[a], use & 1, abort_flag, g.err, kErrTimeoutAccum, P::acc_wait_ns(g))) break;
+			if (!mbar_wait_warp(&accfull[a], use & 1, abort_flag, g.err, kErrTimeoutAccum, P::acc_wait_ns(g))) break;
 			tc_fence_after();
 			const typename P::Tile t = P::tile(g, id);
 #pragma unroll 1
@@ -527,7 +527,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
 		uint32_t nst = 0;  // blocks stored by this warp
 		for (int id = pair0; id < ntiles; id += npairs, ++i) {
 			const int a = i & 1;
-			if (!mbar_wait(&accfull[a], (uint32_t)(i >> 1) & 1, abort_flag, g.err, kErrTimeoutAccum, g.acc_wait_ns)) break;
+			if (!mbar_wait_warp(&accfull[a], (uint32_t)(i >> 1) & 1, abort_flag, g.err, kErrTimeoutAccum, g.acc_wait_ns)) break;
 			tc_fence_after();
 			const int row0 = (id / nt) * 2 * BM + (int)rank * BM + 32 * qd, n0 = (id % nt) * BN;
 #pragma unroll 1
@@ -846,7 +846,7 @@ __global__ void __launch_bounds__(run_threads<T>(), 1)
 		for (int id = t0; id < t1; ++id, ++i) {
 			const int a = i & 1;
 			const uint32_t use = (uint32_t)(i >> 1);
-			if (!mbar_wait(&accfull[a], use & 1, abort_flag, g.err, kErrTimeoutAccum)) break;
+			if (!mbar_wait_warp(&accfull[a], use & 1, abort_flag, g.err, kErrTimeoutAccum)) break;
 			tc_fence_after();
 			const int blk = id / H;
 			int y, pend;
@@ -1154,7 +1154,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 			for (int c = 0; c < SPLIT_BN; ++c) run[c] = 0.0f;
 			for (int ch = 0; ch < nchunk; ++ch, ++cq) {
 				const uint32_t hb = cq & 1;
-				if (!mbar_wait(&hifull[hb], (cq >> 1) & 1, abort_flag, g.err, kErrTimeoutAccum)) {
+				if (!mbar_wait_warp(&hifull[hb], (cq >> 1) & 1, abort_flag, g.err, kErrTimeoutAccum)) {
 					ok = false;
 					break;
 				}
@@ -1173,7 +1173,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 				if (lane == 0) mbar_arrive(&hiempty[hb]);
 			}
 			if (!ok) break;
-			if (!mbar_wait(&accfull[bar_of(i)], phase_of(i), abort_flag, g.err, kErrTimeoutAccum)) break;
+			if (!mbar_wait_warp(&accfull[bar_of(i)], phase_of(i), abort_flag, g.err, kErrTimeoutAccum)) break;
 			tc_fence_after();
 			const typename P::Tile t = P::tile(g, id);
 #pragma unroll
@@ -1856,7 +1856,7 @@ __global__ void __launch_bounds__(roll_threads(), 1)
 		const T::Epi epi(g);
 		for (int r = grp; t0 + r < t1; r += 2) {
 			const int id = t0 + r, sl = roll_slot(r);
-			if (!mbar_wait(&accfull[sl], (uint32_t)(r / ROLL_SLOTS) & 1, abort_flag, g.err, kErrTimeoutAccum)) break;
+			if (!mbar_wait_warp(&accfull[sl], (uint32_t)(r / ROLL_SLOTS) & 1, abort_flag, g.err, kErrTimeoutAccum)) break;
 			tc_fence_after();
 			const uint32_t ta_ = tmem + ((uint32_t)(32 * qd) << 16) + 32u * (uint32_t)sl;
 			float v[32];
