@@ -388,6 +388,10 @@ umi_status umi_gemm_f16(const void* A, const void* B, float* C, int32_t M, int32
  * context usable.  Used by the tests of the timeout path. */
 umi_status umi_gemm_bf16_wait_limit(const void* A, const void* B, float* C, int32_t M, int32_t N, int32_t K,
                                     int32_t* err, unsigned long long epilogue_wait_ns, void* stream);
+/* The tile that umi_gemm_bf16 and umi_gemm_f16 take for a product on the
+ * current device: its columns (64, 128, 224 or 256) and whether a pair of CTAs
+ * computes it (256 rows, else 128).  For tests of the kernels' forms. */
+umi_status umi_gemm_tile(int32_t M, int32_t N, int32_t K, int32_t* width, int32_t* pair);
 /* Maps the error bits a kernel left in its `err` word (read back by the
  * caller after the stream finished) to a status: UMI_OK for 0, else
  * UMI_ERR_TIMEOUT with the bits named in umi_last_error_string(). */

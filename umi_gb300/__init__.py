@@ -90,6 +90,7 @@ SIGNATURES = {
     "umi_cost_volume_dot_f32": ([_vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp], ctypes.c_int),
     "umi_gemm_bf16": ([_vp, _vp, _vp, _i32, _i32, _i32, _vp, _vp], ctypes.c_int),
     "umi_gemm_f16": ([_vp, _vp, _vp, _i32, _i32, _i32, _vp, _vp], ctypes.c_int),
+    "umi_gemm_tile": ([_i32, _i32, _i32, _vp, _vp], ctypes.c_int),
     "umi_gemm_bf16_wait_limit": ([_vp, _vp, _vp, _i32, _i32, _i32, _vp, ctypes.c_ulonglong, _vp], ctypes.c_int),
     "umi_err_status": ([_i32], ctypes.c_int),
     "umi_gemm_f32_bf16x3_workspace_bytes": ([_i32, _i32, _i32], _sz),

@@ -1326,6 +1326,45 @@ umi_status launch_single(const void* B, const CUtensorMap& ta, const CUtensorMap
 	return umi::launch_status("tc_kernel<gemm>");
 }
 
+struct TileChoice {
+	int width, pair, pairs;  // columns; by a pair of CTAs; pairs of SMs
+};
+
+// Tiles are worked through in rounds of one per SM (pair of SMs).  The
+// cheapest tile is taken by a model in nanoseconds fitted to measurements:
+// a K step of 16 of one tile takes 39, 42, 55, 62 at widths 64, 128, 224, 256
+// (below 128 the width no longer matters); rows of A and B that do not start
+// on 128-byte lines halve what TMA brings, then its bytes (4 KB of A, 32 of
+// each column of B, half of that in a pair) at 90 a nanosecond bound the
+// step.  One-CTA tiles on nearly every SM take an eighth longer (their
+// operands' traffic); a pair costs 1.1 us once and more in its epilogue,
+// which hides behind the next round's MMAs.
+// Measured, pair and one-CTA tiles at their best widths: 4096^3 81.1 and 89.7
+// us, 3000 x 2500 x 4096 39.6 and 43.4, 1000 x 1540 x 2056 14.6 and 16.3, but
+// 2048^3 15.7 and 14.3, 512^3 7.9 and 4.9 (6.9 with tiles of 256).
+umi_status choose_tile(int M, int N, int K, TileChoice* t) {
+	int dev = 0, sms = 0;
+	UMI_TRY(umi::cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
+	UMI_TRY(umi::cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"));
+	const int64_t mt = umi::ceil_div(M, BM), mp = umi::ceil_div(M, 2 * BM), pairs = std::max(1, sms / 2);
+	int64_t best = INT64_MAX;
+	auto consider = [&](int width, int step, int pair) {
+		const int64_t tiles = (pair ? mp : mt) * umi::ceil_div(N, width), slots = pair ? pairs : sms;
+		if (K % 64 != 0) step = std::max(step, (4096 + width * (pair ? 16 : 32)) / 90);
+		int64_t round = umi::ceil_div((int64_t)K, (int64_t)16) * step, epi = pair ? 600 + 5 * width : 6 * width;
+		if (!pair && tiles * 10 > slots * 9) round += round / 8;
+		const int64_t cost = umi::ceil_div(tiles, slots) * std::max(round, epi) + epi + (pair ? 1100 : 0);
+		if (cost < best) {
+			best = cost;
+			*t = {width, pair, (int)pairs};
+		}
+	};
+	const int widths[4] = {256, 224, 128, 64}, steps[4] = {62, 55, 42, 39};
+	for (int i = 0; i < 4; ++i) consider(widths[i], steps[i], 0);
+	for (int i = 0; i < 3; ++i) consider(widths[i], steps[i], 1);
+	return UMI_OK;
+}
+
 umi_status gemm_launch(const void* A, const void* B, float* C, int M, int N, int K, int ab_type, int* err,
                        cudaStream_t st, unsigned long long acc_wait_ns = kWaitNs) {
 	if (M < 0 || N < 0 || K < 0) return umi::fail(UMI_ERR_INVALID_ARG, "gemm: negative size");
@@ -1354,47 +1393,16 @@ umi_status gemm_launch(const void* A, const void* B, float* C, int M, int N, int
 	}
 	if ((int64_t)umi::ceil_div(M, BM) * umi::ceil_div(N, 224) > INT32_MAX)
 		return umi::fail(UMI_ERR_UNSUPPORTED, "gemm: too many tiles");
-	// Tiles are worked through in rounds of one per SM (pair of SMs).  The
-	// cheapest tile is taken by a model in nanoseconds fitted to measurements:
-	// a K step of 16 of one tile takes 39, 42, 55, 62 at widths 64, 128, 224, 256
-	// (below 128 the width no longer matters); rows of A and B that do not start
-	// on 128-byte lines halve what TMA brings, then its bytes (4 KB of A, 32 of
-	// each column of B, half of that in a pair) at 90 a nanosecond bound the
-	// step.  One-CTA tiles on nearly every SM take an eighth longer (their
-	// operands' traffic); a pair costs 1.1 us once and more in its epilogue,
-	// which hides behind the next round's MMAs.
-	// Measured, pair and one-CTA tiles at their best widths: 4096^3 81.1 and 89.7
-	// us, 3000 x 2500 x 4096 39.6 and 43.4, 1000 x 1540 x 2056 14.6 and 16.3, but
-	// 2048^3 15.7 and 14.3, 512^3 7.9 and 4.9 (6.9 with tiles of 256).
-	int dev = 0, sms = 0;
-	UMI_TRY(umi::cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
-	UMI_TRY(umi::cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"));
-	const int64_t mt = umi::ceil_div(M, BM), mp = umi::ceil_div(M, 2 * BM), pairs = std::max(1, sms / 2);
-	int bn = 0, best_pair = 0;
-	int64_t best = INT64_MAX;
-	auto consider = [&](int width, int step, int pair) {
-		const int64_t tiles = (pair ? mp : mt) * umi::ceil_div(N, width), slots = pair ? pairs : sms;
-		if (K % 64 != 0) step = std::max(step, (4096 + width * (pair ? 16 : 32)) / 90);
-		int64_t round = umi::ceil_div((int64_t)K, (int64_t)16) * step, epi = pair ? 600 + 5 * width : 6 * width;
-		if (!pair && tiles * 10 > slots * 9) round += round / 8;
-		const int64_t cost = umi::ceil_div(tiles, slots) * std::max(round, epi) + epi + (pair ? 1100 : 0);
-		if (cost < best) {
-			best = cost;
-			bn = width;
-			best_pair = pair;
-		}
-	};
-	const int widths[4] = {256, 224, 128, 64}, steps[4] = {62, 55, 42, 39};
-	for (int i = 0; i < 4; ++i) consider(widths[i], steps[i], 0);
-	for (int i = 0; i < 3; ++i) consider(widths[i], steps[i], 1);
-	if (best_pair) {
-		if (bn == 256) return launch_pair<256>(B, ta, tc, dt, g, ab_type, (int)pairs, st);
-		if (bn == 224) return launch_pair<224>(B, ta, tc, dt, g, ab_type, (int)pairs, st);
-		return launch_pair<128>(B, ta, tc, dt, g, ab_type, (int)pairs, st);
+	TileChoice t;
+	UMI_TRY(choose_tile(M, N, K, &t));
+	if (t.pair) {
+		if (t.width == 256) return launch_pair<256>(B, ta, tc, dt, g, ab_type, t.pairs, st);
+		if (t.width == 224) return launch_pair<224>(B, ta, tc, dt, g, ab_type, t.pairs, st);
+		return launch_pair<128>(B, ta, tc, dt, g, ab_type, t.pairs, st);
 	}
-	if (bn == 256) return launch_single<256>(B, ta, tc, dt, g, ab_type, st);
-	if (bn == 224) return launch_single<224>(B, ta, tc, dt, g, ab_type, st);
-	if (bn == 128) return launch_single<128>(B, ta, tc, dt, g, ab_type, st);
+	if (t.width == 256) return launch_single<256>(B, ta, tc, dt, g, ab_type, st);
+	if (t.width == 224) return launch_single<224>(B, ta, tc, dt, g, ab_type, st);
+	if (t.width == 128) return launch_single<128>(B, ta, tc, dt, g, ab_type, st);
 	return launch_single<64>(B, ta, tc, dt, g, ab_type, st);
 }
 
@@ -1416,6 +1424,15 @@ extern "C" umi_status umi_gemm_bf16_wait_limit(const void* A, const void* B, flo
                                                int32_t* err, unsigned long long epilogue_wait_ns, void* stream) {
 	const umi_status s = gemm_launch(A, B, C, M, N, K, 1, err, umi::as_stream(stream), epilogue_wait_ns);
 	return s == UMI_OK ? umi::ok() : s;
+}
+
+extern "C" umi_status umi_gemm_tile(int32_t M, int32_t N, int32_t K, int32_t* width, int32_t* pair) {
+	if (M < 1 || N < 1 || K < 1 || !width || !pair) return umi::fail(UMI_ERR_INVALID_ARG, "gemm_tile: size or null pointer");
+	TileChoice t;
+	UMI_TRY(choose_tile(M, N, K, &t));
+	*width = t.width;
+	*pair = t.pair;
+	return umi::ok();
 }
 
 extern "C" umi_status umi_err_status(int32_t err_bits) {
