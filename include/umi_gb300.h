@@ -192,7 +192,8 @@ umi_status umi_filter3x3_f32_tma(const float* in, float* out, int32_t h, int32_t
  * Loop output, transposed, twice) with two launches: column sums per group
  * of 128 rows, then one output pass.  Needs a device workspace of
  * umi_iimg_u8_i32_workspace_bytes(h, w) bytes (16-byte aligned; about
- * 0.29 byte per pixel; its content need not be initialised).  Frames with
+ * 0.27 byte per pixel, 0.29 for frames wider than 2048, which also run with
+ * 0.27; its content need not be initialised).  Frames with
  * h*w*255 >= 2^31 are rejected (UMI_ERR_UNSUPPORTED: sums could overflow
  * int32). */
 size_t umi_iimg_u8_i32_workspace_bytes(int32_t h, int32_t w);

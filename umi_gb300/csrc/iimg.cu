@@ -295,7 +295,7 @@ struct BandGeom {
 	int h, w, nb, ng, wpad, nch;
 	int vec_in, vec_out;
 	int vec_out8;    // rows of out are 32-byte aligned
-	int left;        // several segments per band: kernel 1 writes the last three arrays
+	int left;        // a CTA per segment, several per band: kernel 1 writes the last three arrays
 	uint16_t* wsum;  // [ng * GB][wpad]  W
 	uint16_t* gsum;  // [ng][wpad]       S
 	uint16_t* rsum;  // [nch][ng * GB * RB]  row sums per chunk
@@ -303,9 +303,13 @@ struct BandGeom {
 	uint32_t* gtot;  // [nch][ng]        S summed over the chunk
 };
 
-// Workspace layout (offsets of the arrays above, total in bytes[5]).
+// Frames up to this width are one segment of 256 threads.
+constexpr int kOneSegment = 256 * CPL;
+
+// Workspace layout: offsets of the arrays above, the bytes up to the last one and
+// those of the first two alone, which serve any frame.
 struct BandWork {
-	size_t off[5], bytes;
+	size_t off[5], bytes, least;
 	BandWork(int h, int w) {
 		const size_t nb = umi::ceil_div(h, RB), ng = umi::ceil_div(nb, (size_t)GB);
 		const size_t wpad = (size_t)umi::ceil_div(w, CPL) * CPL, nch = umi::ceil_div(w, CHUNK);
@@ -315,10 +319,10 @@ struct BandWork {
 			off[i] = bytes;
 			bytes += (n[i] + 255) & ~size_t(255);
 		}
+		least = off[2];
+		if (w <= kOneSegment) bytes = least;
 	}
 };
-
-size_t band_ws_bytes(int h, int w) { return BandWork(h, w).bytes; }
 
 // Rows y0 .. y0 + RB - 1 of a thread's 8 columns.  Rows of any alignment are
 // read as three aligned words each, decided once for all of them (a decision
@@ -419,8 +423,9 @@ __device__ __forceinline__ void add_u16x8(uint32_t (&v)[CPL], uint4 p) {
 	v[6] += p.w & 0xffffu; v[7] += p.w >> 16;
 }
 
-// NT2: threads, 8 columns each.
-template <int NT2>
+// NT2: threads, 8 columns each.  WALK: a CTA takes a band's segments one after the
+// other, its sums carried along (a workspace without the sums per chunk).
+template <int NT2, bool WALK>
 __global__ void __launch_bounds__(NT2, NT2 == 128 ? 6 : 2) iimg_band_out(const uint8_t* __restrict__ in, int32_t* __restrict__ out,
                                                       const BandGeom g) {
 	constexpr int NW2 = NT2 / 32, SEG = NT2 * CPL;
@@ -429,116 +434,127 @@ __global__ void __launch_bounds__(NT2, NT2 == 128 ? 6 : 2) iimg_band_out(const u
 	__shared__ uint32_t left[NW2][RB + 1];  // per warp: sums over the chunks left of the segment (rows, then the V row)
 	__shared__ __align__(16) uint32_t rowbuf[NW2][4][32 * CPL];
 	const int b = blockIdx.x, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-	const int y0 = b * RB, x0 = blockIdx.y * SEG + threadIdx.x * CPL;
-	const bool live = x0 < g.w;
+	const int y0 = b * RB;
 	IimgGeom ig{};
 	ig.h = g.h; ig.w = g.w; ig.vec_in = g.vec_in;
-	uint2 raw[RB] = {};
-	if (live) load_rows(in, ig, y0, x0, raw);
-	pdl_wait();
-	const int gb = b / GB, nleft = blockIdx.y * (SEG / CHUNK);  // groups above, chunks to the left
-	uint32_t vv[CPL] = {};
-	if (live) {  // V = W of this band + S of every group above
-		add_u16x8(vv, __ldcg(reinterpret_cast<const uint4*>(g.wsum + (size_t)b * g.wpad + x0)));
+	uint32_t carry[RB + 1] = {};  // WALK: of each row and of the V row, left of the segment
+	int seg = WALK ? 0 : blockIdx.y;
+	do {
+		const int x0 = seg * SEG + threadIdx.x * CPL;
+		const bool live = x0 < g.w;
+		uint2 raw[RB] = {};
+		if (live) load_rows(in, ig, y0, x0, raw);
+		pdl_wait();
+		const int gb = b / GB, nleft = WALK ? 0 : seg * (SEG / CHUNK);  // groups above, chunks to the left
+		uint32_t vv[CPL] = {};
+		if (live) {  // V = W of this band + S of every group above
+			add_u16x8(vv, __ldcg(reinterpret_cast<const uint4*>(g.wsum + (size_t)b * g.wpad + x0)));
 #pragma unroll 8
-		for (int q = 0; q < gb; ++q) add_u16x8(vv, __ldcg(reinterpret_cast<const uint4*>(g.gsum + (size_t)q * g.wpad + x0)));
-	}
-	if (nleft) {
-		uint32_t rl[CPL] = {}, vl = 0;
-		for (int c = threadIdx.x; c < nleft; c += NT2) {
-			add_u16x8(rl, __ldcg(reinterpret_cast<const uint4*>(g.rsum + ((size_t)c * g.ng * GB + b) * RB)));
-			vl += __ldcg(g.wtot + (size_t)c * g.ng * GB + b);
+			for (int q = 0; q < gb; ++q) add_u16x8(vv, __ldcg(reinterpret_cast<const uint4*>(g.gsum + (size_t)q * g.wpad + x0)));
 		}
-		for (int c = wp; c < nleft; c += NW2)
-			for (int q = lane; q < gb; q += 32) vl += __ldcg(g.gtot + (size_t)c * g.ng + q);
+		if (nleft) {
+			uint32_t rl[CPL] = {}, vl = 0;
+			for (int c = threadIdx.x; c < nleft; c += NT2) {
+				add_u16x8(rl, __ldcg(reinterpret_cast<const uint4*>(g.rsum + ((size_t)c * g.ng * GB + b) * RB)));
+				vl += __ldcg(g.wtot + (size_t)c * g.ng * GB + b);
+			}
+			for (int c = wp; c < nleft; c += NW2)
+				for (int q = lane; q < gb; q += 32) vl += __ldcg(g.gtot + (size_t)c * g.ng + q);
 #pragma unroll
-		for (int r = 0; r < RB; ++r) rl[r] = __reduce_add_sync(0xffffffffu, rl[r]);
-		vl = __reduce_add_sync(0xffffffffu, vl);
-		if (lane == 0) {
+			for (int r = 0; r < RB; ++r) rl[r] = __reduce_add_sync(0xffffffffu, rl[r]);
+			vl = __reduce_add_sync(0xffffffffu, vl);
+			if (lane == 0) {
 #pragma unroll
-			for (int r = 0; r < RB; ++r) left[wp][r] = rl[r];
-			left[wp][RB] = vl;
-		}
-	}
-	// thread totals of each row and of the V row, scanned over the block
-	uint32_t tsum[RB + 1];
-#pragma unroll
-	for (int r = 0; r < RB; ++r) {
-		uint32_t v[CPL];
-		unpack8(raw[r], v);
-		uint32_t t = 0;
-#pragma unroll
-		for (int k = 0; k < CPL; ++k) t += v[k];
-		tsum[r] = t;
-	}
-	{
-		uint32_t t = 0;
-#pragma unroll
-		for (int k = 0; k < CPL; ++k) t += vv[k];
-		tsum[RB] = t;
-	}
-	uint32_t ex[RB + 1];
-#pragma unroll
-	for (int r = 0; r <= RB; ++r) {
-		const uint32_t inc = warp_incl_scan(tsum[r], lane);
-		ex[r] = inc - tsum[r];
-		if (lane == 31) wtot[wp][r] = inc;
-	}
-	__syncthreads();
-#pragma unroll
-	for (int r = 0; r <= RB; ++r) {
-#pragma unroll
-		for (int k = 0; k < NW2 - 1; ++k) ex[r] += k < wp ? wtot[k][r] : 0u;
-		if (nleft)
-#pragma unroll
-			for (int k = 0; k < NW2; ++k) ex[r] += left[k][r];
-	}
-	// outputs: T(x) = V-row prefix, plus the running column sum of the row prefixes
-	uint32_t T[CPL];
-	{
-		uint32_t tp = ex[RB];
-#pragma unroll
-		for (int k = 0; k < CPL; ++k) {
-			tp += vv[k];
-			T[k] = tp;
-		}
-	}
-#pragma unroll
-	for (int r = 0; r < RB; ++r) {
-		uint32_t rp = ex[r];
-#pragma unroll
-		for (int k = 0; k < CPL; ++k) {
-			rp += (k < 4 ? (raw[r].x >> (8 * k)) : (raw[r].y >> (8 * (k - 4)))) & 0xffu;
-			T[k] += rp;
-		}
-		const int y = y0 + r;
-		if (y >= g.h) break;
-		int32_t* op = out + (size_t)y * g.w + x0;
-		if (g.vec_out8) {  // w % 8 == 0: every live thread has 8 columns
-			if (live)
-				asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(op), "r"(T[0]), "r"(T[1]),
-				             "r"(T[2]), "r"(T[3]), "r"(T[4]), "r"(T[5]), "r"(T[6]), "r"(T[7])
-				             : "memory");
-		} else if (g.vec_out) {  // w % 4 == 0
-			if (live) reinterpret_cast<int4*>(op)[0] = make_int4(T[0], T[1], T[2], T[3]);
-			if (x0 + 7 < g.w) reinterpret_cast<int4*>(op)[1] = make_int4(T[4], T[5], T[6], T[7]);
-		} else {  // any alignment: the warp's 256 columns through shared memory, four rows at a time
-			uint32_t* row = rowbuf[wp][r & 3];
-			*reinterpret_cast<uint4*>(row + CPL * lane) = make_uint4(T[0], T[1], T[2], T[3]);
-			*reinterpret_cast<uint4*>(row + CPL * lane + 4) = make_uint4(T[4], T[5], T[6], T[7]);
-			if ((r & 3) == 3 || y == g.h - 1) {
-				__syncwarp();
-				const int xw = x0 - CPL * lane + lane;
-				for (int i = 0; i <= (r & 3); ++i) {
-					int32_t* o = out + (size_t)(y - (r & 3) + i) * g.w + xw;
-#pragma unroll
-					for (int k = 0; k < CPL; ++k)  // 128 contiguous bytes per store
-						if (xw + 32 * k < g.w) o[32 * k] = (int32_t)rowbuf[wp][i][32 * k + lane];
-				}
-				__syncwarp();
+				for (int r = 0; r < RB; ++r) left[wp][r] = rl[r];
+				left[wp][RB] = vl;
 			}
 		}
-	}
+		// thread totals of each row and of the V row, scanned over the block
+		uint32_t tsum[RB + 1];
+#pragma unroll
+		for (int r = 0; r < RB; ++r) {
+			uint32_t v[CPL];
+			unpack8(raw[r], v);
+			uint32_t t = 0;
+#pragma unroll
+			for (int k = 0; k < CPL; ++k) t += v[k];
+			tsum[r] = t;
+		}
+		{
+			uint32_t t = 0;
+#pragma unroll
+			for (int k = 0; k < CPL; ++k) t += vv[k];
+			tsum[RB] = t;
+		}
+		uint32_t ex[RB + 1];
+#pragma unroll
+		for (int r = 0; r <= RB; ++r) {
+			const uint32_t inc = warp_incl_scan(tsum[r], lane);
+			ex[r] = inc - tsum[r];
+			if (lane == 31) wtot[wp][r] = inc;
+		}
+		__syncthreads();
+#pragma unroll
+		for (int r = 0; r <= RB; ++r) {
+#pragma unroll
+			for (int k = 0; k < NW2 - 1; ++k) ex[r] += k < wp ? wtot[k][r] : 0u;
+			if (nleft)
+#pragma unroll
+				for (int k = 0; k < NW2; ++k) ex[r] += left[k][r];
+			if constexpr (WALK) {
+				ex[r] += carry[r];
+#pragma unroll
+				for (int k = 0; k < NW2; ++k) carry[r] += wtot[k][r];
+			}
+		}
+		// outputs: T(x) = V-row prefix, plus the running column sum of the row prefixes
+		uint32_t T[CPL];
+		{
+			uint32_t tp = ex[RB];
+#pragma unroll
+			for (int k = 0; k < CPL; ++k) {
+				tp += vv[k];
+				T[k] = tp;
+			}
+		}
+#pragma unroll
+		for (int r = 0; r < RB; ++r) {
+			uint32_t rp = ex[r];
+#pragma unroll
+			for (int k = 0; k < CPL; ++k) {
+				rp += (k < 4 ? (raw[r].x >> (8 * k)) : (raw[r].y >> (8 * (k - 4)))) & 0xffu;
+				T[k] += rp;
+			}
+			const int y = y0 + r;
+			if (y >= g.h) break;
+			int32_t* op = out + (size_t)y * g.w + x0;
+			if (g.vec_out8) {  // w % 8 == 0: every live thread has 8 columns
+				if (live)
+					asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(op), "r"(T[0]), "r"(T[1]),
+					             "r"(T[2]), "r"(T[3]), "r"(T[4]), "r"(T[5]), "r"(T[6]), "r"(T[7])
+					             : "memory");
+			} else if (g.vec_out) {  // w % 4 == 0
+				if (live) reinterpret_cast<int4*>(op)[0] = make_int4(T[0], T[1], T[2], T[3]);
+				if (x0 + 7 < g.w) reinterpret_cast<int4*>(op)[1] = make_int4(T[4], T[5], T[6], T[7]);
+			} else {  // any alignment: the warp's 256 columns through shared memory, four rows at a time
+				uint32_t* row = rowbuf[wp][r & 3];
+				*reinterpret_cast<uint4*>(row + CPL * lane) = make_uint4(T[0], T[1], T[2], T[3]);
+				*reinterpret_cast<uint4*>(row + CPL * lane + 4) = make_uint4(T[4], T[5], T[6], T[7]);
+				if ((r & 3) == 3 || y == g.h - 1) {
+					__syncwarp();
+					const int xw = x0 - CPL * lane + lane;
+					for (int i = 0; i <= (r & 3); ++i) {
+						int32_t* o = out + (size_t)(y - (r & 3) + i) * g.w + xw;
+#pragma unroll
+						for (int k = 0; k < CPL; ++k)  // 128 contiguous bytes per store
+							if (xw + 32 * k < g.w) o[32 * k] = (int32_t)rowbuf[wp][i][32 * k + lane];
+					}
+					__syncwarp();
+				}
+			}
+		}
+		if constexpr (WALK) __syncthreads();  // the next segment's totals overwrite these
+	} while (WALK && ++seg * SEG < g.w);
 }
 
 cudaLaunchAttribute pdl_attr() {
@@ -552,7 +568,7 @@ cudaLaunchAttribute pdl_attr() {
 
 extern "C" size_t umi_iimg_u8_i32_workspace_bytes(int32_t h, int32_t w) {
 	if (h <= 0 || w <= 0) return 0;
-	return band_ws_bytes(h, w);
+	return BandWork(h, w).bytes;
 }
 
 extern "C" umi_status umi_iimg_u8_i32(const uint8_t* in, int32_t* out, int32_t h, int32_t w, void* workspace,
@@ -561,9 +577,9 @@ extern "C" umi_status umi_iimg_u8_i32(const uint8_t* in, int32_t* out, int32_t h
 	if (h == 0 || w == 0) return umi::ok();
 	if (!in || !out || !workspace) return umi::fail(UMI_ERR_INVALID_ARG, "iimg: null pointer");
 	if (!umi::aligned(workspace, 16)) return umi::fail(UMI_ERR_INVALID_ARG, "iimg: workspace not 16-byte aligned");
-	if (workspace_bytes < band_ws_bytes(h, w))
-		return umi::fail(UMI_ERR_NO_MEMORY, "iimg: workspace of %zu bytes, need %zu", workspace_bytes,
-		                 band_ws_bytes(h, w));
+	const BandWork work(h, w);
+	if (workspace_bytes < work.least)
+		return umi::fail(UMI_ERR_NO_MEMORY, "iimg: workspace of %zu bytes, need %zu", workspace_bytes, work.bytes);
 	if ((int64_t)h * w > ((int64_t)1 << 31) / 255)
 		return umi::fail(UMI_ERR_UNSUPPORTED, "iimg: %dx%d frame: sums could exceed int32", h, w);
 	BandGeom g{};
@@ -575,10 +591,13 @@ extern "C" umi_status umi_iimg_u8_i32(const uint8_t* in, int32_t* out, int32_t h
 	g.vec_in = umi::aligned(in, 8) && (w % 8) == 0;
 	g.vec_out = umi::aligned(out, 16) && (w % 4) == 0;
 	g.vec_out8 = umi::aligned(out, 32) && (w % 8) == 0;
-	// a frame of at most 2048 columns is one segment (nothing lies left of it)
-	const int nt2 = w <= 256 * CPL ? 256 : 128;
-	g.left = w > nt2 * CPL;
-	const BandWork work(h, w);
+	// a frame of at most 2048 columns is one segment (nothing lies left of it); a
+	// wider one has a CTA per segment where the workspace holds the sums to the
+	// left of them, else one per band (graph replays, us: 1440 x 2560 9.3 and 11.3,
+	// 1081 x 2561 10.8 and 13.1, 2160 x 3840 15.5 and 14.5)
+	const bool segments = w > kOneSegment && workspace_bytes >= work.bytes;
+	const int nt2 = segments ? 128 : 256;
+	g.left = segments;
 	char* ws = static_cast<char*>(workspace);
 	g.wsum = reinterpret_cast<uint16_t*>(ws + work.off[0]);
 	g.gsum = reinterpret_cast<uint16_t*>(ws + work.off[1]);
@@ -591,13 +610,13 @@ extern "C" umi_status umi_iimg_u8_i32(const uint8_t* in, int32_t* out, int32_t h
 	UMI_TRY(umi::launch_status("iimg_group_sums"));
 	cudaLaunchAttribute attr[1] = {pdl_attr()};
 	cudaLaunchConfig_t cfg{};
-	cfg.gridDim = dim3(g.nb, umi::ceil_div(w, nt2 * CPL));
+	cfg.gridDim = dim3(g.nb, segments ? umi::ceil_div(w, nt2 * CPL) : 1);
 	cfg.blockDim = dim3(nt2);
 	cfg.stream = st;
 	cfg.attrs = attr;
 	cfg.numAttrs = 1;
-	UMI_TRY(umi::cuda_status(cudaLaunchKernelEx(&cfg, nt2 == 256 ? iimg_band_out<256> : iimg_band_out<128>, in, out, g),
-	                         "iimg_band_out"));
+	auto kern = segments ? iimg_band_out<128, false> : w <= kOneSegment ? iimg_band_out<256, false> : iimg_band_out<256, true>;
+	UMI_TRY(umi::cuda_status(cudaLaunchKernelEx(&cfg, kern, in, out, g), "iimg_band_out"));
 	return umi::ok();
 }
 
