@@ -55,38 +55,60 @@ struct Layout {
 	}
 };
 
-// ---- workspace layout for a frame of h x w pixels
+// ---- workspace layout for a frame of h x w pixels, in `have` bytes.  What a
+// backward pass takes over from the forward pass and what the motion search
+// needs lie apart; the rest is scratch that the passes share.  A workspace
+// smaller than `bytes` (at least `least`) holds fewer rows of partial sums, and
+// one too small for every layer's forward weights at once takes them in turn.
 struct Work {
 	int H4, W4, P, nbx, nby, nblk;
-	size_t x0, act[NL], dA[2], wf[NL], wt[NL], pred, centers, list, count, alist, amv, wpart, hpart;
-	size_t parts[2];         // training: gradients as bf16 parts (menet_parts.cu)
-	size_t nhwc[2], wtc[NL], err;  // tensor-core inference: bf16 (H4, W4, 32) activations, packed weights
-	size_t bytes;
-	Work(int h, int w) {
+	size_t x0, act[NL], wt[NL], pred, centers, list, count, alist, amv, err;
+	size_t wf[NL];           // forward: weights (menet_train.cuh), fp32, after the first layer every value twice
+	size_t nhwc[2], wtc[NL]; // tensor-core inference: bf16 (H4, W4, 32) activations, packed weights
+	size_t slot[3], part;    // backward: gradients, fp32 or as bf16 parts (menet_parts.cu); partial sums
+	int htx, htiles, units;  // the head's tiles; rows of 32 columns that the weight gradients walk
+	int parts, head_parts;   // rows of partial sums
+	bool whole;              // every layer's forward weights at once
+	size_t least, bytes;
+	Work(int h, int w, size_t have = ~(size_t)0) {
 		H4 = h / 4; W4 = w / 4; P = H4 * W4;
 		nbx = w / 16; nby = h / 16; nblk = nbx * nby;
+		htx = umi::ceil_div(nbx, 8); htiles = htx * nby;
+		units = umi::ceil_div(W4, 32) * H4;
+		auto al = [](size_t n) { return (n + 255) & ~size_t(255); };
 		size_t o = 0;
-		auto take = [&](size_t n) { size_t r = o; o += (n + 255) & ~size_t(255); return r; };
+		auto take = [&](size_t n) { size_t r = o; o += al(n); return r; };
 		x0 = take(sizeof(float) * 2 * P);
 		for (int l = 0; l < NL; ++l) act[l] = take(sizeof(float) * CH * P);
-		for (int i = 0; i < 2; ++i) dA[i] = take(sizeof(float) * CH * P);
-		// training weights (menet_train.cuh): fp32 for the forward layers (after
-		// the first every value twice), bf16 for the data gradient
-		for (int l = 0; l < NL; ++l) wf[l] = take(sizeof(float) * (l ? 2 : 1) * CH * CIN[l] * 9);
-		for (int l = 0; l < NL; ++l) wt[l] = l ? take(2 * CH * CIN[l] * 9) : 0;
+		for (int l = 0; l < NL; ++l) wt[l] = l ? take(2 * CH * CIN[l] * 9) : 0;  // bf16, for the data gradient
 		pred = take(sizeof(float) * 2 * nblk);
 		centers = take(sizeof(int32_t) * 2 * nblk);
 		list = take(sizeof(int32_t) * nblk);
 		count = take(sizeof(int32_t) * 4);  // [0] fallback blocks, [2] audited blocks
 		alist = take(sizeof(int32_t) * nblk);
 		amv = take(sizeof(int32_t) * 3 * nblk);
-		wpart = take(sizeof(float) * (size_t)menet_train::PARTS * (CH * CH * 9 + CH));
-		hpart = take(sizeof(float) * (size_t)menet_train::HEAD_PARTS * (2 * HEADF + 3));
-		for (int i = 0; i < 2; ++i) parts[i] = take((size_t)P * 3 * CH * 2);
-		for (int i = 0; i < 2; ++i) nhwc[i] = take((size_t)P * 64);
-		for (int l = 0; l < NL; ++l) wtc[l] = take(2 * CH * 9 * CH);
 		err = take(sizeof(int32_t));
-		bytes = o;
+		const size_t scratch = o;
+		constexpr size_t ROW = sizeof(float) * (CH * CH * 9 + CH), HEAD_ROW = sizeof(float) * (2 * HEADF + 3);
+		constexpr size_t WF0 = sizeof(float) * CH * CIN[0] * 9, WF = sizeof(float) * 2 * CH * CH * 9;
+		for (int i = 0; i < 2; ++i) nhwc[i] = take((size_t)P * 64);
+		for (int l = 1; l < NL; ++l) wtc[l] = take(2 * CH * 9 * CH);
+		const size_t infer = o;
+		o = scratch;
+		for (int i = 0; i < 3; ++i) slot[i] = take((size_t)P * 3 * CH * 2);
+		part = o;
+		parts = std::min(units, menet_train::PARTS);
+		head_parts = std::min(htiles, menet_train::HEAD_PARTS);
+		const size_t forward = scratch + al(WF0) + (NL - 1) * al(WF);
+		bytes = std::max({infer, forward, part + al(std::max(parts * ROW, head_parts * HEAD_ROW))});
+		least = std::max({infer, scratch + al(WF0) + al(WF), part + al(std::max(ROW, HEAD_ROW))});
+		const size_t end = std::min(have, bytes);
+		const size_t room = end > part ? end - part : 0;
+		parts = (int)std::min<size_t>(parts, room / ROW);
+		head_parts = (int)std::min<size_t>(head_parts, room / HEAD_ROW);
+		whole = end >= forward;
+		wf[0] = scratch;
+		for (int l = 1; l < NL; ++l) wf[l] = scratch + al(WF0) + (whole ? l - 1 : 0) * al(WF);
 	}
 	template <class T> T* at(void* ws, size_t off) const { return reinterpret_cast<T*>(static_cast<char*>(ws) + off); }
 };
@@ -408,36 +430,39 @@ umi_status reduce_rows(const float* part, float* out, float* extra, int n, int m
 	return umi::launch_status("reduce_rows_kernel");
 }
 
-umi_status forward(const uint8_t* cur, const uint8_t* ref, int h, int w, const float* params, void* ws,
+umi_status forward(const uint8_t* cur, const uint8_t* ref, int w, const float* params, const Work& K, void* ws,
                    cudaStream_t st) {
 	const Layout& L = layout();
-	const Work K(h, w);
 	downsample4_kernel<<<grid_for(2 * (size_t)K.P), NT, 0, st>>>(cur, ref, K.at<float>(ws, K.x0), w, K.H4, K.W4);
 	UMI_TRY(umi::launch_status("downsample4_kernel"));
-	menet_train::Pack pk{};
-	for (int l = 0; l < NL; ++l) {
-		pk.w[l] = params + L.w[l];
-		pk.fwd[l] = K.at<float>(ws, K.wf[l]);
-		pk.bwd[l] = l ? K.at<__nv_bfloat16>(ws, K.wt[l]) : nullptr;
-	}
-	menet_train::pack_weights_kernel<<<dim3(grid_for(CH * CH * 9), NL), NT, 0, st>>>(pk);
-	UMI_TRY(umi::launch_status("pack_weights_kernel"));
+	auto pack = [&](int first, int n) {  // the weights of layers first .. first + n - 1
+		menet_train::Pack pk{};
+		for (int l = first; l < first + n; ++l) {
+			pk.w[l] = params + L.w[l];
+			pk.fwd[l] = K.at<float>(ws, K.wf[l]);
+			pk.bwd[l] = l ? K.at<__nv_bfloat16>(ws, K.wt[l]) : nullptr;
+		}
+		menet_train::pack_weights_kernel<<<dim3(grid_for(CH * CH * 9), n), NT, 0, st>>>(pk, first);
+		return umi::launch_status("pack_weights_kernel");
+	};
+	UMI_TRY(pack(0, K.whole ? NL : 1));
 	menet_train::conv_first_kernel<<<umi::ceil_div(K.P / 4, NT), NT, 0, st>>>(
 		K.at<float>(ws, K.x0), K.at<float>(ws, K.wf[0]), params + L.b[0], K.at<float>(ws, K.act[0]), K.H4, K.W4);
 	UMI_TRY(umi::launch_status("conv_first_kernel"));
-	for (int l = 1; l < NL; ++l)
+	for (int l = 1; l < NL; ++l) {
+		if (!K.whole) UMI_TRY(pack(l, 1));
 		UMI_TRY(conv_layer(l, K.at<float>(ws, K.act[l - 1]), K.at<float>(ws, K.wf[l]), params + L.b[l],
 		                   K.at<float>(ws, K.act[l]), K, st));
+	}
 	menet_train::head_fwd_kernel<<<dim3(umi::ceil_div(K.nbx, 64), K.nby), NT, 0, st>>>(
 		K.at<float>(ws, K.act[NL - 1]), params + L.wh, params + L.bh, K.at<float>(ws, K.pred), K.H4, K.W4, K.nbx);
 	return umi::launch_status("head_fwd_kernel");
 }
 
 // Inference forward pass with layers 2-4 on the tensor cores; prediction to K.pred.
-umi_status infer(const uint8_t* cur, const uint8_t* ref, int h, int w, const float* params, void* ws, int32_t* err,
+umi_status infer(const uint8_t* cur, const uint8_t* ref, int w, const float* params, const Work& K, void* ws, int32_t* err,
                  cudaStream_t st) {
 	const Layout& L = layout();
-	const Work K(h, w);
 	downsample4_kernel<<<grid_for(2 * (size_t)K.P), NT, 0, st>>>(cur, ref, K.at<float>(ws, K.x0), w, K.H4, K.W4);
 	UMI_TRY(umi::launch_status("downsample4_kernel"));
 	TcWeights tw;
@@ -467,11 +492,11 @@ extern "C" umi_status umi_menet_infer(const uint8_t* cur, const uint8_t* ref, in
                                       float* pred, int32_t* err, void* workspace, size_t workspace_bytes, void* stream) {
 	UMI_TRY(check_frame(h, w));
 	if (!cur || !ref || !params || !workspace) return umi::fail(UMI_ERR_INVALID_ARG, "menet_infer: null pointer");
-	const Work K(h, w);
-	if (workspace_bytes < K.bytes) return umi::fail(UMI_ERR_NO_MEMORY, "menet_infer: workspace too small");
+	const Work K(h, w, workspace_bytes);
+	if (workspace_bytes < K.least) return umi::fail(UMI_ERR_NO_MEMORY, "menet_infer: workspace too small");
 	if (!umi::aligned(workspace, 256)) return umi::fail(UMI_ERR_INVALID_ARG, "menet_infer: workspace alignment");
 	const cudaStream_t st = umi::as_stream(stream);
-	UMI_TRY(infer(cur, ref, h, w, params, workspace, err, st));
+	UMI_TRY(infer(cur, ref, w, params, K, workspace, err, st));
 	if (pred)
 		UMI_TRY(umi::cuda_status(cudaMemcpyAsync(pred, K.at<float>(workspace, K.pred), sizeof(float) * 2 * K.nblk,
 		                                         cudaMemcpyDeviceToDevice, st),
@@ -490,11 +515,11 @@ extern "C" umi_status umi_menet_forward(const uint8_t* cur, const uint8_t* ref, 
                                         float* pred, void* workspace, size_t workspace_bytes, void* stream) {
 	UMI_TRY(check_frame(h, w));
 	if (!cur || !ref || !params || !workspace) return umi::fail(UMI_ERR_INVALID_ARG, "menet_forward: null pointer");
-	const Work K(h, w);
-	if (workspace_bytes < K.bytes) return umi::fail(UMI_ERR_NO_MEMORY, "menet_forward: workspace too small");
+	const Work K(h, w, workspace_bytes);
+	if (workspace_bytes < K.least) return umi::fail(UMI_ERR_NO_MEMORY, "menet_forward: workspace too small");
 	if (!umi::aligned(workspace, 256)) return umi::fail(UMI_ERR_INVALID_ARG, "menet_forward: workspace alignment");
 	const cudaStream_t st = umi::as_stream(stream);
-	UMI_TRY(forward(cur, ref, h, w, params, workspace, st));
+	UMI_TRY(forward(cur, ref, w, params, K, workspace, st));
 	if (pred)
 		UMI_TRY(umi::cuda_status(cudaMemcpyAsync(pred, K.at<float>(workspace, K.pred), sizeof(float) * 2 * K.nblk,
 		                                         cudaMemcpyDeviceToDevice, st),
@@ -508,43 +533,46 @@ extern "C" umi_status umi_menet_backward_err(const int32_t* target, int32_t targ
                                              void* stream) {
 	UMI_TRY(check_frame(h, w));
 	if (!target || !params || !grads || !workspace) return umi::fail(UMI_ERR_INVALID_ARG, "menet_backward: null pointer");
-	const Work K(h, w);
-	if (workspace_bytes < K.bytes) return umi::fail(UMI_ERR_NO_MEMORY, "menet_backward: workspace too small");
+	const Work K(h, w, workspace_bytes);
+	if (workspace_bytes < K.least) return umi::fail(UMI_ERR_NO_MEMORY, "menet_backward: workspace too small");
 	if (!umi::aligned(workspace, 256)) return umi::fail(UMI_ERR_INVALID_ARG, "menet_backward: workspace alignment");
 	const Layout& L = layout();
 	const cudaStream_t st = umi::as_stream(stream);
 	void* ws = workspace;
-	float* dcur = K.at<float>(ws, K.dA[0]);
-	float* dnext = K.at<float>(ws, K.dA[1]);
+	// the gradient in fp32, the same as parts, and a free slot for the next one's
+	// fp32 form; its parts replace the fp32 form that the weight gradient has read
+	size_t dcur = K.slot[0], din = K.slot[1], dnext = K.slot[2];
 	int32_t* bits = K.at<int32_t>(ws, K.err);  // of this pass's waits, cleared by its first kernel
-	const int htx = umi::ceil_div(K.nbx, 8), htiles = htx * K.nby, nh = std::min(htiles, menet_train::HEAD_PARTS);
-	menet_train::head_bwd_kernel<<<nh, NT, 0, st>>>(K.at<float>(ws, K.act[NL - 1]), params + L.wh,
-	                                                K.at<float>(ws, K.pred), target, target_stride, dcur,
-	                                                K.at<float>(ws, K.hpart), K.H4, K.W4, K.nbx, K.nblk, htx, htiles, bits);
+	menet_train::head_bwd_kernel<<<K.head_parts, NT, 0, st>>>(K.at<float>(ws, K.act[NL - 1]), params + L.wh,
+	                                                K.at<float>(ws, K.pred), target, target_stride,
+	                                                K.at<float>(ws, dcur), K.at<float>(ws, K.part), K.H4, K.W4, K.nbx,
+	                                                K.nblk, K.htx, K.htiles, bits);
 	UMI_TRY(umi::launch_status("head_bwd_kernel"));
-	UMI_TRY(reduce_rows(K.at<float>(ws, K.hpart), grads + L.wh, loss, nh, 2 * HEADF + 3, 2 * HEADF + 2, bits, nullptr, st));
-	void *din = K.at<void>(ws, K.parts[0]), *dout = K.at<void>(ws, K.parts[1]);
-	UMI_TRY(umi::menet_to_parts(dcur, din, K.P, st));
-	const int units = umi::ceil_div(K.W4, 32) * K.H4, per = umi::ceil_div(units, menet_train::PARTS);
-	const int grid = umi::ceil_div(units, per);
-	float* part = K.at<float>(ws, K.wpart);
+	float* part = K.at<float>(ws, K.part);
+	UMI_TRY(reduce_rows(part, grads + L.wh, loss, K.head_parts, 2 * HEADF + 3, 2 * HEADF + 2, bits, nullptr, st));
+	UMI_TRY(umi::menet_to_parts(K.at<float>(ws, dcur), K.at<void>(ws, din), K.P, st));
+	const int units = K.units, per = umi::ceil_div(units, K.parts), grid = umi::ceil_div(units, per);
 	for (int l = NL - 1; l >= 0; --l) {
 		const float* in = l == 0 ? K.at<float>(ws, K.x0) : K.at<float>(ws, K.act[l - 1]);
+		const float* d = K.at<float>(ws, dcur);
 		const int m = CH * CIN[l] * 9 + CH;
-		if (l == 3) UMI_TRY(wgrad_dil<DIL[3]>(in, dcur, part, K, units, per, grid, st));
-		else if (l == 2) UMI_TRY(wgrad_dil<DIL[2]>(in, dcur, part, K, units, per, grid, st));
-		else if (l == 1) UMI_TRY(wgrad_dil<DIL[1]>(in, dcur, part, K, units, per, grid, st));
+		if (l == 3) UMI_TRY(wgrad_dil<DIL[3]>(in, d, part, K, units, per, grid, st));
+		else if (l == 2) UMI_TRY(wgrad_dil<DIL[2]>(in, d, part, K, units, per, grid, st));
+		else if (l == 1) UMI_TRY(wgrad_dil<DIL[1]>(in, d, part, K, units, per, grid, st));
 		else {
-			menet_train::wgrad_first_kernel<<<grid, NT, 0, st>>>(in, dcur, part, K.H4, K.W4, units, per);
+			menet_train::wgrad_first_kernel<<<grid, NT, 0, st>>>(in, d, part, K.H4, K.W4, units, per);
 			UMI_TRY(umi::launch_status("wgrad_first_kernel"));
 		}
 		// grads[w_l], then grads[b_l] right after it (same layout as the partial rows)
 		UMI_TRY(reduce_rows(part, grads + L.w[l], nullptr, grid, m, m, bits, l == 0 ? err : nullptr, st));
 		if (l > 0) {  // data gradient, masked by ReLU(a_{l-1})
-			UMI_TRY(umi::menet_dgrad(din, K.at<void>(ws, K.wt[l]), K.at<float>(ws, K.act[l - 1]), dnext,
-			                         l > 1 ? dout : nullptr, K.H4, K.W4, DIL[l], bits, wait_ns, st));
-			std::swap(dcur, dnext);
-			std::swap(din, dout);
+			UMI_TRY(umi::menet_dgrad(K.at<void>(ws, din), K.at<void>(ws, K.wt[l]), K.at<float>(ws, K.act[l - 1]),
+			                         K.at<float>(ws, dnext), l > 1 ? K.at<void>(ws, dcur) : nullptr, K.H4, K.W4, DIL[l],
+			                         bits, wait_ns, st));
+			const size_t read = din;
+			din = dcur;
+			dcur = dnext;
+			dnext = read;
 		}
 	}
 	return umi::ok();
@@ -574,8 +602,8 @@ extern "C" umi_status umi_me_learned_u8(const uint8_t* cur, const uint8_t* ref, 
                                         void* workspace, size_t workspace_bytes, void* stream) {
 	UMI_TRY(check_frame(h, w));
 	if (!cur || !ref || !params || !mv || !workspace) return umi::fail(UMI_ERR_INVALID_ARG, "me_learned: null pointer");
-	const Work K(h, w);
-	if (workspace_bytes < K.bytes) return umi::fail(UMI_ERR_NO_MEMORY, "me_learned: workspace too small");
+	const Work K(h, w, workspace_bytes);
+	if (workspace_bytes < K.least) return umi::fail(UMI_ERR_NO_MEMORY, "me_learned: workspace too small");
 	if (!umi::aligned(workspace, 256)) return umi::fail(UMI_ERR_INVALID_ARG, "me_learned: workspace alignment");
 	if (refine_r < 1 || full_r < refine_r || full_r > 64)
 		return umi::fail(UMI_ERR_UNSUPPORTED, "me_learned: refine %d / full %d ranges", refine_r, full_r);
@@ -586,7 +614,7 @@ extern "C" umi_status umi_me_learned_u8(const uint8_t* cur, const uint8_t* ref, 
 	                              K.at<int32_t>(ws, K.amv)};
 	umi::MeAudit audit;
 	UMI_TRY(umi::me_audit_begin(cur, ref, h, w, full_r, audit_stride, fb, st, &audit));
-	UMI_TRY(infer(cur, ref, h, w, params, ws, K.at<int32_t>(ws, K.err), st));
+	UMI_TRY(infer(cur, ref, w, params, K, ws, K.at<int32_t>(ws, K.err), st));
 	int32_t* centers = K.at<int32_t>(ws, K.centers);
 	centers_kernel<<<grid_for(2 * (size_t)K.nblk), NT, 0, st>>>(K.at<float>(ws, K.pred), centers, K.nblk,
 	                                                             full_r - refine_r, umi::MeZero{fb.count, audit_sums});

@@ -77,8 +77,8 @@ struct Pack {
 	float* fwd[4];
 	__nv_bfloat16* bwd[4];
 };
-__global__ void pack_weights_kernel(const Pack p) {
-	const int l = blockIdx.y, cin = l == 0 ? 2 : CH;
+__global__ void pack_weights_kernel(const Pack p, int first) {
+	const int l = first + blockIdx.y, cin = l == 0 ? 2 : CH;
 	const float* w = l == 0 ? p.w[0] : l == 1 ? p.w[1] : l == 2 ? p.w[2] : p.w[3];
 	float* fwd = l == 0 ? p.fwd[0] : l == 1 ? p.fwd[1] : l == 2 ? p.fwd[2] : p.fwd[3];
 	__nv_bfloat16* bwd = l == 1 ? p.bwd[1] : l == 2 ? p.bwd[2] : p.bwd[3];
