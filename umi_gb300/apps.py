@@ -29,6 +29,7 @@ from __future__ import annotations
 
 import functools
 import math
+import operator
 
 import numpy as np
 
@@ -61,22 +62,12 @@ def _img(h, w, mode=WRAP, a_view=None, stage=1, out=False):
     return m
 
 
-_PLAIN = (int, float, bool, str, type(None))
+def _int(v):
+    """v as a plain int: plans are kept by value, never by an array's or a tensor's identity."""
+    return v if type(v) is int else operator.index(v)
 
 
-def _kept(make):
-    """make(...) with its last results kept.  Arguments that are not plain values
-    (an array or a tensor, which its owner may change) are computed anew."""
-    kept = functools.lru_cache(maxsize=64, typed=True)(make)
-
-    @functools.wraps(make)
-    def get(*args):
-        plain = all(type(a) in _PLAIN or isinstance(a, np.generic) for a in args)
-        return (kept if plain else make)(*args)
-    return get
-
-
-@_kept
+@functools.lru_cache(maxsize=64, typed=True)
 def _census_plan(h, w, radius):
     k = 2 * radius + 1
     d = U.make_desc(p=_p(h, w), a=[(1, 1), (1, 1), (k, k), (k, k)],
@@ -84,7 +75,7 @@ def _census_plan(h, w, radius):
     return U.PlannedLaunch(d, U.STRATEGY_CENSUS_I32)
 
 
-@_kept
+@functools.lru_cache(maxsize=64, typed=True)
 def _extremum_plan(h, w, radius, strategy, init):
     k = 2 * radius + 1
     d = U.make_desc(p=_p(h, w), a=[(1, 1), (1, 1), (k, k), (k, k)],
@@ -92,7 +83,7 @@ def _extremum_plan(h, w, radius, strategy, init):
     return U.PlannedLaunch(d, strategy, [init])
 
 
-@_kept
+@functools.lru_cache(maxsize=64, typed=True)
 def _box_plan(h, w, radius):
     k = 2 * radius + 1
     # corner (a_y, a_x) of point (y, x): J[clamp(y - r + a_y k)][clamp(x - r + a_x k)]
@@ -104,7 +95,7 @@ def _box_plan(h, w, radius):
     return U.PlannedLaunch(d, U.STRATEGY_WEIGHTED_SUM_I32, [0])
 
 
-@_kept
+@functools.lru_cache(maxsize=64, typed=True)
 def _gaussian_plans(h, w, k):
     r = k // 2
     dh = U.make_desc(p=_p(h, w), a=[(1, 1), (1, 1), (1, 1), (k, k)],
@@ -131,7 +122,7 @@ def census(img, radius: int = 1, out=None, stream=None):
     h, w = img.shape
     if out is None:
         out = torch.empty((h, w), dtype=torch.int32, device=img.device)
-    _census_plan(h, w, radius)((img, img), (out,), stream)
+    _census_plan(h, w, _int(radius))((img, img), (out,), stream)
     return out
 
 
@@ -140,7 +131,7 @@ def _extremum(img, radius, strategy, init, out, stream):
     h, w = img.shape
     if out is None:
         out = torch.empty((h, w), dtype=torch.int32, device=img.device)
-    _extremum_plan(h, w, radius, strategy, init)((img,), (out,), stream)
+    _extremum_plan(h, w, _int(radius), strategy, init)((img,), (out,), stream)
     return out
 
 
@@ -159,7 +150,7 @@ def _box_direct(img, radius, out, J, ii):
     image: buffers of its shape that do not overlap (through J, each step had
     read its input before the next one wrote)."""
     h, w = img.shape
-    if not (0 < h <= 500000 and 0 < w and isinstance(radius, int) and 0 <= radius <= 1 << 20):
+    if not (0 < h <= 500000 and 0 < w and 0 <= radius <= 1 << 20):
         return False
     if (J is not None and tuple(J.shape) != (h + 1, w + 1)) or any(
             t is not None and tuple(t.shape) != (h, w) for t in (out, ii)):
@@ -176,6 +167,7 @@ def box_sum(img_u8, radius: int, out=None, J=None, ii=None, workspace=None, stre
     import torch
     h, w = img_u8.shape
     dev = img_u8.device
+    radius = _int(radius)
     if _box_direct(img_u8, radius, out, J, ii):
         U._need(img_u8, torch.uint8, "inp")
         ii = torch.empty((h, w), dtype=torch.int32, device=dev) if ii is None else ii
@@ -204,9 +196,15 @@ def gaussian_kernel(sigma: float, radius: int | None = None) -> np.ndarray:
     return _gaussian_kernel(sigma, radius).copy()
 
 
-@_kept
-def _gaussian_kernel(sigma: float, radius: int | None) -> np.ndarray:
-    r = int(math.ceil(3 * sigma)) if radius is None else int(radius)
+def _gaussian_kernel(sigma, radius) -> np.ndarray:
+    if type(sigma) is not float and isinstance(sigma, np.ndarray):
+        sigma = sigma[()]
+    return _kernel_of(sigma, radius if radius is None or type(radius) is int else int(radius))
+
+
+@functools.lru_cache(maxsize=64, typed=True)
+def _kernel_of(sigma: float, radius: int | None) -> np.ndarray:
+    r = int(math.ceil(3 * sigma)) if radius is None else radius
     t = np.arange(-r, r + 1, dtype=np.float64)
     k = np.exp(-t * t / (2.0 * sigma * sigma))
     return (k / k.sum()).astype(np.float32)
