@@ -22,8 +22,10 @@ inline umi_status launch_status(const char* what) { return cuda_status(cudaGetLa
 // there is (4 KB of the 227 left to its static arrays).  The limit belongs to
 // the function, not to a launch: set to what one launch needs, it would refuse
 // another host thread's larger launch between that one's setting and its launch.
+// 48 KB, static arrays included, are allowed from the start.
 constexpr int kMaxDynamicShared = 223 * 1024;
-template <class K> umi_status allow_shared(K* kern) {
+template <class K> umi_status allow_shared(K* kern, size_t bytes) {
+	if (bytes <= 44 * 1024) return UMI_OK;
 	return cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicShared),
 	                   "cudaFuncSetAttribute");
 }

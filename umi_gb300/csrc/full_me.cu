@@ -600,7 +600,7 @@ template <int B, int G>
 umi_status launch_g(const uint8_t* cur, const uint8_t* ref, int32_t* out, const MeGeom& g, int threads, size_t smem,
                     cudaStream_t st) {
 	auto kern = full_me_kernel<B, G>;
-	if (smem > 48 * 1024) UMI_TRY(umi::allow_shared(kern));
+	UMI_TRY(umi::allow_shared(kern, smem));
 	// Without this the driver may pick a small shared-memory carveout and
 	// allow only one CTA per SM.
 	UMI_TRY(umi::cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -614,7 +614,7 @@ template <int B, int G>
 umi_status launch_pipe_g(const uint8_t* cur, const uint8_t* ref, const int32_t* centers, int32_t* out, const MeGeom& g,
                          int threads, size_t smem, cudaStream_t st) {
 	auto kern = full_me_pipe_kernel<B, G>;
-	if (smem > 48 * 1024) UMI_TRY(umi::allow_shared(kern));
+	UMI_TRY(umi::allow_shared(kern, smem));
 	UMI_TRY(umi::cuda_status(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
 	                                              (int)cudaSharedmemCarveoutMaxShared), "cudaFuncSetAttribute"));
 	int dev = 0, sms = 0, per_sm = 0;

@@ -226,7 +226,7 @@ umi_status full_me_8(const uint8_t* cur, const uint8_t* ref, int h, int w, int r
 	const int warps = rounds <= kMaxWarps ? std::max(rounds, 4) : 8;
 	const size_t smem = 2 * (size_t)a.wrows * a.pitch * sizeof(uint32_t);
 	auto kern = a.lanes < kLanes ? full_me_8_kernel<true> : full_me_8_kernel<false>;
-	if (smem > 48 * 1024) UMI_TRY(allow_shared(kern));
+	UMI_TRY(allow_shared(kern, smem));
 	kern<<<a.runs_x * nby, 32 * warps, smem, st>>>(a);
 	return launch_status("full_me_8_kernel");
 }

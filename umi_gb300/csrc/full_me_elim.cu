@@ -570,7 +570,7 @@ __global__ void __launch_bounds__(HALVES ? 2 * MAXT : MAXT, MINB) full_me_elim_k
 template <int MINB, bool HALVES>
 umi_status launch(const ElimArgs& a, int threads, size_t smem, int sms, cudaStream_t st) {
 	auto kern = full_me_elim_kernel<MINB, HALVES>;
-	if (smem > 48 * 1024) UMI_TRY(umi::allow_shared(kern));
+	UMI_TRY(umi::allow_shared(kern, smem));
 	// a list's length is known on the GPU only: CTAs that fill it once take its blocks in turn
 	const int grid = a.list ? std::min(a.units, MINB * sms) : a.units;
 	kern<<<grid, threads, smem, st>>>(a);

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(NT) separable_kernel(const SepArgs a) {
 
 template <int K>
 umi_status launch(const SepArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
-	if (smem > 48 * 1024) UMI_TRY(umi::allow_shared(separable_kernel<K>));
+	UMI_TRY(umi::allow_shared(separable_kernel<K>, smem));
 	separable_kernel<K><<<grid, NT, smem, st>>>(a);
 	return umi::launch_status("separable_kernel");
 }

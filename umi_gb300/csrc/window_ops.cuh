@@ -317,7 +317,7 @@ inline bool image_map(const umi_mem_plan& m, bool loop, int* sy, int* sx) {
 template <class Op, int KX>
 umi_status launch_kx(const Args<Op>& a, dim3 grid, size_t smem, cudaStream_t st) {
 	auto kern = window_kernel<Op, KX>;
-	if (smem > 48 * 1024) UMI_TRY(umi::allow_shared(kern));
+	UMI_TRY(umi::allow_shared(kern, smem));
 	kern<<<grid, NT, smem, st>>>(a);
 	return UMI_OK;
 }
