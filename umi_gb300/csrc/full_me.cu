@@ -728,8 +728,11 @@ umi_status full_me_common(const uint8_t* cur, const uint8_t* ref, int32_t h, int
 	const size_t smem = (size_t)m * g.mb_stride * 4;
 	const cudaStream_t st = umi::as_stream(stream);
 	umi_status rc;
+	// The leftover columns' groups of G2 rows may end below the main groups; their
+	// last rows' sums are not used, but their words are read.
+	const size_t below = g.ng2 ? std::max(0, g.ng2 * G2 - g.ng * G) * (size_t)g.win_words * 4 : 0;
 	if (!volume)  // 8x8 blocks: at most 160 KB of the two buffers (+-64)
-		rc = launch_pipe_b<8>(G, cur, ref, centers, out, g, threads_for(m * g.tasks_pipe), 2 * smem, st);
+		rc = launch_pipe_b<8>(G, cur, ref, centers, out, g, threads_for(m * g.tasks_pipe), 2 * smem + below, st);
 	else
 		rc = b == 16 ? launch_b<16>(G, cur, ref, out, g, threads, smem, st) : launch_b<8>(G, cur, ref, out, g, threads, smem, st);
 	return rc == UMI_OK ? umi::ok() : rc;
