@@ -11,16 +11,17 @@
 // C = sum |q_cur - q_ref|: four `vabsdiff4` per candidate instead of 64.  The
 // candidate of least C is summed exactly; with U its SAD, only candidates with
 // 16 C - 240 <= U can reach the minimum (or tie with it), and only those are
-// summed.  On the benchmark's frame pairs that leaves about 30 of 4225 at
-// +-32, on a panning camera 170; a block that keeps more than an eighth of
-// its candidates (noise, unrelated frames) is searched exhaustively by the
-// same CTA.
+// summed: about 30 of 4225 at +-32 on the benchmark's frame pairs, 170 on a
+// panning camera.  Where more are left (unrelated frames: a sixth), whole columns
+// of eleven rows that hold one are summed; where a cell's mean says no more than
+// its neighbours' (noise; told from the first two blocks' pixels) every candidate
+// is, without the bound.
 //
 // What bounds it: the integer ALU pipe (the bound's `vabsdiff4`, the cells'
-// byte permutations) and issue.  One CTA serves a run of NB horizontally
-// adjacent blocks (their windows overlap, so the cells of the run's window are
-// formed once), one block when the blocks come from a list or are moved by
-// centres:
+// byte permutations, the exact sums) and issue.  One CTA serves a run of NB
+// horizontally adjacent blocks (their windows overlap, so the cells of the run's
+// window are formed once), one block when the blocks come from a list or are
+// moved by centres:
 //   0. the window's pixels to shared memory (rows and columns clamped);
 //   1. cells: lane = 16 columns x 3 rows; every position x stores the word of
 //      its four cells x, x + 4, x + 8, x + 12, so that a candidate's cell row
@@ -31,21 +32,23 @@
 //   3. the least C of each block; its exact SAD, by every warp for itself;
 //   4. the survivors' list, from the costs still in registers;
 //   5. exact SADs of the survivors, eight lanes of two rows per candidate;
-//      blocks with too many survivors: every candidate, thread = (column,
-//      5 rows).
+//      blocks with too many survivors: thread = (column, group of rows).
 // Everything is shared memory and barriers: no workspace, no waits on other
 // CTAs.
 //
-// Measured on a GB300, exhaustive search before -> now: 1080p +-32, blocks
-// moved one by one 0.150 -> 0.0435 ms, panning camera 0.150 -> 0.064 ms; 1080p
-// +-16 0.088 -> 0.025 ms; 4K +-64 2.19 -> 0.76 ms.  Content the bound does not
-// serve pays for trying it: unrelated frames 0.150 -> 0.179 ms, independent
-// noise 0.150 -> 0.218 ms.  62 % of the issue slots are used (27 warps per SM
-// between barriers); by phase at 1080p +-32: pixels 12 us, cells 8, bound 14,
-// survivors 5, exact sums 5.  Tried: two blocks per run on 160 threads (0.058
-// ms), three on 224 (0.047), six cell rows per lane (0.048), a persistent form
-// with the next run's pixels in flight (0.051), noise left to a second,
-// warp-specialised launch (0.055 with noise at 0.173).
+// Measured on a GB300 (graph replays, ms), every candidate summed by a
+// warp-specialised kernel -> here: 1080p +-32, blocks moved one by one 0.148 ->
+// 0.0405, panning camera 0.148 -> 0.046, unrelated frames 0.148 -> 0.119, noise
+// 0.148 -> 0.155; +-64 0.580 -> 0.202, unrelated 0.52, noise 0.585; +-16 (by the
+// general kernel) 0.087 -> 0.0225, 0.051, 0.054; 4K +-64 2.19 -> 0.74, noise 2.29.
+// Noise costs up to 7 % (4K, +-32) where the windows were fetched ahead by warps of
+// their own.  At 86 % of the ALU pipe it is bound by that.  By phase at 1080p +-32:
+// pixels 12 us, cells 8, bound 14, survivors 5, exact sums 5.  Tried: two blocks per
+// run on 160 threads (0.058 ms), three on 224 (0.047), six cell rows per lane
+// (0.048), a persistent form with the next run's pixels in flight (0.051), noise
+// left to a second, warp-specialised launch (0.055 with noise at 0.173), two to four
+// neighbouring runs per CTA, the later ones without the bound after a hard one
+// (0.045, panning camera 0.070).
 #include <algorithm>
 
 #include "common.h"
@@ -53,13 +56,25 @@
 namespace {
 
 constexpr int RC = 33;       // candidate rows per pass of the bound, two passes per thread
-constexpr int QS = 132;      // words per row of the cell words: columns of a run's window, a multiple of 4
-constexpr int MAXT = 288;    // threads: the columns of one run
+// SW: words per window row, an odd number of 16-byte pieces for 16 nb + 2 r
+// pixels; QS: words per row of the cell words, the columns of a run's window, a
+// multiple of 4; THREADS: at most, for a column each.
+struct Wide {
+	static constexpr int SW = 36, QS = 132, THREADS = 288;
+};
+// One block, +-32 at most: lists, centres and frames with too few runs.  A third of
+// Wide's shared memory, so that seven CTAs fit (1080p with centres, +-32: 99 us, 157
+// with Wide; 256 x 448, +-32: 14.6 and 17.0).
+struct Narrow {
+	static constexpr int SW = 20, QS = 68, THREADS = 128;
+};
+constexpr int MAXT = Wide::THREADS;
 constexpr int MAXNB = 8;
 constexpr int NC = MAXNB / 2;     // cells of a run per lane
 constexpr size_t kSmemThree = 74 * 1024;  // dynamic shared memory that leaves room for three CTAs per SM
 constexpr int CR = 3;        // cell rows per lane and step
-constexpr int BG = 5;        // candidate rows per thread of the exhaustive search
+constexpr int GA = 17, GB = 22;  // candidate rows per thread of the search of every candidate
+constexpr int GS = 11;           // and where rows without a survivor are left out (8: 6 % slower)
 
 __device__ __forceinline__ uint32_t sad4(uint32_t a, uint32_t b, uint32_t c) {
 	uint32_t d;
@@ -117,18 +132,22 @@ struct ElimArgs {
 	int nb;                     // blocks per run (1 with a list or centres)
 	int runs_x, units;          // runs per block row; runs in all (slots with a list or centres)
 	int nchunk;                 // threads per column, two passes of RC rows each (one when nd <= RC)
-	int wrows, wwords, sw;      // window: rows, words per row, row stride in words (an odd number of 16-byte pieces)
+	int wrows, wwords;          // window: rows, words per row
 	int qrows, ncols, spw;      // cells: rows, columns; row pieces a warp forms at a time
 	int pieces;                 // 16-byte pieces per window row
 	int limit;                  // survivors a block may keep before it is searched exhaustively
+	int rows;                   // of every candidate's search: GA or GB
+	int cols;                   // columns of the exhaustive search in tasks, the others one by one
+	int tasks;                  // of the exhaustive search, per block
 	int cur_words;              // cur's rows are 4-byte aligned
 	int ref_pieces;             // ref's rows are 16-byte aligned
 	int cur_pieces;             // cur's rows are 16-byte aligned
 	Div div_x;                  // by blocks or runs per block row
-	SmallDiv div_nd, div_task, div_piece, div_spw;  // by nd, nd * nchunk, pieces, spw
+	SmallDiv div_nd, div_task, div_piece, div_spw, div_tasks, div_cols;  // by nd, nd * nchunk, pieces, spw, tasks, cols
 	uint32_t mul16, mul64k;     // 16 and 2^16 (runtime values: the keys stay multiply-adds, off the ALU pipe)
 	// shared memory offsets in words
 	int copy, o_copy;           // stride and start of the shifted windows (over the cell words)
+	int o_task;                 // tasks of the exhaustive search (over the cell words too)
 	int team_words;             // shared memory of a team
 	int o_q, o_blk, o_cell, o_list;
 };
@@ -143,44 +162,44 @@ __device__ __forceinline__ uint32_t pixels4(const uint8_t* __restrict__ frame, s
 	return v;
 }
 
-// SADs of BG candidate rows of one column against the block: the least, as
-// sad * 16 + row.  p: the column's words, shifted so that they start on a word
-// (row stride sw).  A ring of BG window rows meets each block row.
-__device__ __forceinline__ uint32_t exhaustive_rows(const uint32_t* __restrict__ p, int sw,
-                                                    const uint4* __restrict__ blk, int rows) {
-	uint32_t ring[BG][4], acc[BG];
-	auto fetch = [&](uint32_t (&v)[4]) {
+// SADs of G candidate rows of one column against the block: the least, as
+// sad * 32 + row (of the first `rows`, where they are fewer).  p: the column's words, shifted so that they
+// start on a word.  One word of the rows at a time: a ring of G window words
+// meets each block row, so the registers hold G sums and G words, and the SADs
+// need 0.15 loads each and no address arithmetic.
+template <int G, int SW>
+__device__ __forceinline__ uint32_t exhaustive_rows(const uint32_t* __restrict__ p, const uint32_t* __restrict__ blk,
+                                                    int rows) {
+	uint32_t acc[G];
 #pragma unroll
-		for (int k = 0; k < 4; ++k) v[k] = p[k];
-		p += sw;
-	};
+	for (int q = 0; q < G; ++q) acc[q] = 0;
+#pragma unroll 1
+	for (int k = 0; k < 4; ++k, ++p, ++blk) {
+		uint32_t ring[G];
 #pragma unroll
-	for (int q = 0; q < BG; ++q) acc[q] = 0;
+		for (int q = 0; q < G - 1; ++q) ring[q] = p[q * SW];
 #pragma unroll
-	for (int q = 0; q < BG - 1; ++q) fetch(ring[q]);
+		for (int py = 0; py < 16; ++py) {
+			const uint32_t c = blk[4 * py];
+			ring[(py + G - 1) % G] = p[(py + G - 1) * SW];
 #pragma unroll
-	for (int py = 0; py < 16; ++py) {
-		const uint4 c = blk[py];
-		fetch(ring[(py + BG - 1) % BG]);
-#pragma unroll
-		for (int q = 0; q < BG; ++q) {
-			const uint32_t(&v)[4] = ring[(py + q) % BG];
-			acc[q] = sad4(c.x, v[0], acc[q]);
-			acc[q] = sad4(c.y, v[1], acc[q]);
-			acc[q] = sad4(c.z, v[2], acc[q]);
-			acc[q] = sad4(c.w, v[3], acc[q]);
+			for (int q = 0; q < G; ++q) acc[q] = sad4(c, ring[(py + q) % G], acc[q]);
 		}
 	}
-	uint32_t k = 0xffffffffu;
+	if (rows < G)  // a range below eight
 #pragma unroll
-	for (int q = 0; q < BG; ++q)
-		if (q < rows) k = min(k, acc[q] * 16u + (uint32_t)q);
+		for (int q = 1; q < G; ++q)
+			if (q >= rows) acc[q] = 1u << 26;
+	uint32_t k = acc[0] * 32u;
+#pragma unroll
+	for (int q = 1; q < G; ++q) k = min(k, acc[q] * 32u + (uint32_t)q);
 	return k;
 }
 
 // Costs of rows y0 .. y0 + RC - 1 of one column (col: the shared address of
 // cell row y0), packed: p[i] = cost[i] | cost[i + 16] << 16, p16 = cost[32].
 // Returns the least cost * 64 + row (the first row among equals).
+template <int QS>
 __device__ __forceinline__ uint32_t bound_rows(unsigned col, const uint32_t (&c)[4], int rows, uint32_t mul16,
                                                uint32_t mul64k, uint32_t (&p)[16], uint32_t& p16) {
 	uint32_t cost[RC];
@@ -223,10 +242,11 @@ __device__ __forceinline__ uint32_t survivors(const uint32_t (&p)[16], uint32_t 
 struct Run {
 	int blk0, bx0, by, nb, cy, cx;
 };
+template <bool LIST>
 __device__ __forceinline__ Run run_of(const ElimArgs& a, int unit) {
 	Run u{0, 0, 0, 1, 0, 0};
-	if (a.list || a.centers) {
-		u.blk0 = a.list ? a.list[unit] : unit;
+	if (LIST || a.centers) {
+		u.blk0 = LIST ? a.list[unit] : unit;
 		u.by = a.div_x(u.blk0);
 		u.bx0 = u.blk0 - u.by * a.nbx;
 		if (a.centers) {
@@ -244,6 +264,7 @@ __device__ __forceinline__ Run run_of(const ElimArgs& a, int unit) {
 
 // A run's window and blocks into shared memory, cp.async where the source is
 // aligned (words past the last block's window are loaded but not used).
+template <int SW>
 __device__ __forceinline__ void load_run(const ElimArgs& a, const Run& u, uint32_t* win, uint32_t* blkw, int row0,
                                          int piece, int piece_rows, int tid, int nt) {
 	const int warp = tid >> 5, lane = tid & 31, nwarps = nt >> 5;
@@ -251,14 +272,14 @@ __device__ __forceinline__ void load_run(const ElimArgs& a, const Run& u, uint32
 	if (a.ref_pieces && (gx0 & 15) == 0 && gx0 >= 0 && gx0 + 16 * a.pieces <= a.w) {
 		const uint8_t* src = a.ref + gx0 + 16 * piece;
 		for (int row = row0; row < a.wrows; row += piece_rows)
-			copy16(win + row * a.sw + 4 * piece, src + (size_t)min(max(gy0 + row, 0), a.h - 1) * a.w);
+			copy16(win + row * SW + 4 * piece, src + (size_t)min(max(gy0 + row, 0), a.h - 1) * a.w);
 	} else {
 		const size_t total = (size_t)a.h * a.w;
 		for (int row = warp; row < a.wrows; row += nwarps) {
 			const size_t off = (size_t)min(max(gy0 + row, 0), a.h - 1) * a.w;
 			for (int k = lane; k < a.wwords; k += 32) {
 				const int gx = gx0 + 4 * k;
-				uint32_t* dst = win + row * a.sw + k;
+				uint32_t* dst = win + row * SW + k;
 				const size_t o = off + gx;
 				const uintptr_t p = reinterpret_cast<uintptr_t>(a.ref) + o;
 				if (gx < 0 || gx + 4 > a.w) {
@@ -299,14 +320,15 @@ __device__ __forceinline__ void load_run(const ElimArgs& a, const Run& u, uint32
 // The next group's columns come from lane + spw (the last group's are not
 // needed: it holds the window's last 16 columns).
 // Sums are clamped to [lo, lo + 2^s * 256) and stored as (sum - lo) >> s.
+template <int SW, int QS>
 __device__ __forceinline__ void form_cells(const ElimArgs& a, const uint32_t* __restrict__ win, uint32_t* __restrict__ q,
                                            int y0, int g, int cols, uint32_t lo, int sh) {
 	const uint32_t lo2 = lo * 0x10001u, hi2 = lo2 + ((256u << sh) - 1u) * 0x10001u;
-	const uint32_t* src = win + y0 * a.sw + 4 * g;
+	const uint32_t* src = win + y0 * SW + 4 * g;
 	uint32_t ring[3][8], sum[8];
 	auto row = [&](uint32_t (&v)[8]) {
 		const uint4 x = *reinterpret_cast<const uint4*>(src);
-		src += a.sw;
+		src += SW;
 		const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
 		for (int k = 0; k < 4; ++k) {
@@ -359,31 +381,92 @@ __device__ __forceinline__ void form_cells(const ElimArgs& a, const uint32_t* __
 	}
 }
 
+// Exact SAD of a candidate of block b by eight lanes (sub 0 .. 7), two rows each.
+template <int SW>
+__device__ __forceinline__ void exact_sum(const ElimArgs& a, const uint32_t* win, const uint32_t* blkw, uint32_t* best,
+                                          int b, int iy, int ix, int sub) {
+	const int X = 16 * b + ix;
+	const uint32_t* w = win + (iy + sub) * SW + (X >> 2);
+	const uint4* cr = reinterpret_cast<const uint4*>(blkw + b * 64) + sub;
+	const uint32_t sel = 0x3210u + 0x1111u * (uint32_t)(X & 3);
+	uint32_t s = 0;
+#pragma unroll
+	for (int h = 0; h < 2; ++h) {
+		const uint4 c = cr[8 * h];
+		uint32_t v[5];
+#pragma unroll
+		for (int k = 0; k < 5; ++k) v[k] = w[8 * h * SW + k];
+		s = sad4(c.x, __byte_perm(v[0], v[1], sel), s);
+		s = sad4(c.y, __byte_perm(v[1], v[2], sel), s);
+		s = sad4(c.z, __byte_perm(v[2], v[3], sel), s);
+		s = sad4(c.w, __byte_perm(v[3], v[4], sel), s);
+	}
+#pragma unroll
+	for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+	if (sub == 0) atomicMin(&best[b], (s << 15) | (uint32_t)(iy * a.nd + ix));
+}
+
+// A whole warp's keys into their blocks' least.
+__device__ __forceinline__ void least_of(uint32_t* best, int b, uint32_t key, int lane) {
+	if (__all_sync(0xffffffffu, b == __shfl_sync(0xffffffffu, b, 0))) {
+		const uint32_t least = __reduce_min_sync(0xffffffffu, key);
+		if (lane == 0) atomicMin(&best[b], least);
+	} else {
+		atomicMin(&best[b], key);
+	}
+}
+
+// Exact SADs of `count` tasks (block, group of G rows, column), one per thread, by
+// the warps that make as many for each of the SM's four schedulers (a ninth would
+// keep one of them busy half as long again).
+template <int G, int SW>
+__device__ __forceinline__ void exhaustive(const ElimArgs& a, const uint32_t* tasks, int count, const uint32_t* win,
+                                           const uint32_t* copies, const uint32_t* blkw, uint32_t* best, int tid, int nt) {
+	const int lane = tid & 31, nw = nt >= 128 ? nt & ~127 : nt;
+	if (tid >= nw) return;
+	for (int t0 = tid - lane; t0 < count; t0 += nw) {  // warp-uniform
+		const uint32_t e = tasks[min(t0 + lane, count - 1)];  // lanes past the end repeat the last task
+		const int b = (int)(e >> 16), ix = (int)(e & 255u), iy = max(min((int)(e >> 8 & 255u) * G, a.nd - G), 0);
+		const uint32_t* w = (ix & 3 ? copies + ((ix & 3) - 1) * a.copy : win) + iy * SW + ((16 * b + ix) >> 2);
+		const uint32_t s = exhaustive_rows<G, SW>(w, blkw + b * 64, a.nd);
+		const uint32_t key = ((s >> 5) << 15) | (uint32_t)((iy + (int)(s & 31u)) * a.nd + ix);
+		least_of(best, b, key, lane);
+	}
+}
+
+// Whether one of the rows s .. s + n - 1 is a survivor: bit i of m row i, e row 32.
+__device__ __forceinline__ bool any_row(uint32_t m, bool e, int s, int n) {
+	const uint64_t v = m | ((uint64_t)e << 32), rows = ((uint64_t)1 << n) - 1;
+	return s <= -n || s > 32 ? false : (v & (s >= 0 ? rows << s : rows >> -s)) != 0;
+}
+
 // MINB: CTAs per SM (three at 72 registers; two where shared memory holds no
-// more).  HALVES: a list of blocks with windows of more than 66 rows, whose
-// length only the GPU knows.  One CTA per SM takes a block with all its threads
-// if the list has no more blocks than there are CTAs, and otherwise works as two
-// teams with a block each, of half the threads and shared memory, that never
-// wait for one another.  (A fallback list of 130 blocks at 1080p, +-64, most of
-// them hard: the pass around it 79 us with two CTAs per SM, 68 so; 28 000 blocks
-// at 4K: the pass 1.17 ms with all threads on each block, 0.91 so.)
-template <int MINB, bool HALVES>
-__global__ void __launch_bounds__(HALVES ? 2 * MAXT : MAXT, MINB) full_me_elim_kernel(const ElimArgs a) {
+// more; seven of Narrow).  TEAMS 0: a run per CTA.  Otherwise a list of blocks,
+// whose length only the GPU knows: with no more blocks than CTAs a CTA takes a
+// block with all its threads, beyond that it works as TEAMS teams with a block
+// each, of a share of the threads and shared memory, that never wait for one
+// another.  (Fallback list of 130 blocks at 1080p, +-64, most of them hard: the pass
+// around it 79 us with two CTAs per SM, 68 so; 28 000 blocks at 4K: 1.17 ms with all
+// threads on each block, 0.91 so.)
+template <class W, int MINB, int TEAMS>
+__global__ void __launch_bounds__(W::THREADS * (TEAMS ? TEAMS : 1), MINB) full_me_elim_kernel(const ElimArgs a) {
+	constexpr int SW = W::SW, QS = W::QS, NT = W::THREADS, N = TEAMS ? TEAMS : 1;
+	constexpr bool LIST = TEAMS > 0;
 	extern __shared__ __align__(16) uint32_t smem[];
-	__shared__ uint32_t seeds[2][MAXNB], bests[2][MAXNB];
-	__shared__ int cnts[2][MAXNB], totals[2];
+	__shared__ uint32_t seeds[N][MAXNB], bests[N][MAXNB];
+	__shared__ int cnts[N][MAXNB], totals[N], tasks[N];
 	int units = a.units;
-	if (a.list) units = min(units, *a.list_count);
-	const bool teams = HALVES && units > (int)gridDim.x;
-	const int team = teams ? (int)threadIdx.x / MAXT : 0, nteams = teams ? 2 : 1;
-	const int tid = (int)threadIdx.x - team * MAXT, nt = teams ? MAXT : (int)blockDim.x;
+	if (LIST) units = min(units, *a.list_count);
+	const bool teams = LIST && units > (int)gridDim.x;
+	const int team = teams ? (int)threadIdx.x / NT : 0, nteams = teams ? N : 1;
+	const int tid = (int)threadIdx.x - team * NT, nt = teams ? NT : (int)blockDim.x;
 	const int warp = tid >> 5, lane = tid & 31, nwarps = nt >> 5;
 	auto sync = [&] {  // the threads of this team
-		if (HALVES) asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(nt) : "memory");
+		if (LIST) asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(nt) : "memory");
 		else __syncthreads();
 	};
 	uint32_t *seed = seeds[team], *best = bests[team];
-	int *cnt = cnts[team], &total_cnt = totals[team];
+	int *cnt = cnts[team], &total_cnt = totals[team], &n_tasks = tasks[team];
 	uint32_t* sm = smem + team * a.team_words;
 	uint32_t* win = sm;              // [wrows][sw]
 	uint32_t* q = sm + a.o_q;        // [max(nd, RC) + 12][QS]: cell words
@@ -402,157 +485,179 @@ __global__ void __launch_bounds__(HALVES ? 2 * MAXT : MAXT, MINB) full_me_elim_k
 	const int piece_rows = nt / a.pieces, row0 = prow < piece_rows ? prow : a.wrows;
 
 	for (int unit = blockIdx.x * nteams + team; unit < units; unit += gridDim.x * nteams) {
-		const Run u = run_of(a, unit);
-		load_run(a, u, win, blkw, row0, piece, piece_rows, tid, nt);
+		const Run u = run_of<LIST>(a, unit);
+		load_run<SW>(a, u, win, blkw, row0, piece, piece_rows, tid, nt);
 		if (tid < MAXNB) {
 			seed[tid] = 0xffffffffu;
 			best[tid] = 0xffffffffu;
 			cnt[tid] = 0;
 		}
-		if (tid == 0) total_cnt = 0;
+		if (tid == 0) total_cnt = n_tasks = 0;
 		asm volatile("cp.async.wait_all;" ::: "memory");
 		sync();
-		// ---- 1. cells: cur's, by every warp for the scale; then the window's
-		uint32_t sums[NC], mn = 0xffffffffu, mx = 0;
+		// ---- 1. cells: cur's, by every warp for the scale and, from the first two
+		// blocks, for whether the bound can serve; then the window's
+		uint32_t sums[NC], mn = 0xffffffffu, mx = 0, differ = 0;
 #pragma unroll
 		for (int t = 0; t < NC; ++t) {
 			if (32 * t >= 16 * u.nb) break;
 			const int i = min(lane + 32 * t, 16 * u.nb - 1);
 			const uint32_t* px = blkw + (i >> 4) * 64 + ((i >> 2) & 3) * 16 + (i & 3);
-			uint32_t v = 0;
+			uint32_t v = 0, w[4];
 #pragma unroll
-			for (int k = 0; k < 4; ++k) v = sad4(px[4 * k], 0u, v);
+			for (int k = 0; k < 4; ++k) {
+				w[k] = px[4 * k];
+				v = sad4(w[k], 0u, v);
+			}
+			if (t == 0) {  // cells' differences with their neighbours (eighths) and pixels' with those below (quarters)
+				const uint32_t l = __shfl_xor_sync(0xffffffffu, v, 1), o = __shfl_xor_sync(0xffffffffu, v, 4);
+				const uint32_t cells = max(v, l) - min(v, l) + max(v, o) - min(v, o);
+				const uint32_t pixels = sad4(w[0], w[1], sad4(w[1], w[2], sad4(w[2], w[3], 0u)));
+				differ = __reduce_add_sync(0xffffffffu, lane < 16 * u.nb ? (cells >> 3) << 16 | pixels >> 2 : 0u);
+			}
 			sums[t] = v;
 			mn = min(mn, v);
 			mx = max(mx, v);
 		}
 		mn = __reduce_min_sync(0xffffffffu, mn);
 		mx = __reduce_max_sync(0xffffffffu, mx);
-		int sh = 2;
-		while (sh < 4 && (256u << sh) < 2 * (mx - mn)) ++sh;
-		const uint32_t half = 128u << sh, mid = (mn + mx) >> 1, lo = mid > half ? mid - half : 0u;
-		if (warp == 0) {
+		int hard = (1 << u.nb) - 1, count = -1;  // blocks and tasks of the exhaustive search (all of them)
+		// A list with few small windows is done soonest without the bound (130 blocks,
+		// +-32: 10 us whatever their content, else 9 to 14).  Elsewhere cells' sums that
+		// differ less from their neighbours' than 1.25 times the pixels from those below
+		// are noise: a random block stays below that in 999 of 1000 cases, one of the
+		// benchmark's texture (sigma 5.6, with noise of 2) above it.
+		const bool alone = LIST && !teams && NT == Narrow::THREADS;
+		if (!alone && 8 * (differ >> 16) >= 5 * (differ & 0xffffu)) {
+			hard = 0;
+			int sh = 2;
+			while (sh < 4 && (256u << sh) < 2 * (mx - mn)) ++sh;
+			const uint32_t half = 128u << sh, mid = (mn + mx) >> 1, lo = mid > half ? mid - half : 0u;
+			if (warp == 0) {
 #pragma unroll
-			for (int t = 0; t < NC; ++t)
-				if (lane + 32 * t < 16 * u.nb)
-					reinterpret_cast<uint8_t*>(cell)[lane + 32 * t] =
-						(uint8_t)((min(max(sums[t], lo), lo + (256u << sh) - 1u) - lo) >> sh);
-		}
-		// lane = (group gl of 16 columns, piece `seg` of CR rows)
-		for (int s0 = warp * a.spw; s0 * CR < a.qrows; s0 += nwarps * a.spw)
-			form_cells(a, win, q, (s0 + seg) * CR, min(gl, a.pieces - 1), gl < a.pieces ? a.ncols - 16 * gl : 0, lo, sh);
-		sync();
-		// ---- 2. bound
-		const bool task = tb < u.nb;
-		uint32_t p0[16], p1[16], l0 = 0, l1 = 0, k0 = 0xffffffffu, k1 = 0xffffffffu;
-		if (task) {
-			uint32_t c[4];
-#pragma unroll
-			for (int i = 0; i < 4; ++i) c[i] = cell[4 * tb + i];
-			const unsigned col = (unsigned)__cvta_generic_to_shared(q + 16 * tb + tx);
-			k0 = bound_rows(col + 4u * QS * iy0, c, nd - iy0, a.mul16, a.mul64k, p0, l0);
-			if (nd > RC) k1 = bound_rows(col + 4u * QS * iy1, c, RC, a.mul16, a.mul64k, p1, l1);
-		}
-		// ---- 3. the least C of each block
-		const uint32_t key = min(((k0 >> 6) << 15) | (uint32_t)((iy0 + (int)(k0 & 63u)) * nd + tx),
-		                         ((k1 >> 6) << 15) | (uint32_t)((iy1 + (int)(k1 & 63u)) * nd + tx));
-		if (wb0 == wb1) {
-			const uint32_t m = __reduce_min_sync(0xffffffffu, task ? key : 0xffffffffu);
-			if (lane == 0 && m != 0xffffffffu) atomicMin(&seed[tb], m);
-		} else if (task) {
-			atomicMin(&seed[tb], key);
-		}
-		sync();
-		uint32_t T = 0;
-		for (int b = wb0; b <= min(wb1, u.nb - 1); ++b) {
-			const uint32_t idx = seed[b] & 0x7fffu;
-			const int iy = a.div_nd((int)idx), X = 16 * b + (int)idx - iy * nd + 8 * (lane & 1);
-			const uint32_t* w = win + (iy + (lane >> 1)) * a.sw + (X >> 2);
-			const uint32_t sel = 0x3210u + 0x1111u * (uint32_t)(X & 3);
-			const uint2 c = *reinterpret_cast<const uint2*>(blkw + b * 64 + 2 * lane);
-			const uint32_t w1 = w[1];
-			const uint32_t s = sad4(c.x, __byte_perm(w[0], w1, sel), sad4(c.y, __byte_perm(w1, w[2], sel), 0u));
-			const uint32_t U = __reduce_add_sync(0xffffffffu, s);
-			if (lane == 0) atomicMin(&best[b], (U << 15) | idx);
-			if (b == tb) T = min((U + (16u << sh) - 16u) >> sh, 4095u);
-		}
-		// ---- 4. survivors
-		if (task && (min(k0, k1) >> 6) <= T) {
-			uint32_t m0 = 0, m1 = 0;
-			bool e0 = false, e1 = false;
-			if ((k0 >> 6) <= T) {
-				m0 = survivors(p0, T);
-				if (nd < RC) m0 &= 0xffffffffu >> (32 - nd);
-				e0 = nd >= RC && l0 <= T;
+				for (int t = 0; t < NC; ++t)
+					if (lane + 32 * t < 16 * u.nb)
+						reinterpret_cast<uint8_t*>(cell)[lane + 32 * t] =
+							(uint8_t)((min(max(sums[t], lo), lo + (256u << sh) - 1u) - lo) >> sh);
 			}
-			if ((k1 >> 6) <= T) {
-				m1 = survivors(p1, T);
-				e1 = l1 <= T;
+			// lane = (group gl of 16 columns, piece `seg` of CR rows)
+			for (int s0 = warp * a.spw; s0 * CR < a.qrows; s0 += nwarps * a.spw)
+				form_cells<SW, QS>(a, win, q, (s0 + seg) * CR, min(gl, a.pieces - 1), gl < a.pieces ? a.ncols - 16 * gl : 0, lo, sh);
+			sync();
+			// ---- 2. bound
+			const bool task = tb < u.nb;
+			uint32_t p0[16], p1[16], l0 = 0, l1 = 0, k0 = 0xffffffffu, k1 = 0xffffffffu;
+			if (task) {
+				uint32_t c[4];
+#pragma unroll
+				for (int i = 0; i < 4; ++i) c[i] = cell[4 * tb + i];
+				const unsigned col = (unsigned)__cvta_generic_to_shared(q + 16 * tb + tx);
+				k0 = bound_rows<QS>(col + 4u * QS * iy0, c, nd - iy0, a.mul16, a.mul64k, p0, l0);
+				if (nd > RC) k1 = bound_rows<QS>(col + 4u * QS * iy1, c, RC, a.mul16, a.mul64k, p1, l1);
 			}
-			const int n = __popc(m0) + __popc(m1) + e0 + e1;
-			if (atomicAdd(&cnt[tb], n) + n <= a.limit) {
-				uint32_t* dst = list + atomicAdd(&total_cnt, n);
-				const uint32_t e = ((uint32_t)tb << 16) | (uint32_t)tx;
-				if (e0) *dst++ = e + ((uint32_t)(iy0 + 32) << 8);
-				if (e1) *dst++ = e + ((uint32_t)(iy1 + 32) << 8);
-				for (; m0; m0 &= m0 - 1) *dst++ = e + ((uint32_t)(iy0 + __ffs((int)m0) - 1) << 8);
-				for (; m1; m1 &= m1 - 1) *dst++ = e + ((uint32_t)(iy1 + __ffs((int)m1) - 1) << 8);
-			}
-		}
-		sync();
-		// ---- 5. exact sums
-		int hard = 0;
-		for (int b = 0; b < u.nb; ++b) hard |= (cnt[b] > a.limit) << b;
-		const int n = hard == (1 << u.nb) - 1 ? 0 : total_cnt, sub = lane & 7;
-		for (int j0 = 4 * warp; j0 < n; j0 += 4 * nwarps) {
-			const uint32_t e = list[min(j0 + (lane >> 3), n - 1)];  // lanes past the end repeat the last candidate
-			const int b = (int)(e >> 16), iy = (int)(e >> 8 & 255u), ix = (int)(e & 255u), X = 16 * b + ix;
-			if (hard && __all_sync(0xffffffffu, hard >> b & 1)) continue;  // listed before its block had too many
-			const uint32_t* w = win + (iy + sub) * a.sw + (X >> 2);
-			const uint4* cr = reinterpret_cast<const uint4*>(blkw + b * 64) + sub;
-			const uint32_t sel = 0x3210u + 0x1111u * (uint32_t)(X & 3);
-			uint32_t s = 0;
-#pragma unroll
-			for (int h = 0; h < 2; ++h) {
-				const uint4 c = cr[8 * h];
-				uint32_t v[5];
-#pragma unroll
-				for (int k = 0; k < 5; ++k) v[k] = w[8 * h * a.sw + k];
-				s = sad4(c.x, __byte_perm(v[0], v[1], sel), s);
-				s = sad4(c.y, __byte_perm(v[1], v[2], sel), s);
-				s = sad4(c.z, __byte_perm(v[2], v[3], sel), s);
-				s = sad4(c.w, __byte_perm(v[3], v[4], sel), s);
-			}
-#pragma unroll
-			for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-			if (sub == 0) atomicMin(&best[b], (s << 15) | (uint32_t)(iy * nd + ix));
-		}
-		if (hard) {  // uniform over the CTA
-			// the window shifted by 1, 2, 3 bytes over the cells, copies 8 banks apart
-			uint32_t* copies = sm + a.o_copy;
-			for (int i = tid; i < a.wrows * a.sw; i += nt) {
-				const uint32_t x = win[i], y = win[i + 1];
-#pragma unroll
-				for (int k = 1; k < 4; ++k) copies[(k - 1) * a.copy + i] = __funnelshift_r(x, y, 8 * k);
+			// ---- 3. the least C of each block
+			const uint32_t key = min(((k0 >> 6) << 15) | (uint32_t)((iy0 + (int)(k0 & 63u)) * nd + tx),
+			                         ((k1 >> 6) << 15) | (uint32_t)((iy1 + (int)(k1 & 63u)) * nd + tx));
+			if (wb0 == wb1) {
+				const uint32_t m = __reduce_min_sync(0xffffffffu, task ? key : 0xffffffffu);
+				if (lane == 0 && m != 0xffffffffu) atomicMin(&seed[tb], m);
+			} else if (task) {
+				atomicMin(&seed[tb], key);
 			}
 			sync();
-			const int ng = (nd + BG - 1) / BG, tasks = nd * ng, all = __popc(hard) * tasks;
-			for (int t0 = tid - lane; t0 < all; t0 += nt) {  // warp-uniform
-				const int t = min(t0 + lane, all - 1);       // lanes past the end repeat the last task
-				const int hb = t / tasks, v = t - hb * tasks, g = a.div_nd(v), ix = v - g * nd;
-				int m = hard;
-				for (int k = 0; k < hb; ++k) m &= m - 1;
-				const int b = __ffs(m) - 1;
-				const uint32_t* w = (ix & 3 ? copies + ((ix & 3) - 1) * a.copy : win) + g * BG * a.sw + ((16 * b + ix) >> 2);
-				const uint32_t e = exhaustive_rows(w, a.sw, reinterpret_cast<const uint4*>(blkw + b * 64), nd - g * BG);
-				const uint32_t ekey = ((e >> 4) << 15) | (uint32_t)((g * BG + (int)(e & 15u)) * nd + ix);
-				if (__all_sync(0xffffffffu, b == __shfl_sync(0xffffffffu, b, 0))) {
-					const uint32_t least = __reduce_min_sync(0xffffffffu, ekey);
-					if (lane == 0) atomicMin(&best[b], least);
-				} else {
-					atomicMin(&best[b], ekey);
+			int T = -1;
+			for (int b = wb0; b <= min(wb1, u.nb - 1); ++b) {
+				const uint32_t idx = seed[b] & 0x7fffu;
+				const int iy = a.div_nd((int)idx), X = 16 * b + (int)idx - iy * nd + 8 * (lane & 1);
+				const uint32_t* w = win + (iy + (lane >> 1)) * SW + (X >> 2);
+				const uint32_t sel = 0x3210u + 0x1111u * (uint32_t)(X & 3);
+				const uint2 c = *reinterpret_cast<const uint2*>(blkw + b * 64 + 2 * lane);
+				const uint32_t w1 = w[1];
+				const uint32_t s = sad4(c.x, __byte_perm(w[0], w1, sel), sad4(c.y, __byte_perm(w1, w[2], sel), 0u));
+				const uint32_t U = __reduce_add_sync(0xffffffffu, s);
+				if (lane == 0) atomicMin(&best[b], (U << 15) | idx);
+				// an exact match: the seed, the first candidate of cost 0, is also the first exact one
+				if (b == tb && U != 0) T = (int)min((U + (16u << sh) - 16u) >> sh, 4095u);
+			}
+			// ---- 4. survivors
+			uint32_t m0 = 0, m1 = 0;
+			bool e0 = false, e1 = false;
+			if (task && (int)(min(k0, k1) >> 6) <= T) {
+				if ((int)(k0 >> 6) <= T) {
+					m0 = survivors(p0, (uint32_t)T);
+					if (nd < RC) m0 &= 0xffffffffu >> (32 - nd);
+					e0 = nd >= RC && (int)l0 <= T;
+				}
+				if ((int)(k1 >> 6) <= T) {
+					m1 = survivors(p1, (uint32_t)T);
+					e1 = (int)l1 <= T;
+				}
+				const int n = __popc(m0) + __popc(m1) + e0 + e1;
+				if (atomicAdd(&cnt[tb], n) + n <= a.limit) {
+					uint32_t* dst = list + atomicAdd(&total_cnt, n);
+					const uint32_t e = ((uint32_t)tb << 16) | (uint32_t)tx;
+					if (e0) *dst++ = e + ((uint32_t)(iy0 + 32) << 8);
+					if (e1) *dst++ = e + ((uint32_t)(iy1 + 32) << 8);
+					for (uint32_t m = m0; m; m &= m - 1) *dst++ = e + ((uint32_t)(iy0 + __ffs((int)m) - 1) << 8);
+					for (uint32_t m = m1; m; m &= m - 1) *dst++ = e + ((uint32_t)(iy1 + __ffs((int)m) - 1) << 8);
 				}
 			}
+			sync();
+			// ---- 5. exact sums
+			for (int b = 0; b < u.nb; ++b) hard |= (cnt[b] > a.limit) << b;
+			const int n = hard == (1 << u.nb) - 1 ? 0 : total_cnt, sub = lane & 7;
+			for (int j0 = 4 * warp; j0 < n; j0 += 4 * nwarps) {
+				const uint32_t e = list[min(j0 + (lane >> 3), n - 1)];  // lanes past the end repeat the last candidate
+				const int b = (int)(e >> 16);
+				if (hard && __all_sync(0xffffffffu, hard >> b & 1)) continue;  // listed before its block had too many
+				exact_sum<SW>(a, win, blkw, best, b, (int)(e >> 8 & 255u), (int)(e & 255u), sub);
+			}
+			if (hard) {  // uniform over the team: the tasks that hold a survivor
+				const bool mine = task && (hard >> tb & 1);
+#pragma unroll 1
+				for (int g = 0; g * GS < nd; ++g) {
+					const int y = max(min(g * GS, nd - GS), 0);
+					const bool any = mine && y + GS > 2 * RC * tc && (any_row(m0, e0, y - iy0, GS) || any_row(m1, e1, y - iy1, GS));
+					const uint32_t lanes = __ballot_sync(0xffffffffu, any);
+					int at = 0;
+					if (lane == 0 && lanes) at = atomicAdd(&n_tasks, __popc(lanes));
+					at = __shfl_sync(0xffffffffu, at, 0) + __popc(lanes & ((1u << lane) - 1u));
+					if (any) sm[a.o_task + at] = ((uint32_t)tb << 16) | ((uint32_t)g << 8) | (uint32_t)tx;
+				}
+			}
+		} else {
+			// every task; whole warps of columns where one or two are left over (+-16,
+			// 32, 48, 64), those by one lane a candidate, below
+			count = u.nb * a.tasks;
+			for (int t = tid; t < count; t += nt) {
+				const int b = a.div_tasks(t), v = t - b * a.tasks, g = a.div_cols(v);
+				sm[a.o_task + t] = ((uint32_t)b << 16) | ((uint32_t)g << 8) | (uint32_t)(v - g * a.cols);
+			}
+		}
+		if (hard) {  // uniform over the team
+			// the window shifted by 1, 2, 3 bytes over the cells, copies 8 banks apart
+			uint32_t* copies = sm + a.o_copy;
+			for (int i = 4 * tid; i < a.wrows * SW; i += 4 * nt) {
+				const uint4 x = *reinterpret_cast<const uint4*>(win + i);
+				const uint32_t y = win[i + 4];
+#pragma unroll
+				for (int k = 1; k < 4; ++k)
+					*reinterpret_cast<uint4*>(copies + (k - 1) * a.copy + i) =
+						make_uint4(__funnelshift_r(x.x, x.y, 8 * k), __funnelshift_r(x.y, x.z, 8 * k),
+					               __funnelshift_r(x.z, x.w, 8 * k), __funnelshift_r(x.w, y, 8 * k));
+			}
+			sync();
+			if (count >= 0) {  // the columns left over
+				const int left = nd - a.cols, more = u.nb * nd * left;
+				for (int j0 = tid - lane; j0 < more; j0 += nt) {  // warp-uniform
+					const int j = min(j0 + lane, more - 1), v = a.div_nd(j), b = left == 2 ? v >> 1 : v, iy = j - v * nd, ix = a.cols + v - b * left;
+					const uint32_t* w = (ix & 3 ? copies + ((ix & 3) - 1) * a.copy : win) + iy * SW + ((16 * b + ix) >> 2);
+					least_of(best, b, (exhaustive_rows<1, SW>(w, blkw + b * 64, 1) >> 5) << 15 | (uint32_t)(iy * nd + ix), lane);
+				}
+			}
+			if (count < 0) exhaustive<GS, SW>(a, sm + a.o_task, n_tasks, win, copies, blkw, best, tid, nt);
+			else if (a.rows == GA) exhaustive<GA, SW>(a, sm + a.o_task, count, win, copies, blkw, best, tid, nt);
+			else exhaustive<GB, SW>(a, sm + a.o_task, count, win, copies, blkw, best, tid, nt);
 		}
 		sync();
 		if (tid < u.nb) {
@@ -563,16 +668,17 @@ __global__ void __launch_bounds__(HALVES ? 2 * MAXT : MAXT, MINB) full_me_elim_k
 			o[1] = u.cx + (idx - iy * nd) - r;
 			o[2] = (int32_t)(key >> 15);
 		}
-		sync();  // a list's next block overwrites the keys and the window
+		if (!LIST) break;  // a run per CTA
+		sync();            // a list's next block overwrites the keys and the window
 	}
 }
 
-template <int MINB, bool HALVES>
+template <class W, int MINB, int TEAMS>
 umi_status launch(const ElimArgs& a, int threads, size_t smem, int sms, cudaStream_t st) {
-	auto kern = full_me_elim_kernel<MINB, HALVES>;
+	auto kern = full_me_elim_kernel<W, MINB, TEAMS>;
 	UMI_TRY(umi::allow_shared(kern, smem));
 	// a list's length is known on the GPU only: CTAs that fill it once take its blocks in turn
-	const int grid = a.list ? std::min(a.units, MINB * sms) : a.units;
+	const int grid = TEAMS ? std::min(a.units, MINB * sms) : a.units;
 	kern<<<grid, threads, smem, st>>>(a);
 	return umi::launch_status("full_me_elim_kernel");
 }
@@ -581,8 +687,8 @@ umi_status launch(const ElimArgs& a, int threads, size_t smem, int sms, cudaStre
 
 namespace umi {
 
-// Every 16x16 argmin search that full_me.cu does not serve from registers:
-// any range 1..64, any width and alignment, lists and centres.
+// 16x16 argmin searches: any range 1..64, any width and alignment, lists and
+// centres (full_me.cu says which come here).
 umi_status full_me_elim(const uint8_t* cur, const uint8_t* ref, int h, int w, int r, const int32_t* centers,
                         int32_t* out, const int32_t* list, const int32_t* list_count, int max_slots, cudaStream_t st) {
 	ElimArgs a{};
@@ -600,19 +706,23 @@ umi_status full_me_elim(const uint8_t* cur, const uint8_t* ref, int h, int w, in
 	a.nb = 1;
 	if (!list && !centers) {
 		// as many blocks per run as the threads and the cell rows hold, as long as the runs fill the GPU
-		a.nb = std::max(1, std::min({MAXT / per_b, (QS - 3 - a.nd) / 16 + 1, MAXNB, a.nbx}));
+		a.nb = std::max(1, std::min({MAXT / per_b, (Wide::QS - 3 - a.nd) / 16 + 1, MAXNB, a.nbx}));
 		while (a.nb > 1 && ceil_div(a.nbx, a.nb) * nby < 2 * sms) --a.nb;
 	}
+	const bool narrow = a.nb == 1 && a.nd <= 65;
+	const int SW = narrow ? Narrow::SW : Wide::SW, QS = narrow ? Narrow::QS : Wide::QS;
 	a.runs_x = ceil_div(a.nbx, a.nb);
 	a.units = list || centers ? a.slots : a.runs_x * nby;
 	a.wrows = 2 * r + 16;
 	a.wwords = ceil_div(16 * a.nb + 2 * r, 4);
 	a.pieces = ceil_div(a.wwords, 4);
-	a.sw = 4 * (a.pieces | 1);
 	a.qrows = 2 * r + 13;
 	a.ncols = 16 * (a.nb - 1) + a.nd;
 	a.spw = 32 / a.pieces;
-	a.limit = std::max(1, a.nd * a.nd / 8);
+	// Survivors cost three times a candidate of the exhaustive search, which takes
+	// whole columns; below +-16 its copies of the window weigh more.  (Unrelated
+	// frames, +-32, a limit of nd^2 / 8: 164 us, / 16 145, / 32 125, / 48 125.)
+	a.limit = std::max(2 * a.nd, a.nd * a.nd / 32);
 	a.cur_words = aligned(cur, 4) && w % 4 == 0;
 	a.ref_pieces = aligned(ref, 16) && w % 16 == 0;
 	a.div_x = Div::by(list || centers ? a.nbx : a.runs_x);
@@ -623,21 +733,39 @@ umi_status full_me_elim(const uint8_t* cur, const uint8_t* ref, int h, int w, in
 	a.div_task = SmallDiv::by(per_b);
 	a.div_piece = SmallDiv::by(a.pieces);
 	a.div_spw = SmallDiv::by(a.spw);
+	// the exhaustive search of a run: rows per thread by the rows that a warp
+	// works through, each task costing three halves of a row more
+	a.cols = a.nd % 32 <= 2 && a.nd > 32 ? a.nd - a.nd % 32 : a.nd;
+	const auto rows_cost = [&](int g) {
+		return ceil_div(a.nb * a.cols * ceil_div(a.nd, g), narrow && !list ? 128 : 256) * (2 * g + 3);
+	};
+	a.rows = rows_cost(GB) < rows_cost(GA) ? GB : GA;
+	a.tasks = a.cols * ceil_div(a.nd, a.rows);
+	a.div_cols = SmallDiv::by(a.cols);
+	a.div_tasks = SmallDiv::by(a.tasks);
 	auto up4 = [](int n) { return (n + 3) & ~3; };
-	const bool halves = list && a.nd > 2 * RC;
-	const int threads = halves ? 2 * MAXT : ceil_div(a.nb * per_b, 32) * 32;
-	a.o_q = up4(a.wrows * a.sw + 4);
-	// the exhaustive search's copies: 8, 16, 24 banks from the window; its last
-	// row group reads up to BG - 1 rows past a window's end
-	a.copy = ceil_div(a.wrows * a.sw, 32) * 32 + 8;
+	const int threads = list ? 2 * (narrow ? Narrow::THREADS : Wide::THREADS)
+	                         : narrow ? Narrow::THREADS : ceil_div(a.nb * per_b, 32) * 32;
+	a.o_q = up4(a.wrows * SW + 4);
+	// the exhaustive search's copies: 8, 16, 24 banks from the window; with fewer
+	// rows than a thread takes it reads past a window's end
+	a.copy = ceil_div(a.wrows * SW, 32) * 32 + 8;
 	a.o_copy = ceil_div(a.o_q, 32) * 32 + 8;
-	a.o_blk = up4(std::max(a.o_q + (std::max(a.nd, RC) + 12) * QS, a.o_copy + 3 * a.copy + (BG - 1) * a.sw));
+	a.o_task = a.o_copy + 3 * a.copy + std::max(0, a.rows - a.nd) * SW;
+	// a task in the rows of two of a column's threads may be listed twice
+	a.o_blk = up4(std::max(a.o_q + (std::max(a.nd, RC) + 12) * QS,
+	                       a.o_task + a.nb * a.nd * (ceil_div(a.nd, GS) + a.nchunk - 1)));
 	a.o_cell = a.o_blk + 64 * a.nb;
 	a.o_list = a.o_cell + 4 * a.nb;
 	a.team_words = up4(a.o_list + a.nb * a.limit);
 	const size_t smem = 4 * (size_t)a.team_words;
-	if (halves) return launch<1, true>(a, threads, 2 * smem, sms, st);
-	return smem > kSmemThree ? launch<2, false>(a, threads, smem, sms, st) : launch<3, false>(a, threads, smem, sms, st);
+	if (list) {
+		if (narrow) return launch<Narrow, 3, 2>(a, threads, 2 * smem, sms, st);
+		return launch<Wide, 1, 2>(a, threads, 2 * smem, sms, st);
+	}
+	if (narrow) return launch<Narrow, 7, 0>(a, threads, smem, sms, st);
+	if (smem > kSmemThree) return launch<Wide, 2, 0>(a, threads, smem, sms, st);
+	return launch<Wide, 3, 0>(a, threads, smem, sms, st);
 }
 
 }  // namespace umi
