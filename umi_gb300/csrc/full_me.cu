@@ -24,10 +24,10 @@
 //    next macroblocks' windows are copied (4-byte cp.async by all threads)
 //    while the current ones are searched (full_me_pipe_kernel); the
 //    SAD-volume output keeps one CTA per group of macroblocks
-//    (full_me_kernel).  It serves 8x8 blocks with centres or lists, or few of
-//    them; other 8x8 blocks go to the strips of full_me_8.cu, 16x16 blocks with
-//    ranges up to 7 to the register-only kernel below, the rest to the exact
-//    elimination of full_me_elim.cu.
+//    (full_me_kernel).  It serves blocks with centres or lists, or few of them
+//    (16x16: up to +-24); other 8x8 blocks go to the strips of full_me_8.cu, 16x16
+//    blocks with ranges up to 7 to the register-only kernel below, the rest to the
+//    exact elimination of full_me_elim.cu.
 #include <algorithm>
 #include <cstring>
 
@@ -677,7 +677,19 @@ umi_status full_me_common(const uint8_t* cur, const uint8_t* ref, int32_t h, int
 		const umi_status rc = launch_small(cur, ref, centers, out, g, umi::as_stream(stream));
 		return rc == UMI_OK ? umi::ok() : rc;
 	}
-	if (!volume && b == 16) {
+	int dev = 0, sms = 0;
+	UMI_TRY(umi::cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
+	UMI_TRY(umi::cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"));
+	// Lists, centres and frames of few blocks leave the elimination one block per
+	// CTA; up to +-24 the general kernel, several blocks per CTA, is then as fast as
+	// it can be or faster, whatever the content (us, general and elimination from
+	// matching to unrelated frames: 2000 listed blocks +-8 13 and 17 to 19, +-16 26 and
+	// 16 to 30, +-24 40 and 31 to 52, +-26 62 and 41 to 61; 1080p with centres +-8 42
+	// and 57 to 80, +-16 91 and 62 to 108, +-26 212 and 86 to 165; 448 blocks +-8 9.6 and
+	// 7.3 to 8, +-16 9.6 and 9 to 12.4, +-32 - and 14.6 to 20; 880 blocks +-16 15.6 and 9
+	// to 13).
+	const bool general16 = r <= 24 && (list || centers || (r > 8 && g.nblk < 3 * sms));
+	if (!volume && b == 16 && !general16) {
 		const umi_status rc = umi::full_me_elim(cur, ref, h, w, r, centers, out, list, list_count, max_slots,
 		                                        umi::as_stream(stream));
 		return rc == UMI_OK ? umi::ok() : rc;
@@ -686,11 +698,8 @@ umi_status full_me_common(const uint8_t* cur, const uint8_t* ref, int32_t h, int
 	// them for the GPU; there the general kernel, one CTA for one or two blocks,
 	// is faster once a block's displacements fill it (240 blocks, +-16: 5.0 us
 	// and 6.6 in strips, 660 blocks 8.3 and 6.3; 240 blocks, +-7: 14.8 and 4.6).
-	int dev = 0, sms = 0;
-	UMI_TRY(umi::cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
-	UMI_TRY(umi::cuda_status(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute"));
 	const bool few = r <= 8 ? g.nblk < 4 : g.nblk <= (r < 16 ? 5 : 3) * sms;
-	if (!volume && !list && !centers && !few) {
+	if (!volume && b == 8 && !list && !centers && !few) {
 		const umi_status rc = umi::full_me_8(cur, ref, h, w, r, out, umi::as_stream(stream));
 		return rc == UMI_OK ? umi::ok() : rc;
 	}
@@ -731,9 +740,11 @@ umi_status full_me_common(const uint8_t* cur, const uint8_t* ref, int32_t h, int
 	// The leftover columns' groups of G2 rows may end below the main groups; their
 	// last rows' sums are not used, but their words are read.
 	const size_t below = g.ng2 ? std::max(0, g.ng2 * G2 - g.ng * G) * (size_t)g.win_words * 4 : 0;
-	if (!volume)  // 8x8 blocks: at most 160 KB of the two buffers (+-64)
-		rc = launch_pipe_b<8>(G, cur, ref, centers, out, g, threads_for(m * g.tasks_pipe), 2 * smem + below, st);
-	else
+	if (!volume) {  // at most 192 KB of the two buffers
+		const int tp = threads_for(m * g.tasks_pipe);
+		rc = b == 16 ? launch_pipe_b<16>(G, cur, ref, centers, out, g, tp, 2 * smem + below, st)
+		             : launch_pipe_b<8>(G, cur, ref, centers, out, g, tp, 2 * smem + below, st);
+	} else
 		rc = b == 16 ? launch_b<16>(G, cur, ref, out, g, threads, smem, st) : launch_b<8>(G, cur, ref, out, g, threads, smem, st);
 	return rc == UMI_OK ? umi::ok() : rc;
 }
