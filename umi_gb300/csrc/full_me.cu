@@ -695,10 +695,16 @@ umi_status full_me_common(const uint8_t* cur, const uint8_t* ref, int32_t h, int
 		return rc == UMI_OK ? umi::ok() : rc;
 	}
 	// 8x8 blocks at their own places go in strips.  A small frame has too few of
-	// them for the GPU; there the general kernel, one CTA for one or two blocks,
-	// is faster once a block's displacements fill it (240 blocks, +-16: 5.0 us
-	// and 6.6 in strips, 660 blocks 8.3 and 6.3; 240 blocks, +-7: 14.8 and 4.6).
-	const bool few = r <= 8 ? g.nblk < 4 : g.nblk <= (r < 16 ? 5 : 3) * sms;
+	// them for the GPU; there the general kernel, one CTA for one or two blocks, is
+	// faster once a block's displacements fill it, and longer where they fill whole
+	// groups of rows (+-9 to 13) or where 32 columns and a few (+-18, 19) leave the
+	// strips' split uneven.  Graph replays, us, general and strips: 100 blocks +-8 7.8
+	// and 5.3, +-16 5.4 and 6.8; 456 blocks +-10 5.2 and 6.2, +-16 6.9 and 6.8, +-18 6.6
+	// and 8.5, +-24 8.9 and 9.5; 616 +-15 8.9 and 7.3, +-21 9.9 and 11.1, +-24 11.3 and
+	// 11.2; 875 +-10 6.2 and 6.6, +-18 7.8 and 10.7; 950 +-10 6.4 and 6.6, +-18 9.4 and
+	// 7.9, +-24 14.8 and 9.7.
+	const int per_sm = (r >= 9 && r <= 13) || r == 18 || r == 19 ? 6 : 3;
+	const bool few = r <= 8 ? g.nblk < 4 : g.nblk <= per_sm * sms;
 	if (!volume && b == 8 && !list && !centers && !few) {
 		const umi_status rc = umi::full_me_8(cur, ref, h, w, r, out, umi::as_stream(stream));
 		return rc == UMI_OK ? umi::ok() : rc;
