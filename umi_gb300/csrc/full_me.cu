@@ -29,12 +29,8 @@
 //    blocks with ranges up to 7 to the register-only kernel below, the rest to the
 //    exact elimination of full_me_elim.cu.
 #include <algorithm>
-#include <cstring>
-
-#include <cudaTypedefs.h>
 
 #include "common.h"
-#include "tc_common.cuh"
 
 namespace umi {
 // Argmin search of 16x16 blocks (full_me_elim.cu): any range 1..64, any width
@@ -82,9 +78,9 @@ __device__ __forceinline__ int slot_block(const MeGeom& g, int slot) {
 	return slot < g.nblk ? slot : -1;
 }
 
-// Register budget per instantiation: the benchmark shape (b = 16, G = 13,
-// 352 threads) is held to 80 registers so that two CTAs (6 warps per SM
-// sub-partition x 80 x 32 <= 16K registers) fit an SM.
+// Register budget per instantiation: b = 16, G = 13 (+-32: 352 threads) is held
+// to 80 registers so that two CTAs (6 warps per SM sub-partition x 80 x 32 <= 16K
+// registers) fit an SM.
 // The other shapes get a budget of about 5G + 30 (ring + accumulators + addressing).
 template <int B, int G> struct MeRegs { static constexpr int value = B == 16 ? (5 * G + 31) / 8 * 8 + 8 : 64; };
 template <> struct MeRegs<16, 13> { static constexpr int value = 80; };
@@ -234,7 +230,6 @@ __device__ __forceinline__ void cp_async4(uint32_t* dst, const void* src) {
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Stage copy 0 of every window of group gi (and its current blocks) into buf.
-// Stage copy 0 of every window of group gi (and its current blocks) into buf.
 template <int B>
 __device__ __forceinline__ void me_stage_group(const MeGeom& g, uint32_t* buf, int gi, const uint8_t* __restrict__ cur,
                                                const uint8_t* __restrict__ ref, const int32_t* __restrict__ centers,
@@ -289,19 +284,6 @@ __device__ __forceinline__ void me_stage_group(const MeGeom& g, uint32_t* buf, i
 			}
 		}
 	}
-}
-
-// Window origin of slot `slot`'s block, or false past the last slot.
-template <int B>
-__device__ __forceinline__ bool me_window(const MeGeom& g, const int32_t* __restrict__ centers, int slot, int& blk,
-                                          int& gy0, int& gx0) {
-	blk = slot_block(g, slot);
-	if (blk < 0) return false;
-	const int by = blk / g.nbx, bx = blk - by * g.nbx;
-	const int cy = centers ? centers[2 * blk] : 0, cx = centers ? centers[2 * blk + 1] : 0;
-	gy0 = by * B + cy - g.r;
-	gx0 = bx * B + cx - g.r;
-	return true;
 }
 
 // Copies 1..3 of every window of group gi (word k of copy s holds bytes

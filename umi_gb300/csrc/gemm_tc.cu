@@ -1694,7 +1694,7 @@ extern "C" umi_status umi_conv2d_fprop_bf16(const void* x_nhwc, const void* w_kr
 
 namespace umi {
 
-// cuTensorMapEncodeTiled for the other translation units (full_me.cu).
+// cuTensorMapEncodeTiled for the other translation units.
 void* tma_encode_fn() { return reinterpret_cast<void*>(encode_fn()); }
 
 // One tensor-core layer of the motion-proposal network (see MenetRun):
