@@ -526,9 +526,13 @@ __global__ void __launch_bounds__(W::THREADS * (TEAMS ? TEAMS : 1), MINB) full_m
 		// +-32: 10 us whatever their content, else 9 to 14).  Elsewhere cells' sums that
 		// differ less from their neighbours' than 1.25 times the pixels from those below
 		// are noise: a random block stays below that in 999 of 1000 cases, one of the
-		// benchmark's texture (sigma 5.6, with noise of 2) above it.
+		// benchmark's texture (sigma 5.6, with noise of 2) above it.  Not so blocks at the
+		// frame's edges; in a list of a few rounds one of them, summed in full, would
+		// outlast the others, so shorter ones of wide windows go by the bound (the
+		// coarse pass at 4K, 8 pairs: 136.6 us, 134.5 so).
 		const bool alone = LIST && !teams && NT == Narrow::THREADS;
-		if (!alone && 8 * (differ >> 16) >= 5 * (differ & 0xffffu)) {
+		const bool tell = !LIST || NT == Narrow::THREADS || units > 4 * nteams * (int)gridDim.x;
+		if (!alone && (!tell || 8 * (differ >> 16) >= 5 * (differ & 0xffffu))) {
 			hard = 0;
 			int sh = 2;
 			while (sh < 4 && (256u << sh) < 2 * (mx - mn)) ++sh;
