@@ -1,8 +1,9 @@
 """Window operators of the UMI family on the generic operator (umi_launch).
 
 The reference ships eight example applications; these are four more of the
-same kind, each one descriptor over the closed-form generic kernel with a
-built-in strategy (no specialised kernel):
+same kind, each a descriptor with a built-in strategy, which umi_launch serves
+from staged image tiles where the window allows it and else by the closed-form
+generic kernel:
 
 * ``census``: census transform, one bit per window pixel (row-major), set
   where the pixel is below the centre (CENSUS_I32); edges replicated.
